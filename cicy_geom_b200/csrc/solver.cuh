@@ -108,20 +108,17 @@ struct MgWork {
     std::vector<Lvl> L;
     std::vector<MgLevel> host_lv;
     DBuf<MgLevel> dev_lv;
-    DBuf<double> cinv, z0, wtmp, sval, gj_panel;
+    DBuf<double> cinv, z0, wtmp, gj_panel;
     DBuf<unsigned long long> gj_sync;  // grid Gauss-Jordan: barrier counter, largest diagonal (bits)
     DBuf<int32_t> gj_err;
     DBuf<unsigned long long> bar;
-    DBuf<uint64_t> keys;
-    DBuf<uint32_t> vals;
-    DBuf<int32_t> flag, pos, head, uidx, mate, best, rep, total, scan_tmp, long_rows;
-    RadixScratch radix;
+    DBuf<int32_t> flag, pos, mate, best, rep, total, scan_tmp;
     // smoothed level-1 prolongator (fused hierarchy): Q = P - w D^-1 A_1 P and the sparse
     // products built from it (T = A_1 P, Q^T, W = A_1 Q, Q^T A_1), plus the gather scratch
     struct Smoothed {
-        DBuf<int32_t> tp, tc, qtp, qti, wp, wc, ap, ac, seg, ulen, longr;
+        DBuf<int32_t> tp, tc, qtp, qti, wp, wc, ap, ac, seg, ulen, longr, ocol;
         DBuf<double> tv, qv, qpv, qtv, wv, wpv, av, y, v, gv, gv2, ov, ov2;
-        DBuf<uint64_t> gkey, okey;
+        DBuf<uint64_t> gkey;
     } sa;
     int levels = 0;
     bool dense = false;

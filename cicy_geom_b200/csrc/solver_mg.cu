@@ -87,15 +87,34 @@ __global__ void k_rowsum0(int n, const int32_t* __restrict__ rp, const int32_t* 
     }
 }
 
+// The setup's row kernels take `lanes` (a power of two up to 32) threads per row: rows have 2-5
+// couplings on the chain level and hundreds on the lower levels of dense networks, where one
+// thread per row read them one uncoalesced entry after another (47.7k-CNT / 5 um realisation:
+// k_strongest 8.6 ms and k_rr_fill 9.7 ms in all, now 0.78 and 0.66 ms).
+struct RowLanes {
+    int first, step, lane;  // first row and row stride of the group, lane within it
+};
+__device__ __forceinline__ RowLanes row_lanes(int lanes) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    return RowLanes{t / lanes, (int)(gridDim.x * blockDim.x) / lanes, t % lanes};
+}
+int lanes_of(long long entries, int rows) {  // about two entries per thread
+    int l = 1;
+    while (l < 32 && 2LL * l * rows < entries) l <<= 1;
+    return l;
+}
+
 // Strongest neighbour of each row (|a_ij| largest, ties: smaller j); with
 // free_only, among unmatched rows and only for unmatched rows.
-__global__ void k_strongest(int n, int free_only, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+__global__ void k_strongest(int n, int lanes, int free_only, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                             const double* __restrict__ v, const int32_t* __restrict__ mate, int32_t* __restrict__ best) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const RowLanes g = row_lanes(lanes);
+    const unsigned mask = lanes >= 32 ? 0xffffffffu : (((1u << lanes) - 1) << ((threadIdx.x & 31) & ~(lanes - 1)));
+    for (int i = g.first; i < n; i += g.step) {
         int bj = -1;
+        double bs = -1.0;
         if (!(free_only && mate[i] >= 0)) {
-            double bs = -1.0;
-            for (int k = rp[i]; k < rp[i + 1]; k++) {
+            for (int k = rp[i] + g.lane; k < rp[i + 1]; k += lanes) {
                 const int j = ci[k];
                 if (free_only && mate[j] >= 0) continue;
                 const double s = fabs(v[k]);
@@ -105,7 +124,15 @@ __global__ void k_strongest(int n, int free_only, const int32_t* __restrict__ rp
                 }
             }
         }
-        best[i] = bj;
+        for (int o = lanes / 2; o > 0; o >>= 1) {
+            const double s = __shfl_xor_sync(mask, bs, o, lanes);
+            const int j = __shfl_xor_sync(mask, bj, o, lanes);
+            if (s > bs || (s == bs && j < bj)) {
+                bs = s;
+                bj = j;
+            }
+        }
+        if (g.lane == 0) best[i] = bj;
     }
 }
 
@@ -144,11 +171,12 @@ __global__ void k_fill_neg(int n, int32_t* __restrict__ a) {
 
 // Dense coarsest matrix (M zeroed before), then its inverse in place by Gauss-Jordan
 // without pivoting (SPD up to floating islands).
-__global__ void k_dense_coarse(int nc, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ v,
+__global__ void k_dense_coarse(int nc, int lanes, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ v,
                                const double* __restrict__ diag, double* __restrict__ M) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x) {
-        for (int k = rp[i]; k < rp[i + 1]; k++) M[(size_t)i * nc + ci[k]] = v[k];
-        M[(size_t)i * nc + i] = diag[i];
+    const RowLanes g = row_lanes(lanes);
+    for (int i = g.first; i < nc; i += g.step) {
+        for (int k = rp[i] + g.lane; k < rp[i + 1]; k += lanes) M[(size_t)i * nc + ci[k]] = v[k];
+        if (g.lane == 0) M[(size_t)i * nc + i] = diag[i];
     }
 }
 
@@ -255,21 +283,24 @@ __global__ void __launch_bounds__(kGjThreads) k_gauss_jordan(int n, double* __re
     for (int e = t; e < n * n; e += kGjThreads) M[e] = S[e];
 }
 
-__global__ void k_ra_fill(int nc, const int32_t* __restrict__ mptr, const int32_t* __restrict__ midx, const int32_t* __restrict__ rp,
+__global__ void k_ra_fill(int nc, int lanes, const int32_t* __restrict__ mptr, const int32_t* __restrict__ midx, const int32_t* __restrict__ rp,
                           const int32_t* __restrict__ ci, const double* __restrict__ v, const double* __restrict__ diag,
                           const int32_t* __restrict__ ra_ptr, int32_t* __restrict__ ra_col, double* __restrict__ ra_val) {
-    for (int J = blockIdx.x * blockDim.x + threadIdx.x; J < nc; J += gridDim.x * blockDim.x) {
+    const RowLanes g = row_lanes(lanes);
+    for (int J = g.first; J < nc; J += g.step) {
         int e = ra_ptr[J];
         for (int m = mptr[J]; m < mptr[J + 1]; m++) {
-            const int I = midx[m];
-            ra_col[e] = I;
-            ra_val[e] = diag[I];
-            e++;
-            for (int k = rp[I]; k < rp[I + 1]; k++) {
-                ra_col[e] = ci[k];
-                ra_val[e] = v[k];
-                e++;
+            const int I = midx[m], b = rp[I], len = rp[I + 1] - b;
+            if (g.lane == 0) {
+                ra_col[e] = I;
+                ra_val[e] = diag[I];
             }
+            e++;
+            for (int k = g.lane; k < len; k += lanes) {
+                ra_col[e + k] = ci[b + k];
+                ra_val[e + k] = v[b + k];
+            }
+            e += len;
         }
     }
 }
@@ -279,27 +310,35 @@ __global__ void k_ra_fill(int nc, const int32_t* __restrict__ mptr, const int32_
 // diagonal and couplings (column n + c: z_l[c], weight -a), the rows of P^T A_l, so
 // r_{l+1} = P^T (r_l - A_l z_l) is one gathered dot product.  rr_ptr = mptr + ra_ptr, both
 // prefix sums (ra_ptr: the P^T A_l row lengths).
-__global__ void k_rr_fill(int nc, int n, const int32_t* __restrict__ mptr, const int32_t* __restrict__ midx,
+__global__ void k_rr_fill(int nc, int n, int lanes, const int32_t* __restrict__ mptr, const int32_t* __restrict__ midx,
                           const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ v,
                           const double* __restrict__ diag, const int32_t* __restrict__ ra_ptr, int32_t* __restrict__ rr_ptr,
                           int32_t* __restrict__ rr_col, double* __restrict__ rr_val) {
-    for (int J = blockIdx.x * blockDim.x + threadIdx.x; J < nc; J += gridDim.x * blockDim.x) {
-        int e = mptr[J] + ra_ptr[J];
-        rr_ptr[J] = e;
-        if (J == nc - 1) rr_ptr[nc] = mptr[nc] + ra_ptr[nc];
-        for (int m = mptr[J]; m < mptr[J + 1]; m++, e++) {
-            rr_col[e] = midx[m];
-            rr_val[e] = 1.0;
+    const RowLanes g = row_lanes(lanes);
+    for (int J = g.first; J < nc; J += g.step) {
+        const int m0 = mptr[J], m1 = mptr[J + 1];
+        int e = m0 + ra_ptr[J];
+        if (g.lane == 0) {
+            rr_ptr[J] = e;
+            if (J == nc - 1) rr_ptr[nc] = mptr[nc] + ra_ptr[nc];
         }
-        for (int m = mptr[J]; m < mptr[J + 1]; m++) {
-            const int I = midx[m];
-            rr_col[e] = n + I;
-            rr_val[e] = -diag[I];
-            e++;
-            for (int k = rp[I]; k < rp[I + 1]; k++, e++) {
-                rr_col[e] = n + ci[k];
-                rr_val[e] = -v[k];
+        for (int m = g.lane; m < m1 - m0; m += lanes) {
+            rr_col[e + m] = midx[m0 + m];
+            rr_val[e + m] = 1.0;
+        }
+        e += m1 - m0;
+        for (int m = m0; m < m1; m++) {
+            const int I = midx[m], b = rp[I], len = rp[I + 1] - b;
+            if (g.lane == 0) {
+                rr_col[e] = n + I;
+                rr_val[e] = -diag[I];
             }
+            e++;
+            for (int k = g.lane; k < len; k += lanes) {
+                rr_col[e + k] = n + ci[b + k];
+                rr_val[e + k] = -v[b + k];
+            }
+            e += len;
         }
     }
 }
@@ -307,24 +346,28 @@ __global__ void k_rr_fill(int nc, int n, const int32_t* __restrict__ mptr, const
 // Fused prolongation-smoother rows of level l (1 <= l < coarsest): row I holds its diagonal
 // and off-diagonal couplings twice, on z_l (column c < n) and on the coarse correction
 // (column n + aggregate of c), so w = r_l - A_l (z_l + P zc) is one gathered dot product.
-__global__ void k_pq_fill(int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ v,
+__global__ void k_pq_fill(int n, int lanes, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ v,
                           const double* __restrict__ diag, const int32_t* __restrict__ agg, int32_t* __restrict__ pq_ptr,
                           int32_t* __restrict__ pq_col, double* __restrict__ pq_val) {
-    for (int I = blockIdx.x * blockDim.x + threadIdx.x; I < n; I += gridDim.x * blockDim.x) {
-        int e = 2 * (rp[I] + I);
-        pq_ptr[I] = e;
-        if (I == n - 1) pq_ptr[n] = 2 * (rp[n] + n);
-        pq_col[e] = I;
-        pq_val[e] = diag[I];
-        pq_col[e + 1] = n + agg[I];
-        pq_val[e + 1] = diag[I];
+    const RowLanes g = row_lanes(lanes);
+    for (int I = g.first; I < n; I += g.step) {
+        const int b = rp[I], len = rp[I + 1] - b;
+        int e = 2 * (b + I);
+        if (g.lane == 0) {
+            pq_ptr[I] = e;
+            if (I == n - 1) pq_ptr[n] = 2 * (rp[n] + n);
+            pq_col[e] = I;
+            pq_val[e] = diag[I];
+            pq_col[e + 1] = n + agg[I];
+            pq_val[e + 1] = diag[I];
+        }
         e += 2;
-        for (int k = rp[I]; k < rp[I + 1]; k++, e += 2) {
-            const int c = ci[k];
-            pq_col[e] = c;
-            pq_val[e] = v[k];
-            pq_col[e + 1] = n + agg[c];
-            pq_val[e + 1] = v[k];
+        for (int k = g.lane; k < len; k += lanes) {
+            const int c = ci[b + k];
+            pq_col[e + 2 * k] = c;
+            pq_val[e + 2 * k] = v[b + k];
+            pq_col[e + 2 * k + 1] = n + agg[c];
+            pq_val[e + 2 * k + 1] = v[b + k];
         }
     }
 }
@@ -1513,188 +1556,24 @@ __global__ void k_member_sort(int nc, const int32_t* __restrict__ mptr, int32_t*
     }
 }
 
-// Per aggregate: couplings gathered from its members' rows (seg_len) and the
-// length of its restriction row P^T A_l (members' rows with their diagonals).
-__global__ void k_agg_lengths(int nc, const int32_t* __restrict__ mptr, const int32_t* __restrict__ midx, const int32_t* __restrict__ rp,
-                              int32_t* __restrict__ seg_len, int32_t* __restrict__ ra_len) {
+// Length of each aggregate's restriction row P^T A_l (members' rows with their diagonals).
+__global__ void k_ra_lengths(int nc, const int32_t* __restrict__ mptr, const int32_t* __restrict__ midx, const int32_t* __restrict__ rp,
+                             int32_t* __restrict__ ra_len) {
     for (int J = blockIdx.x * blockDim.x + threadIdx.x; J < nc; J += gridDim.x * blockDim.x) {
-        int s = 0;
+        int s = mptr[J + 1] - mptr[J];
         for (int m = mptr[J]; m < mptr[J + 1]; m++) {
             const int I = midx[m];
             s += rp[I + 1] - rp[I];
         }
-        seg_len[J] = s;
-        if (ra_len) ra_len[J] = s + (mptr[J + 1] - mptr[J]);
+        ra_len[J] = s;
     }
 }
 
-// Coarse row J: the cross-aggregate couplings of its members (in member then entry
-// order), gathered as keys (coarse column, gather position) with their values, are sorted
-// (keys are unique, so the order equals a stable sort by column) and summed per column in
-// gather order (deterministic); the row's diagonal comes from the summed row sums (no
-// cancellation of the large intra-aggregate entries), and its l1-Jacobi weight from
-// |d| + sum |a|.  `reduce_row` does the summing and writes the compacted row at seg_off[J].
-__device__ __forceinline__ void reduce_row(int J, int cnt, double rs, const uint64_t* key, const double* val, uint64_t* __restrict__ okey,
-                                           double* __restrict__ oval, int32_t* __restrict__ ulen, double* __restrict__ rs_c,
-                                           double* __restrict__ diag, double* __restrict__ l1inv) {
-    int u = 0;
-    double off = 0, offabs = 0;
-    for (int i = 0; i < cnt;) {  // sum runs of equal columns, in gather order
-        const uint32_t c = (uint32_t)(key[i] >> 32);
-        double acc = 0;
-        while (i < cnt && (uint32_t)(key[i] >> 32) == c) acc += val[i++];
-        okey[u] = c;
-        oval[u] = acc;
-        u++;
-        off += acc;
-        offabs += fabs(acc);
-    }
-    ulen[J] = u;
-    const double d = rs - off;
-    rs_c[J] = rs;
-    diag[J] = d;
-    const double l1 = fabs(d) + offabs;
-    l1inv[J] = l1 > 0 ? 1.0 / l1 : 0.0;
-}
-
-// One warp per coarse row: the lanes gather a member row's couplings 32 at a time (ballot
-// ranks keep the gather order), a bitonic sort orders them in shared memory, lane 0 sums the
-// runs.  Rows with more than kCrCap couplings are listed for k_coarse_rows_long.
-constexpr int kCrWarps = 4;
-constexpr int kCrCap = 512;  // power of two
-__global__ void __launch_bounds__(kCrWarps * 32) k_coarse_rows(int nc, const int32_t* __restrict__ mptr, const int32_t* __restrict__ midx,
-                                                               const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
-                                                               const double* __restrict__ v, const int32_t* __restrict__ agg,
-                                                               const double* __restrict__ rs_f, const int32_t* __restrict__ seg_off,
-                                                               uint64_t* __restrict__ skey, double* __restrict__ sval, int32_t* __restrict__ ulen,
-                                                               double* __restrict__ rs_c, double* __restrict__ diag, double* __restrict__ l1inv,
-                                                               int32_t* __restrict__ long_rows, int32_t* __restrict__ n_long) {
-    __shared__ uint64_t sk[kCrWarps][kCrCap];
-    __shared__ double sv[kCrWarps][kCrCap];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint64_t* K = sk[warp];
-    double* V = sv[warp];
-    for (int J = blockIdx.x * kCrWarps + warp; J < nc; J += gridDim.x * kCrWarps) {
-        int cnt = 0;
-        double rs = 0;
-        for (int m = mptr[J]; m < mptr[J + 1]; m++) {
-            const int I = midx[m];
-            if (lane == 0) rs += rs_f[I];
-            const int b = rp[I], e = rp[I + 1];
-            for (int k0 = b; k0 < e; k0 += 32) {
-                const int k = k0 + lane;
-                int c = -1;
-                double x = 0;
-                if (k < e) {
-                    c = agg[ci[k]];
-                    x = v[k];
-                }
-                const bool keep = k < e && c != J;
-                const unsigned bal = __ballot_sync(0xffffffffu, keep);
-                const int pos = cnt + __popc(bal & ((1u << lane) - 1));
-                if (keep && pos < kCrCap) {
-                    K[pos] = ((uint64_t)(uint32_t)c << 32) | (uint32_t)pos;
-                    V[pos] = x;
-                }
-                cnt += __popc(bal);
-            }
-        }
-        if (cnt > kCrCap) {
-            if (lane == 0) long_rows[atomicAdd(n_long, 1)] = J;
-            __syncwarp();
-            continue;
-        }
-        int P = 1;
-        while (P < cnt) P <<= 1;
-        for (int i = cnt + lane; i < P; i += 32) K[i] = ~0ull;
-        __syncwarp();
-        for (int size = 2; size <= P; size <<= 1)
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                for (int i = lane; i < P; i += 32) {
-                    const int j = i ^ stride;
-                    if (j > i) {
-                        const bool up = (i & size) == 0;
-                        const uint64_t ki = K[i], kj = K[j];
-                        if ((ki > kj) == up) {
-                            K[i] = kj;
-                            K[j] = ki;
-                            const double t = V[i];
-                            V[i] = V[j];
-                            V[j] = t;
-                        }
-                    }
-                }
-                __syncwarp();
-            }
-        if (lane == 0) {
-            const int o = seg_off[J];
-            reduce_row(J, cnt, rs, K, V, skey + o, sval + o, ulen, rs_c, diag, l1inv);
-        }
-        __syncwarp();
-    }
-}
-
-// The rows k_coarse_rows listed as too long for shared memory: one thread each, gathered and
-// Shell-sorted in the global scratch at seg_off[J].
-__global__ void k_coarse_rows_long(const int32_t* __restrict__ long_rows, const int32_t* __restrict__ n_long, const int32_t* __restrict__ mptr,
-                                   const int32_t* __restrict__ midx, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
-                                   const double* __restrict__ v, const int32_t* __restrict__ agg, const double* __restrict__ rs_f,
-                                   const int32_t* __restrict__ seg_off, uint64_t* __restrict__ skey, double* __restrict__ sval,
-                                   int32_t* __restrict__ ulen, double* __restrict__ rs_c, double* __restrict__ diag, double* __restrict__ l1inv) {
-    const int nl = *n_long;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nl; t += gridDim.x * blockDim.x) {
-        const int J = long_rows[t];
-        const int o = seg_off[J];
-        int cnt = 0;
-        double rs = 0;
-        for (int m = mptr[J]; m < mptr[J + 1]; m++) {
-            const int I = midx[m];
-            rs += rs_f[I];
-            for (int k = rp[I]; k < rp[I + 1]; k++) {
-                const int c = agg[ci[k]];
-                if (c == J) continue;
-                skey[o + cnt] = ((uint64_t)(uint32_t)c << 32) | (uint32_t)cnt;
-                sval[o + cnt] = v[k];
-                cnt++;
-            }
-        }
-        int gap = 1;
-        while (gap * 9 / 4 + 1 < cnt) gap = gap * 9 / 4 + 1;
-        for (;; gap = max(1, (gap - 1) * 4 / 9)) {  // ..., 2, 1: the last pass is insertion sort
-            for (int i = gap; i < cnt; i++) {
-                const uint64_t key = skey[o + i];
-                const double x = sval[o + i];
-                int j = i;
-                while (j >= gap && skey[o + j - gap] > key) {
-                    skey[o + j] = skey[o + j - gap];
-                    sval[o + j] = sval[o + j - gap];
-                    j -= gap;
-                }
-                skey[o + j] = key;
-                sval[o + j] = x;
-            }
-            if (gap == 1) break;
-        }
-        reduce_row(J, cnt, rs, skey + o, sval + o, skey + o, sval + o, ulen, rs_c, diag, l1inv);
-    }
-}
-
-__global__ void k_coarse_copy(int nc, const int32_t* __restrict__ seg_off, const int32_t* __restrict__ ulen, const int32_t* __restrict__ rp_c,
-                              const uint64_t* __restrict__ scol, const double* __restrict__ sval, int32_t* __restrict__ ci_c,
-                              double* __restrict__ v_c) {
-    for (int J = blockIdx.x * blockDim.x + threadIdx.x; J < nc; J += gridDim.x * blockDim.x) {
-        const int o = seg_off[J], d = rp_c[J];
-        for (int i = 0; i < ulen[J]; i++) {
-            ci_c[d + i] = (int32_t)scol[o + i];
-            v_c[d + i] = sval[o + i];
-        }
-    }
-}
-
-__global__ void k_cagg_rows(int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const int32_t* __restrict__ agg,
-                            int32_t* __restrict__ cagg) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        for (int k = rp[i]; k < rp[i + 1]; k++) cagg[k] = agg[ci[k]];
+// Aggregate of every entry's column.
+__global__ void k_cagg(const int32_t* __restrict__ nnz, const int32_t* __restrict__ ci, const int32_t* __restrict__ agg,
+                       int32_t* __restrict__ cagg) {
+    const int n = *nnz;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) cagg[k] = agg[ci[k]];
 }
 
 // ---------------------------------------------------------------------------
@@ -1713,10 +1592,30 @@ __global__ void k_cagg_rows(int n, const int32_t* __restrict__ rp, const int32_t
 // sources (s, w); the terms are sorted by column (keys (column, gather position) are
 // unique) and summed in gather order, so no result depends on thread timing.
 constexpr double kSaOmega = 4.0 / 3.0;
-constexpr int kGrWarps = 4;
-constexpr int kGrCap = 512;  // power of two
 
-struct RowSrc {  // sources of output row J: (J, 1) when ptr is null, else (J, diag[J]) (with diag) and row J of the CSR
+// Row gather: output row J is the sum of w * (row s of B) over its sources (s, w), used for the
+// Galerkin coarse rows (sources: an aggregate's members, columns mapped to aggregates) and for
+// the products of the smoothed prolongator.  The candidate terms of a row are numbered in
+// source, then entry order; their keys (column, number) are unique, so sorting them and adding
+// each column's run in that order gives sums that do not depend on thread timing.
+//
+// What bounds it: the chains of dependent loads (source -> its row -> its entries) and, for rows
+// of more than a few hundred terms, the sort.  Sources are therefore read one per thread with a
+// scan of their lengths, and the terms are spread over all threads (three dependent loads per
+// batch of sources, not per source); rows are dealt by length to a warp (up to kGrWarpCap
+// terms), a small CTA (kGrMidCap), a large CTA (kGrBigCap, all in shared memory) or a large CTA
+// sorting in global memory.  Each column's first term adds its run, so runs are summed in
+// parallel.  Dense networks have mostly rows of 500-6,000 terms: on a 47.7k-CNT / 5 um
+// realisation the gathers of both hierarchies took 464 ms with one thread per row above 512
+// terms and serial run sums, 4.8 ms so; on 9,117 CNTs in 3.37 um 18.4 ms and 0.6 ms.
+constexpr int kGrWarps = 4;
+constexpr int kGrWarpCap = 512;
+constexpr int kGrMidThreads = 256, kGrMidCap = 2048;
+constexpr int kGrBigThreads = 1024, kGrBigCap = 8192;
+constexpr int kGrTiers = 3;  // lists of the rows above kGrWarpCap: mid, big, global
+constexpr uint64_t kGrNone = ~0ull;
+
+struct RowSrc {  // sources of output row J: (J, 1) when ptr is null, else (J, diag[J]) (with diag) and row J of the CSR (val null: weight 1)
     const int32_t* ptr;
     const int32_t* idx;
     const double* val;
@@ -1732,16 +1631,16 @@ struct RowMat {  // row s of B: (s, diag[s]) (with diag), then its CSR entries; 
     const int32_t* cmap;  // column map (null: identity)
 };
 struct GatherOut {
-    const int32_t* seg;                 // per output row: offset of its segment (candidate terms)
-    uint64_t* gkey;                     // long rows: gathered terms (segment layout)
+    const int32_t* seg;                 // per output row: offset of its segment (candidate terms), nrows + 1
+    uint64_t* gkey;                     // terms of the rows sorted in global memory (segment layout)
     double* gv;
     double* gv2;
-    uint64_t* okey;                     // summed runs (segment layout)
+    int32_t* ocol;                      // summed runs (segment layout)
     double* ov;
     double* ov2;
     int32_t* ulen;                      // runs per row
-    int32_t* longr;                     // rows with more than kGrCap terms
-    int32_t* nlong;
+    const int32_t* list;                // kGrTiers lists of nrows
+    const int32_t* nlist;               // their lengths
     int skip_diag;                      // drop column J of row J
     const double* rsv;                  // with rs_out: row sum of row J = sum_t w_t rsv[s_t]
     double* rs_out;
@@ -1767,7 +1666,7 @@ __device__ __forceinline__ void src_get(const RowSrc& S, int J, int t, int& s, d
     }
     const int k = S.ptr[J] + t;
     s = S.idx[k];
-    w = S.val[k];
+    w = S.val ? S.val[k] : 1.0;
 }
 
 __device__ __forceinline__ int mat_len(const RowMat& B, int s) { return (B.ptr[s + 1] - B.ptr[s]) + (B.diag ? 1 : 0); }
@@ -1786,177 +1685,243 @@ __device__ __forceinline__ void mat_get(const RowMat& B, int s, int t, int& c, d
     if (B.cmap) c = B.cmap[c];
 }
 
-__global__ void k_gather_len(int nrows, RowSrc S, RowMat B, int32_t* __restrict__ seg) {
-    for (int J = blockIdx.x * blockDim.x + threadIdx.x; J < nrows; J += gridDim.x * blockDim.x) {
+// Candidate terms per row, and the rows too long for a warp listed by length (nlist zeroed before).
+__global__ void k_gather_len(int nrows, int lanes, RowSrc S, RowMat B, int32_t* __restrict__ seg, int32_t* __restrict__ list, int32_t* nlist) {
+    const RowLanes g = row_lanes(lanes);
+    const unsigned mask = lanes >= 32 ? 0xffffffffu : (((1u << lanes) - 1) << ((threadIdx.x & 31) & ~(lanes - 1)));
+    for (int J = g.first; J < nrows; J += g.step) {
         int c = 0;
         const int ns = src_count(S, J);
-        for (int t = 0; t < ns; t++) {
+        for (int t = g.lane; t < ns; t += lanes) {
             int s;
             double w;
             src_get(S, J, t, s, w);
             c += mat_len(B, s);
         }
+        for (int o = lanes / 2; o > 0; o >>= 1) c += __shfl_xor_sync(mask, c, o, lanes);
+        if (g.lane != 0) continue;
         seg[J] = c;
         if (J == 0) seg[nrows] = 0;
-    }
-}
-
-// Sorted keys of one row (gather positions in their low half) summed into runs of equal
-// columns in gather order; with rs_out, the row's diagonal from its row sum (skip_diag rows)
-// and its l1-Jacobi weight, as reduce_row does.
-__device__ __forceinline__ void gather_reduce(int J, int cnt, const uint64_t* key, const double* val, const double* val2, double rs,
-                                              const GatherOut& O, int o) {
-    int u = 0;
-    double off = 0, offabs = 0;
-    for (int i = 0; i < cnt;) {
-        const uint32_t c = (uint32_t)(key[i] >> 32);
-        double acc = 0, acc2 = 0;
-        while (i < cnt && (uint32_t)(key[i] >> 32) == c) {
-            const uint32_t p = (uint32_t)key[i];
-            acc += val[p];
-            if (val2) acc2 += val2[p];
-            i++;
+        if (c > kGrWarpCap) {
+            const int tier = c <= kGrMidCap ? 0 : c <= kGrBigCap ? 1 : 2;
+            list[(size_t)tier * nrows + atomicAdd(&nlist[tier], 1)] = J;
         }
-        O.okey[o + u] = c;
-        O.ov[o + u] = acc;
-        if (val2) O.ov2[o + u] = acc2;
-        u++;
-        off += acc;
-        offabs += fabs(acc);
-    }
-    O.ulen[J] = u;
-    if (O.rs_out) {
-        const double d = rs - off;
-        O.rs_out[J] = rs;
-        O.diag_out[J] = d;
-        const double l1 = fabs(d) + offabs;
-        O.l1_out[J] = l1 > 0 ? 1.0 / l1 : 0.0;
     }
 }
 
-// One warp per output row: ballot-ranked gather into shared memory, bitonic sort of the
-// keys, lane 0 sums the runs.  Rows with more than kGrCap terms go to k_gather_rows_long.
+// The T threads of one row (a warp or a CTA); sync() orders their shared or global memory accesses.
+template <int T>
+__device__ __forceinline__ void row_sync() {
+    if constexpr (T == 32) __syncwarp();
+    else __syncthreads();
+}
+
+// Ascending bitonic sort of key[0 .. n) for any n (flip-merge form: every comparison puts the
+// smaller key first, so the missing keys past n act as +infinity and need no padding).
+template <int T>
+__device__ __forceinline__ void row_sort(uint64_t* key, int n, int tid) {
+    int P = 1;
+    while (P < n) P <<= 1;
+    auto order = [&](int a, int b) {
+        if (b >= n) return;
+        const uint64_t ka = key[a], kb = key[b];
+        if (ka > kb) {
+            key[a] = kb;
+            key[b] = ka;
+        }
+    };
+    for (int half = 1, lg = 0; 2 * half <= P; half <<= 1, lg++) {
+        for (int q = tid; q < P / 2; q += T) {
+            const int base = (q >> lg) << (lg + 1), r = q & (half - 1);
+            order(base + r, base + 2 * half - 1 - r);
+        }
+        row_sync<T>();
+        for (int stride = half >> 1; stride > 0; stride >>= 1) {
+            for (int q = tid; q < P / 2; q += T) {
+                const int a = ((q & ~(stride - 1)) << 1) | (q & (stride - 1));
+                order(a, a + stride);
+            }
+            row_sync<T>();
+        }
+    }
+}
+
+template <int T>
+__device__ __forceinline__ int row_scan(int v, int tid, int* ws, int& total) {  // exclusive sum over the T threads
+    const int lane = tid & 31;
+    int incl = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
+    }
+    if constexpr (T == 32) {
+        total = __shfl_sync(0xffffffffu, incl, 31);
+        return incl - v;
+    } else {
+        if (lane == 31) ws[tid >> 5] = incl;
+        __syncthreads();
+        int below = 0, all = 0;
+        for (int k = 0; k < T / 32; k++) {
+            if (k < (tid >> 5)) below += ws[k];
+            all += ws[k];
+        }
+        __syncthreads();
+        total = all;
+        return below + incl - v;
+    }
+}
+
+template <int T>
+__device__ __forceinline__ double row_total(double v, int tid, double* ws) {  // sum over the T threads, fixed order
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if constexpr (T == 32) {
+        return v;
+    } else {
+        if ((tid & 31) == 0) ws[tid >> 5] = v;
+        __syncthreads();
+        double s = 0;
+        for (int k = 0; k < T / 32; k++) s += ws[k];
+        __syncthreads();
+        return s;
+    }
+}
+
+// One output row by T threads: terms into key / val (/ val2), sort, run sums at segment offset o.
+// ssrc, sw, spre: T shared entries each; wsi, wsd: T / 32 shared entries each.
+template <int T, bool TWO>
+__device__ __forceinline__ void gather_row(int J, const RowSrc& S, const RowMat& B, const GatherOut& O, uint64_t* key, double* val,
+                                           double* val2, int tid, int* ssrc, double* sw, int* spre, int* wsi, double* wsd) {
+    const int o = O.seg[J];
+    const int ns = src_count(S, J);
+    int cnt = 0;
+    double rs = 0;
+    for (int t0 = 0; t0 < ns; t0 += T) {
+        int s = 0, L = 0, tot;
+        double w = 0;
+        if (t0 + tid < ns) {
+            src_get(S, J, t0 + tid, s, w);
+            L = mat_len(B, s);
+            if (O.rsv) rs += w * O.rsv[s];
+        }
+        const int pre = row_scan<T>(L, tid, wsi, tot);
+        ssrc[tid] = s;
+        sw[tid] = w;
+        spre[tid] = pre;
+        row_sync<T>();
+        const int nb = min(T, ns - t0);
+        for (int f = tid; f < tot; f += T) {
+            int lo = 0, hi = nb;  // last source whose first term is <= f (empty rows share a start; the last one holds f)
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (spre[mid] <= f) lo = mid;
+                else hi = mid;
+            }
+            int c;
+            double x, x2;
+            mat_get(B, ssrc[lo], f - spre[lo], c, x, x2);
+            key[cnt + f] = (O.skip_diag && c == J) ? kGrNone : (((uint64_t)(uint32_t)c << 32) | (uint32_t)(cnt + f));
+            val[cnt + f] = sw[lo] * x;
+            if (TWO) val2[cnt + f] = sw[lo] * x2;
+        }
+        cnt += tot;
+        row_sync<T>();
+    }
+    row_sort<T>(key, cnt, tid);
+    int u0 = 0;
+    double off = 0, offabs = 0;
+    for (int i0 = 0; i0 < cnt; i0 += T) {
+        const int i = i0 + tid;
+        const uint64_t k = i < cnt ? key[i] : kGrNone;
+        const uint32_t c = (uint32_t)(k >> 32);
+        const bool head = k != kGrNone && (i == 0 || (uint32_t)(key[i - 1] >> 32) != c);
+        int nh;
+        const int u = o + u0 + row_scan<T>(head ? 1 : 0, tid, wsi, nh);
+        if (head) {
+            double acc = 0, acc2 = 0;
+            uint64_t kj = k;
+            for (int j = i;;) {
+                const uint32_t p = (uint32_t)kj;
+                acc += val[p];
+                if (TWO) acc2 += val2[p];
+                if (++j >= cnt) break;
+                kj = key[j];
+                if ((uint32_t)(kj >> 32) != c) break;
+            }
+            O.ocol[u] = (int32_t)c;
+            O.ov[u] = acc;
+            if (TWO) O.ov2[u] = acc2;
+            off += acc;
+            offabs += fabs(acc);
+        }
+        u0 += nh;
+    }
+    if (tid == 0) O.ulen[J] = u0;
+    if (O.rs_out) {  // the row's diagonal from its row sum (no cancellation of large entries) and its l1-Jacobi weight
+        rs = row_total<T>(rs, tid, wsd);
+        off = row_total<T>(off, tid, wsd);
+        offabs = row_total<T>(offabs, tid, wsd);
+        if (tid == 0) {
+            const double d = rs - off;
+            O.rs_out[J] = rs;
+            O.diag_out[J] = d;
+            const double l1 = fabs(d) + offabs;
+            O.l1_out[J] = l1 > 0 ? 1.0 / l1 : 0.0;
+        }
+    }
+    row_sync<T>();
+}
+
+// Rows of up to kGrWarpCap terms, one warp each.
+template <bool TWO>
 __global__ void __launch_bounds__(kGrWarps * 32) k_gather_rows(int nrows, RowSrc S, RowMat B, GatherOut O) {
     extern __shared__ __align__(16) unsigned char gr_sm[];
+    __shared__ int ssrc[kGrWarps][32], spre[kGrWarps][32];
+    __shared__ double sw[kGrWarps][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const bool two = B.val2 != nullptr;
-    uint64_t* K = reinterpret_cast<uint64_t*>(gr_sm) + warp * kGrCap;
-    double* V = reinterpret_cast<double*>(gr_sm) + (kGrWarps + warp) * kGrCap;
-    double* V2 = two ? reinterpret_cast<double*>(gr_sm) + (2 * kGrWarps + warp) * kGrCap : nullptr;
+    uint64_t* K = reinterpret_cast<uint64_t*>(gr_sm) + warp * kGrWarpCap;
+    double* V = reinterpret_cast<double*>(gr_sm) + (kGrWarps + warp) * kGrWarpCap;
+    double* V2 = TWO ? reinterpret_cast<double*>(gr_sm) + (2 * kGrWarps + warp) * kGrWarpCap : nullptr;
     for (int J = blockIdx.x * kGrWarps + warp; J < nrows; J += gridDim.x * kGrWarps) {
-        int cnt = 0;
-        double rs = 0;
-        const int ns = src_count(S, J);
-        for (int t = 0; t < ns; t++) {
-            int s;
-            double w;
-            src_get(S, J, t, s, w);
-            if (O.rsv && lane == 0) rs += w * O.rsv[s];
-            const int L = mat_len(B, s);
-            for (int k0 = 0; k0 < L; k0 += 32) {
-                const int k = k0 + lane;
-                int c = 0;
-                double x = 0, x2 = 0;
-                bool keep = false;
-                if (k < L) {
-                    mat_get(B, s, k, c, x, x2);
-                    keep = !(O.skip_diag && c == J);
-                }
-                const unsigned bal = __ballot_sync(0xffffffffu, keep);
-                const int pos = cnt + __popc(bal & ((1u << lane) - 1u));
-                if (keep && pos < kGrCap) {
-                    K[pos] = ((uint64_t)(uint32_t)c << 32) | (uint32_t)pos;
-                    V[pos] = w * x;
-                    if (two) V2[pos] = w * x2;
-                }
-                cnt += __popc(bal);
-            }
-        }
-        if (cnt > kGrCap) {
-            if (lane == 0) O.longr[atomicAdd(O.nlong, 1)] = J;
-            __syncwarp();
-            continue;
-        }
-        int P = 1;
-        while (P < cnt) P <<= 1;
-        for (int i = cnt + lane; i < P; i += 32) K[i] = ~0ull;
-        __syncwarp();
-        for (int size = 2; size <= P; size <<= 1)
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                for (int i = lane; i < P; i += 32) {
-                    const int j = i ^ stride;
-                    if (j > i) {
-                        const bool up = (i & size) == 0;
-                        const uint64_t ki = K[i], kj = K[j];
-                        if ((ki > kj) == up) {
-                            K[i] = kj;
-                            K[j] = ki;
-                        }
-                    }
-                }
-                __syncwarp();
-            }
-        if (lane == 0) gather_reduce(J, cnt, K, V, V2, rs, O, O.seg[J]);
-        __syncwarp();
+        if (O.seg[J + 1] - O.seg[J] > kGrWarpCap) continue;
+        gather_row<32, TWO>(J, S, B, O, K, V, V2, lane, ssrc[warp], sw[warp], spre[warp], nullptr, nullptr);
     }
 }
 
-// The rows k_gather_rows listed as too long: one thread each, gathered and Shell-sorted in
-// the global scratch at the row's segment (same keys, so the same sums as the warp path).
-__global__ void k_gather_rows_long(RowSrc S, RowMat B, GatherOut O) {
-    const int nl = *O.nlong;
-    const bool two = B.val2 != nullptr;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nl; q += gridDim.x * blockDim.x) {
-        const int J = O.longr[q];
-        const int o = O.seg[J];
-        uint64_t* K = O.gkey + o;
-        double* V = O.gv + o;
-        double* V2 = two ? O.gv2 + o : nullptr;
-        int cnt = 0;
-        double rs = 0;
-        const int ns = src_count(S, J);
-        for (int t = 0; t < ns; t++) {
-            int s;
-            double w;
-            src_get(S, J, t, s, w);
-            if (O.rsv) rs += w * O.rsv[s];
-            const int L = mat_len(B, s);
-            for (int k = 0; k < L; k++) {
-                int c;
-                double x, x2;
-                mat_get(B, s, k, c, x, x2);
-                if (O.skip_diag && c == J) continue;
-                K[cnt] = ((uint64_t)(uint32_t)c << 32) | (uint32_t)cnt;
-                V[cnt] = w * x;
-                if (two) V2[cnt] = w * x2;
-                cnt++;
-            }
+// The listed rows of one tier, one CTA of T threads each: terms in shared memory (CAP > 0) or in
+// the row's segment of the global scratch (CAP == 0).
+template <int T, int CAP, bool TWO>
+__global__ void __launch_bounds__(T) k_gather_rows_cta(int tier, int nrows, RowSrc S, RowMat B, GatherOut O) {
+    extern __shared__ __align__(16) unsigned char gr_sm[];
+    __shared__ int ssrc[T], spre[T], wsi[T / 32];
+    __shared__ double sw[T], wsd[T / 32];
+    const int n = O.nlist[tier];
+    for (int q = blockIdx.x; q < n; q += gridDim.x) {
+        const int J = O.list[(size_t)tier * nrows + q];
+        uint64_t* K;
+        double *V, *V2;
+        if constexpr (CAP > 0) {
+            K = reinterpret_cast<uint64_t*>(gr_sm);
+            V = reinterpret_cast<double*>(K + CAP);
+            V2 = TWO ? V + CAP : nullptr;
+        } else {
+            const int o = O.seg[J];
+            K = O.gkey + o;
+            V = O.gv + o;
+            V2 = TWO ? O.gv2 + o : nullptr;
         }
-        int gap = 1;
-        while (gap * 9 / 4 + 1 < cnt) gap = gap * 9 / 4 + 1;
-        for (;; gap = max(1, (gap - 1) * 4 / 9)) {  // ..., 2, 1: the last pass is insertion sort
-            for (int i = gap; i < cnt; i++) {
-                const uint64_t key = K[i];
-                int j = i;
-                while (j >= gap && K[j - gap] > key) {
-                    K[j] = K[j - gap];
-                    j -= gap;
-                }
-                K[j] = key;
-            }
-            if (gap == 1) break;
-        }
-        gather_reduce(J, cnt, K, V, V2, rs, O, o);
+        gather_row<T, TWO>(J, S, B, O, K, V, V2, threadIdx.x, ssrc, sw, spre, wsi, wsd);
     }
 }
 
-__global__ void k_gather_copy(int nrows, const int32_t* __restrict__ seg, const int32_t* __restrict__ ulen, const int32_t* __restrict__ rp,
-                              const uint64_t* __restrict__ okey, const double* __restrict__ ov, const double* __restrict__ ov2,
-                              int32_t* __restrict__ col, double* __restrict__ val, double* __restrict__ val2) {
-    for (int J = blockIdx.x * blockDim.x + threadIdx.x; J < nrows; J += gridDim.x * blockDim.x) {
-        const int o = seg[J], d = rp[J];
-        for (int i = 0; i < ulen[J]; i++) {
-            col[d + i] = (int32_t)okey[o + i];
+// Segments to compact CSR rows, `lanes` threads per row.
+__global__ void k_gather_copy(int nrows, int lanes, const int32_t* __restrict__ seg, const int32_t* __restrict__ ulen,
+                              const int32_t* __restrict__ rp, const int32_t* __restrict__ ocol, const double* __restrict__ ov,
+                              const double* __restrict__ ov2, int32_t* __restrict__ col, double* __restrict__ val, double* __restrict__ val2) {
+    const RowLanes g = row_lanes(lanes);
+    for (int J = g.first; J < nrows; J += g.step) {
+        const int o = seg[J], d = rp[J], n = ulen[J];
+        for (int i = g.lane; i < n; i += lanes) {
+            col[d + i] = ocol[o + i];
             val[d + i] = ov[o + i];
             if (val2) val2[d + i] = ov2[o + i];
         }
@@ -1995,9 +1960,29 @@ __global__ void k_col_place(int n, const int32_t* __restrict__ rp, const int32_t
         }
 }
 
-__global__ void k_seg_sort(int nc, const int32_t* __restrict__ ptr, int32_t* __restrict__ idx, double* __restrict__ val) {
-    for (int J = blockIdx.x * blockDim.x + threadIdx.x; J < nc; J += gridDim.x * blockDim.x) {
-        const int b = ptr[J], e = ptr[J + 1];
+// One warp per column; a column of more than kGrWarpCap rows by one thread in place.
+__global__ void __launch_bounds__(kGrWarps * 32) k_seg_sort(int nc, const int32_t* __restrict__ ptr, int32_t* __restrict__ idx,
+                                                            double* __restrict__ val) {
+    __shared__ uint64_t sk[kGrWarps][kGrWarpCap];
+    __shared__ double sv[kGrWarps][kGrWarpCap];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int J = blockIdx.x * kGrWarps + warp; J < nc; J += gridDim.x * kGrWarps) {
+        const int b = ptr[J], e = ptr[J + 1], n = e - b;
+        if (n <= kGrWarpCap) {
+            for (int i = lane; i < n; i += 32) {
+                sk[warp][i] = ((uint64_t)(uint32_t)idx[b + i] << 32) | (uint32_t)i;
+                sv[warp][i] = val[b + i];
+            }
+            __syncwarp();
+            row_sort<32>(sk[warp], n, lane);
+            for (int i = lane; i < n; i += 32) {
+                idx[b + i] = (int32_t)(sk[warp][i] >> 32);
+                val[b + i] = sv[warp][(uint32_t)sk[warp][i]];
+            }
+            __syncwarp();
+            continue;
+        }
+        if (lane != 0) continue;
         for (int i = b + 1; i < e; i++) {
             const int x = idx[i];
             const double y = val[i];
@@ -2030,94 +2015,122 @@ __global__ void k_sa_v(int n, const int32_t* __restrict__ rp, const int32_t* __r
 
 // Fused restriction rows of the smoothed level: row J = Q^T row J on r_1 (columns < n), then
 // -(Q^T A_1) row J on z_1 (columns n + c).
-__global__ void k_rr_fill_sa(int nc, int n, const int32_t* __restrict__ qtp, const int32_t* __restrict__ qti, const double* __restrict__ qtv,
+__global__ void k_rr_fill_sa(int nc, int n, int lanes, const int32_t* __restrict__ qtp, const int32_t* __restrict__ qti, const double* __restrict__ qtv,
                              const int32_t* __restrict__ ap, const int32_t* __restrict__ ac, const double* __restrict__ av,
                              int32_t* __restrict__ rr_ptr, int32_t* __restrict__ rr_col, double* __restrict__ rr_val) {
-    for (int J = blockIdx.x * blockDim.x + threadIdx.x; J < nc; J += gridDim.x * blockDim.x) {
-        int e = qtp[J] + ap[J];
-        rr_ptr[J] = e;
-        if (J == nc - 1) rr_ptr[nc] = qtp[nc] + ap[nc];
-        for (int k = qtp[J]; k < qtp[J + 1]; k++, e++) {
-            rr_col[e] = qti[k];
-            rr_val[e] = qtv[k];
+    const RowLanes g = row_lanes(lanes);
+    for (int J = g.first; J < nc; J += g.step) {
+        const int q = qtp[J], nq = qtp[J + 1] - q, a = ap[J], na = ap[J + 1] - a, e = q + a;
+        if (g.lane == 0) {
+            rr_ptr[J] = e;
+            if (J == nc - 1) rr_ptr[nc] = qtp[nc] + ap[nc];
         }
-        for (int k = ap[J]; k < ap[J + 1]; k++, e++) {
-            rr_col[e] = n + ac[k];
-            rr_val[e] = -av[k];
+        for (int k = g.lane; k < nq; k += lanes) {
+            rr_col[e + k] = qti[q + k];
+            rr_val[e + k] = qtv[q + k];
+        }
+        for (int k = g.lane; k < na; k += lanes) {
+            rr_col[e + nq + k] = n + ac[a + k];
+            rr_val[e + nq + k] = -av[a + k];
         }
     }
 }
 
 // Fused prolongation-smoother rows of the smoothed level: row I = A_1 row I with its diagonal
 // on z_1, then A_1 (Q + w P) row I on zc (columns n + J).
-__global__ void k_pq_fill_sa(int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ v,
+__global__ void k_pq_fill_sa(int n, int lanes, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ v,
                              const double* __restrict__ diag, const int32_t* __restrict__ wp, const int32_t* __restrict__ wc,
                              const double* __restrict__ wv, int32_t* __restrict__ pq_ptr, int32_t* __restrict__ pq_col,
                              double* __restrict__ pq_val) {
-    for (int I = blockIdx.x * blockDim.x + threadIdx.x; I < n; I += gridDim.x * blockDim.x) {
-        int e = rp[I] + I + wp[I];
-        pq_ptr[I] = e;
-        if (I == n - 1) pq_ptr[n] = rp[n] + n + wp[n];
-        pq_col[e] = I;
-        pq_val[e] = diag[I];
-        e++;
-        for (int k = rp[I]; k < rp[I + 1]; k++, e++) {
-            pq_col[e] = ci[k];
-            pq_val[e] = v[k];
+    const RowLanes g = row_lanes(lanes);
+    for (int I = g.first; I < n; I += g.step) {
+        const int b = rp[I], nb = rp[I + 1] - b, w = wp[I], nw = wp[I + 1] - w, e = b + I + w;
+        if (g.lane == 0) {
+            pq_ptr[I] = e;
+            if (I == n - 1) pq_ptr[n] = rp[n] + n + wp[n];
+            pq_col[e] = I;
+            pq_val[e] = diag[I];
         }
-        for (int k = wp[I]; k < wp[I + 1]; k++, e++) {
-            pq_col[e] = n + wc[k];
-            pq_val[e] = wv[k];
+        for (int k = g.lane; k < nb; k += lanes) {
+            pq_col[e + 1 + k] = ci[b + k];
+            pq_val[e + 1 + k] = v[b + k];
+        }
+        for (int k = g.lane; k < nw; k += lanes) {
+            pq_col[e + 1 + nb + k] = n + wc[w + k];
+            pq_val[e + 1 + nb + k] = wv[w + k];
         }
     }
 }
 
-// One row-gather product: the compacted CSR (optr, ocol, oval[, oval2]) of nrows rows, its
-// arrays sized by the candidate-term count (one host read), which is returned (>= entries).
-long long gather_product(MgWork& g, int nrows, const RowSrc& S, const RowMat& B, bool skip_diag, const double* rsv, double* rs_out,
-                         double* diag_out, double* l1_out, DBuf<int32_t>& optr, DBuf<int32_t>& ocol, DBuf<double>& oval,
-                         DBuf<double>* oval2, cudaStream_t s, int64_t& launches) {
-    MgWork::Smoothed& w = g.sa;
-    w.seg.ensure(nrows + 1);
-    k_gather_len<<<grid_for(nrows), 256, 0, s>>>(nrows, S, B, w.seg.get());
-    launches++;
-    scan_small(w.seg.get(), w.seg.get(), nrows + 1, g.total.get(), g, s, launches);
-    int cand = 0;
-    CICY_CUDA(cudaMemcpyAsync(&cand, g.total.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
-    CICY_CUDA(cudaStreamSynchronize(s));
-    const size_t cap = (size_t)std::max(cand, 1);
-    const bool two = B.val2 != nullptr;
-    w.gkey.ensure(cap);
-    w.gv.ensure(cap);
-    w.okey.ensure(cap);
-    w.ov.ensure(cap);
-    if (two) {
-        w.gv2.ensure(cap);
-        w.ov2.ensure(cap);
-    }
-    w.ulen.ensure(nrows + 1);
-    w.longr.ensure(nrows + 1);
-    CICY_CUDA(cudaMemsetAsync(g.total.get() + 1, 0, sizeof(int32_t), s));
-    CICY_CUDA(cudaMemsetAsync(w.ulen.get() + nrows, 0, sizeof(int32_t), s));
-    const GatherOut O{w.seg.get(),  w.gkey.get(), w.gv.get(),  two ? w.gv2.get() : nullptr, w.okey.get(), w.ov.get(),
-                      two ? w.ov2.get() : nullptr, w.ulen.get(), w.longr.get(), g.total.get() + 1, skip_diag ? 1 : 0,
-                      rsv, rs_out, diag_out, l1_out};
-    const int smem = (int)(sizeof(double) * kGrWarps * kGrCap * (two ? 3 : 2));
+template <bool TWO>
+void launch_gather(int nrows, const RowSrc& S, const RowMat& B, const GatherOut& O, bool global_tier, cudaStream_t s, int64_t& launches) {
+    constexpr int kSets = TWO ? 3 : 2;
+    constexpr int warp_sm = (int)sizeof(double) * kGrWarps * kGrWarpCap * kSets;
+    constexpr int mid_sm = (int)sizeof(double) * kGrMidCap * kSets, big_sm = (int)sizeof(double) * kGrBigCap * kSets;
     static bool attr = false;
     if (!attr) {
-        CICY_CUDA(cudaFuncSetAttribute(k_gather_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(double) * kGrWarps * kGrCap * 3)));
+        CICY_CUDA(cudaFuncSetAttribute(k_gather_rows<TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, warp_sm));
+        CICY_CUDA(cudaFuncSetAttribute(k_gather_rows_cta<kGrMidThreads, kGrMidCap, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, mid_sm));
+        CICY_CUDA(cudaFuncSetAttribute(k_gather_rows_cta<kGrBigThreads, kGrBigCap, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, big_sm));
         attr = true;
     }
-    k_gather_rows<<<grid_for((long long)nrows * 32, kGrWarps * 32), kGrWarps * 32, smem, s>>>(nrows, S, B, O);
-    k_gather_rows_long<<<grid_for(nrows, 128), 128, 0, s>>>(S, B, O);
+    // grids: the CTAs that are resident at once (4 to 6 of the small, 1 of the large CTAs per SM); lists are shared out by stride
+    k_gather_rows<TWO><<<grid_for((long long)nrows * 32, kGrWarps * 32), kGrWarps * 32, warp_sm, s>>>(nrows, S, B, O);
+    k_gather_rows_cta<kGrMidThreads, kGrMidCap, TWO><<<std::min(nrows, 148 * 6), kGrMidThreads, mid_sm, s>>>(0, nrows, S, B, O);
+    k_gather_rows_cta<kGrBigThreads, kGrBigCap, TWO><<<std::min(nrows, 148), kGrBigThreads, big_sm, s>>>(1, nrows, S, B, O);
+    launches += 3;
+    if (global_tier) {
+        k_gather_rows_cta<kGrBigThreads, 0, TWO><<<std::min(nrows, 148), kGrBigThreads, 0, s>>>(2, nrows, S, B, O);
+        launches++;
+    }
+}
+
+// One row-gather product: the compacted CSR (optr, ocol, oval[, oval2]) of nrows rows.  Its arrays
+// are sized by the number of candidate terms, which is returned (>= entries): `cand`, an upper
+// bound known to the caller, or (-1) read from the device.
+long long gather_product(MgWork& g, int nrows, const RowSrc& S, const RowMat& B, bool skip_diag, const double* rsv, double* rs_out,
+                         double* diag_out, double* l1_out, long long cand, int lanes, DBuf<int32_t>& optr, DBuf<int32_t>& ocol,
+                         DBuf<double>& oval, DBuf<double>* oval2, cudaStream_t s, int64_t& launches) {
+    MgWork::Smoothed& w = g.sa;
+    w.seg.ensure(nrows + 1);
+    w.longr.ensure((size_t)kGrTiers * nrows + 1);
+    int32_t* nlist = g.total.get() + 1;
+    CICY_CUDA(cudaMemsetAsync(nlist, 0, sizeof(int32_t) * kGrTiers, s));
+    k_gather_len<<<grid_for(8LL * nrows), 256, 0, s>>>(nrows, 8, S, B, w.seg.get(), w.longr.get(), nlist);
+    launches++;
+    scan_small(w.seg.get(), w.seg.get(), nrows + 1, g.total.get(), g, s, launches);
+    bool global_tier = cand > kGrBigCap;  // some row may have more terms than a CTA's shared memory holds
+    if (cand < 0) {
+        int h[1 + kGrTiers];
+        CICY_CUDA(cudaMemcpyAsync(h, g.total.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+        CICY_CUDA(cudaStreamSynchronize(s));
+        cand = h[0];
+        global_tier = h[kGrTiers] > 0;
+    }
+    const size_t cap = (size_t)std::max<long long>(cand, 1);
+    const bool two = B.val2 != nullptr;
+    w.ocol.ensure(cap);
+    w.ov.ensure(cap);
+    if (two) w.ov2.ensure(cap);
+    if (global_tier) {
+        w.gkey.ensure(cap);
+        w.gv.ensure(cap);
+        if (two) w.gv2.ensure(cap);
+    }
+    w.ulen.ensure(nrows + 1);
+    const GatherOut O{w.seg.get(), w.gkey.get(), w.gv.get(), w.gv2.get(), w.ocol.get(), w.ov.get(), two ? w.ov2.get() : nullptr, w.ulen.get(),
+                      w.longr.get(), nlist, skip_diag ? 1 : 0, rsv, rs_out, diag_out, l1_out};
+    if (two) launch_gather<true>(nrows, S, B, O, global_tier, s, launches);
+    else launch_gather<false>(nrows, S, B, O, global_tier, s, launches);
     optr.ensure(nrows + 1);
     scan_small(w.ulen.get(), optr.get(), nrows + 1, nullptr, g, s, launches);
     ocol.ensure(cap);
     oval.ensure(cap);
     if (two) oval2->ensure(cap);
-    k_gather_copy<<<grid_for(nrows), 256, 0, s>>>(nrows, w.seg.get(), w.ulen.get(), optr.get(), w.okey.get(), w.ov.get(),
-                                                  two ? w.ov2.get() : nullptr, ocol.get(), oval.get(), two ? oval2->get() : nullptr);
-    launches += 3;
+    k_gather_copy<<<grid_for((long long)nrows * lanes), 256, 0, s>>>(nrows, lanes, w.seg.get(), w.ulen.get(), optr.get(), w.ocol.get(),
+                                                                     w.ov.get(), two ? w.ov2.get() : nullptr, ocol.get(), oval.get(),
+                                                                     two ? oval2->get() : nullptr);
+    launches++;
     CICY_LAUNCH_CHECK();
     return cand;
 }
@@ -2134,7 +2147,8 @@ void coarsen_smoothed(MgWork& g, int nc, cudaStream_t s, int64_t& launches) {
     const RowMat a1{F.rp_ptr, F.ci_ptr, F.val_ptr, F.diag.get(), nullptr, nullptr, nullptr};
     const RowMat a1_agg{F.rp_ptr, F.ci_ptr, F.val_ptr, F.diag.get(), nullptr, nullptr, F.agg.get()};
     // T = A_1 P, then Q and Q + w P on its pattern
-    const long long nt = gather_product(g, n, one, a1_agg, false, nullptr, nullptr, nullptr, nullptr, w.tp, w.tc, w.tv, nullptr, s, launches);
+    const long long nt = gather_product(g, n, one, a1_agg, false, nullptr, nullptr, nullptr, nullptr, (long long)F.nnz + n, 8, w.tp, w.tc, w.tv,
+                                        nullptr, s, launches);
     w.qv.ensure(nt);
     w.qpv.ensure(nt);
     k_sa_q<<<grid_for(n), 256, 0, s>>>(n, w.tp.get(), w.tc.get(), w.tv.get(), F.agg.get(), F.l1inv.get(), w.qv.get(), w.qpv.get());
@@ -2148,14 +2162,14 @@ void coarsen_smoothed(MgWork& g, int nc, cudaStream_t s, int64_t& launches) {
     scan_small(g.flag.get(), w.qtp.get(), nc + 1, nullptr, g, s, launches);
     CICY_CUDA(cudaMemsetAsync(g.flag.get(), 0, sizeof(int32_t) * (nc + 1), s));
     k_col_place<<<grid_for(n), 256, 0, s>>>(n, w.tp.get(), w.tc.get(), w.qv.get(), w.qtp.get(), g.flag.get(), w.qti.get(), w.qtv.get());
-    k_seg_sort<<<grid_for(nc), 256, 0, s>>>(nc, w.qtp.get(), w.qti.get(), w.qtv.get());
+    k_seg_sort<<<grid_for((long long)nc * 32, kGrWarps * 32), kGrWarps * 32, 0, s>>>(nc, w.qtp.get(), w.qti.get(), w.qtv.get());
     launches += 4;
     const RowSrc qt_src{w.qtp.get(), w.qti.get(), w.qtv.get(), nullptr};
     // W = A_1 Q and A_1 (Q + w P)
     const RowMat q{w.tp.get(), w.tc.get(), w.qv.get(), nullptr, w.qpv.get(), nullptr, nullptr};
-    const long long nw = gather_product(g, n, a1_src, q, false, nullptr, nullptr, nullptr, nullptr, w.wp, w.wc, w.wv, &w.wpv, s, launches);
+    const long long nw = gather_product(g, n, a1_src, q, false, nullptr, nullptr, nullptr, nullptr, -1, 32, w.wp, w.wc, w.wv, &w.wpv, s, launches);
     // Q^T A_1 (the restriction rows' part on z_1)
-    const long long na = gather_product(g, nc, qt_src, a1, false, nullptr, nullptr, nullptr, nullptr, w.ap, w.ac, w.av, nullptr, s, launches);
+    const long long na = gather_product(g, nc, qt_src, a1, false, nullptr, nullptr, nullptr, nullptr, -1, 32, w.ap, w.ac, w.av, nullptr, s, launches);
     // A_2 = Q^T W off the diagonal; its diagonal from the row sums Q^T A_1 Q 1
     w.y.ensure(n);
     w.v.ensure(n);
@@ -2167,7 +2181,7 @@ void coarsen_smoothed(MgWork& g, int nc, cudaStream_t s, int64_t& launches) {
     G.diag.ensure(nc);
     G.l1inv.ensure(nc);
     const RowMat wm{w.wp.get(), w.wc.get(), w.wv.get(), nullptr, nullptr, nullptr, nullptr};
-    const long long n2 = gather_product(g, nc, qt_src, wm, true, w.v.get(), G.rs.get(), G.diag.get(), G.l1inv.get(), G.rp, G.ci, G.val,
+    const long long n2 = gather_product(g, nc, qt_src, wm, true, w.v.get(), G.rs.get(), G.diag.get(), G.l1inv.get(), -1, 32, G.rp, G.ci, G.val,
                                         nullptr, s, launches);
     G.nnz = (int)std::max<long long>(n2, 1);
     G.rp_ptr = G.rp.get();
@@ -2177,12 +2191,12 @@ void coarsen_smoothed(MgWork& g, int nc, cudaStream_t s, int64_t& launches) {
     F.rr_ptr.ensure(nc + 1);
     F.rr_col.ensure(std::max<long long>(nt + na, 1));
     F.rr_val.ensure(std::max<long long>(nt + na, 1));
-    k_rr_fill_sa<<<grid_for(nc), 256, 0, s>>>(nc, n, w.qtp.get(), w.qti.get(), w.qtv.get(), w.ap.get(), w.ac.get(), w.av.get(), F.rr_ptr.get(),
+    k_rr_fill_sa<<<grid_for(32LL * nc), 256, 0, s>>>(nc, n, 32, w.qtp.get(), w.qti.get(), w.qtv.get(), w.ap.get(), w.ac.get(), w.av.get(), F.rr_ptr.get(),
                                                F.rr_col.get(), F.rr_val.get());
     F.pq_ptr.ensure(n + 1);
     F.pq_col.ensure(std::max<long long>((long long)F.nnz + n + nw, 1));
     F.pq_val.ensure(std::max<long long>((long long)F.nnz + n + nw, 1));
-    k_pq_fill_sa<<<grid_for(n), 256, 0, s>>>(n, F.rp_ptr, F.ci_ptr, F.val_ptr, F.diag.get(), w.wp.get(), w.wc.get(), w.wpv.get(),
+    k_pq_fill_sa<<<grid_for(32LL * n), 256, 0, s>>>(n, 32, F.rp_ptr, F.ci_ptr, F.val_ptr, F.diag.get(), w.wp.get(), w.wc.get(), w.wpv.get(),
                                               F.pq_ptr.get(), F.pq_col.get(), F.pq_val.get());
     launches += 2;
     CICY_LAUNCH_CHECK();
@@ -2200,7 +2214,7 @@ void coarsen(MgWork& g, int l, int nc, cudaStream_t s, int64_t& launches) {
     }
     MgWork::Lvl& F = g.L[l];
     MgWork::Lvl& G = g.L[l + 1];
-    const int nf = F.n, nnz = F.nnz;
+    const int nf = F.n, nnz = F.nnz, lf = lanes_of(nnz, nf);
     F.mptr.ensure(nc + 1);
     F.midx.ensure(std::max(nf, 1));
     if (l == 0) {
@@ -2216,38 +2230,21 @@ void coarsen(MgWork& g, int l, int nc, cudaStream_t s, int64_t& launches) {
         k_member_sort<<<grid_for(nc), 256, 0, s>>>(nc, F.mptr.get(), F.midx.get());
         launches += 3;
     }
-    // lengths and offsets
-    g.pos.ensure(nc + 1);
-    g.head.ensure(nc + 1);
-    g.uidx.ensure(nc + 1);
-    if (l >= 1) F.ra_ptr.ensure(nc + 1);
-    k_agg_lengths<<<grid_for(nc), 256, 0, s>>>(nc, F.mptr.get(), F.midx.get(), F.rp_ptr, g.pos.get(), l >= 1 ? F.ra_ptr.get() : nullptr);
-    launches++;
-    scan_small(g.pos.get(), g.pos.get(), nc + 1, nullptr, g, s, launches);  // seg_off
+    if (l >= 1) {
+        F.ra_ptr.ensure(nc + 1);
+        k_ra_lengths<<<grid_for(nc), 256, 0, s>>>(nc, F.mptr.get(), F.midx.get(), F.rp_ptr, F.ra_ptr.get());
+        launches++;
+    }
     // coarse rows
-    g.keys.ensure(std::max(nnz, 1));
-    g.sval.ensure(std::max(nnz, 1));
     G.n = nc;
-    G.nnz = nnz;  // capacity bound
-    G.rp.ensure(nc + 1);
-    G.ci.ensure(std::max(nnz, 1));
-    G.val.ensure(std::max(nnz, 1));
+    G.nnz = nnz;  // upper bound (build_mg_hierarchy reads the length)
     G.rs.ensure(nc);
     G.diag.ensure(nc);
     G.l1inv.ensure(nc);
-    g.long_rows.ensure(nc + 1);
-    CICY_CUDA(cudaMemsetAsync(g.total.get() + 1, 0, sizeof(int32_t), s));
-    k_coarse_rows<<<grid_for((long long)nc * 32, kCrWarps * 32), kCrWarps * 32, 0, s>>>(
-        nc, F.mptr.get(), F.midx.get(), F.rp_ptr, F.ci_ptr, F.val_ptr, F.agg.get(), F.rs.get(), g.pos.get(), g.keys.get(), g.sval.get(),
-        g.head.get(), G.rs.get(), G.diag.get(), G.l1inv.get(), g.long_rows.get(), g.total.get() + 1);
-    k_coarse_rows_long<<<grid_for(nc, 128), 128, 0, s>>>(g.long_rows.get(), g.total.get() + 1, F.mptr.get(), F.midx.get(), F.rp_ptr,
-                                                       F.ci_ptr, F.val_ptr, F.agg.get(), F.rs.get(), g.pos.get(), g.keys.get(),
-                                                       g.sval.get(), g.head.get(), G.rs.get(), G.diag.get(), G.l1inv.get());
-    launches++;
-    scan_small(g.head.get(), G.rp.get(), nc + 1, nullptr, g, s, launches);
-    k_coarse_copy<<<grid_for(nc), 256, 0, s>>>(nc, g.pos.get(), g.head.get(), G.rp.get(), g.keys.get(), g.sval.get(), G.ci.get(),
-                                               G.val.get());
-    launches += 2;
+    const RowSrc members{F.mptr.get(), F.midx.get(), nullptr, nullptr};
+    const RowMat fine{F.rp_ptr, F.ci_ptr, F.val_ptr, nullptr, nullptr, nullptr, F.agg.get()};
+    gather_product(g, nc, members, fine, true, F.rs.get(), G.rs.get(), G.diag.get(), G.l1inv.get(), nnz, l >= 1 ? 32 : 8, G.rp, G.ci, G.val, nullptr,
+                   s, launches);
     G.rp_ptr = G.rp.get();
     G.ci_ptr = G.ci.get();
     G.val_ptr = G.val.get();
@@ -2258,36 +2255,36 @@ void coarsen(MgWork& g, int l, int nc, cudaStream_t s, int64_t& launches) {
         if (!g.fused) {
             F.ra_col.ensure(std::max(nnz + nf, 1));
             F.ra_val.ensure(std::max(nnz + nf, 1));
-            k_ra_fill<<<grid_for(nc), 256, 0, s>>>(nc, F.mptr.get(), F.midx.get(), F.rp_ptr, F.ci_ptr, F.val_ptr, F.diag.get(),
+            k_ra_fill<<<grid_for((long long)nc * lf), 256, 0, s>>>(nc, lf, F.mptr.get(), F.midx.get(), F.rp_ptr, F.ci_ptr, F.val_ptr, F.diag.get(),
                                                     F.ra_ptr.get(), F.ra_col.get(), F.ra_val.get());
             launches++;
         }
     }
     if (!g.fused || l == 0) {
         F.cagg.ensure(std::max(nnz, 1));
-        k_cagg_rows<<<grid_for(nf), 256, 0, s>>>(nf, F.rp_ptr, F.ci_ptr, F.agg.get(), F.cagg.get());
+        k_cagg<<<grid_for(nnz), 256, 0, s>>>(F.rp_ptr + nf, F.ci_ptr, F.agg.get(), F.cagg.get());
         launches++;
     }
     if (g.fused && l >= 1) {
         F.rr_ptr.ensure(nc + 1);
         F.rr_col.ensure(std::max(nnz + 2 * nf, 1));
         F.rr_val.ensure(std::max(nnz + 2 * nf, 1));
-        k_rr_fill<<<grid_for(nc), 256, 0, s>>>(nc, nf, F.mptr.get(), F.midx.get(), F.rp_ptr, F.ci_ptr, F.val_ptr, F.diag.get(), F.ra_ptr.get(),
+        k_rr_fill<<<grid_for((long long)nc * lf), 256, 0, s>>>(nc, nf, lf, F.mptr.get(), F.midx.get(), F.rp_ptr, F.ci_ptr, F.val_ptr, F.diag.get(), F.ra_ptr.get(),
                                                 F.rr_ptr.get(), F.rr_col.get(), F.rr_val.get());
         F.pq_ptr.ensure(nf + 1);
         F.pq_col.ensure(std::max(2 * (nnz + nf), 1));
         F.pq_val.ensure(std::max(2 * (nnz + nf), 1));
-        k_pq_fill<<<grid_for(nf), 256, 0, s>>>(nf, F.rp_ptr, F.ci_ptr, F.val_ptr, F.diag.get(), F.agg.get(), F.pq_ptr.get(),
+        k_pq_fill<<<grid_for((long long)nf * lf), 256, 0, s>>>(nf, lf, F.rp_ptr, F.ci_ptr, F.val_ptr, F.diag.get(), F.agg.get(), F.pq_ptr.get(),
                                                 F.pq_col.get(), F.pq_val.get());
         launches += 2;
     }
     CICY_LAUNCH_CHECK();
 }
 
-// Pairwise aggregates of level l; returns their number.
+// Pairwise aggregates of level l; returns their number and sets the level's entry count.
 int pairwise(MgWork& g, int l, cudaStream_t s, int64_t& launches) {
     MgWork::Lvl& F = g.L[l];
-    const int n = F.n;
+    const int n = F.n, ln = lanes_of(F.nnz, n), gl = grid_for((long long)n * ln);
     g.mate.ensure(n + 1);
     g.best.ensure(n + 1);
     g.rep.ensure(n + 1);
@@ -2296,12 +2293,12 @@ int pairwise(MgWork& g, int l, cudaStream_t s, int64_t& launches) {
     k_fill_neg<<<grid_for(n), 256, 0, s>>>(n, g.mate.get());
     launches++;
     for (int round = 0; round < 3; round++) {
-        k_strongest<<<grid_for(n), 256, 0, s>>>(n, 1, F.rp_ptr, F.ci_ptr, F.val_ptr, g.mate.get(), g.best.get());
+        k_strongest<<<gl, 256, 0, s>>>(n, ln, 1, F.rp_ptr, F.ci_ptr, F.val_ptr, g.mate.get(), g.best.get());
         k_handshake<<<grid_for(n), 256, 0, s>>>(n, g.best.get(), g.mate.get());
         launches += 2;
     }
     k_pair_rep<<<grid_for(n), 256, 0, s>>>(n, g.mate.get(), g.rep.get());
-    k_strongest<<<grid_for(n), 256, 0, s>>>(n, 0, F.rp_ptr, F.ci_ptr, F.val_ptr, g.mate.get(), g.best.get());
+    k_strongest<<<gl, 256, 0, s>>>(n, ln, 0, F.rp_ptr, F.ci_ptr, F.val_ptr, g.mate.get(), g.best.get());
     k_join<<<grid_for(n), 256, 0, s>>>(n, g.mate.get(), g.best.get(), g.rep.get());
     k_is_rep<<<grid_for(n), 256, 0, s>>>(n, g.rep.get(), g.flag.get());
     launches += 4;
@@ -2311,6 +2308,7 @@ int pairwise(MgWork& g, int l, cudaStream_t s, int64_t& launches) {
     launches++;
     int nc = 0;
     CICY_CUDA(cudaMemcpyAsync(&nc, g.total.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+    CICY_CUDA(cudaMemcpyAsync(&F.nnz, F.rp_ptr + n, sizeof(int), cudaMemcpyDeviceToHost, s));  // until here an upper bound
     CICY_CUDA(cudaStreamSynchronize(s));
     CICY_LAUNCH_CHECK();
     return nc;
@@ -2325,7 +2323,7 @@ void build_mg_hierarchy(SolverWork& w, const SolverSystem& sys, cudaStream_t s, 
     g.fused = fused;
     g.smooth = smooth;
     TraceSeq tr(s);
-    g.total.ensure(2);
+    g.total.ensure(1 + kGrTiers);
     if (g.L.empty()) g.L.resize(1);
     MgWork::Lvl& L0 = g.L[0];
     L0.n = n;
@@ -2363,7 +2361,7 @@ void build_mg_hierarchy(SolverWork& w, const SolverSystem& sys, cudaStream_t s, 
     if (Lc.n <= kMgDenseMax) {
         g.cinv.ensure((size_t)Lc.n * Lc.n);
         CICY_CUDA(cudaMemsetAsync(g.cinv.get(), 0, sizeof(double) * Lc.n * Lc.n, s));
-        k_dense_coarse<<<grid_for(Lc.n, 128), 128, 0, s>>>(Lc.n, Lc.rp.get(), Lc.ci.get(), Lc.val.get(), Lc.diag.get(), g.cinv.get());
+        k_dense_coarse<<<grid_for(32LL * Lc.n, 128), 128, 0, s>>>(Lc.n, 32, Lc.rp.get(), Lc.ci.get(), Lc.val.get(), Lc.diag.get(), g.cinv.get());
         const size_t smem = sizeof(double) * ((size_t)Lc.n * Lc.n + 2 * (size_t)Lc.n * kGjBlock + kGjBlock * (kGjBlock + 1) + kGjBlock);
         if (smem > 48 * 1024)
             CICY_CUDA(cudaFuncSetAttribute(k_gauss_jordan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -2386,7 +2384,7 @@ void build_mg_hierarchy(SolverWork& w, const SolverSystem& sys, cudaStream_t s, 
             err = g.gj_err.get();
         }
         CICY_CUDA(cudaMemsetAsync(g.cinv.get(), 0, sizeof(double) * nC * nC, s));
-        k_dense_coarse<<<grid_for(nC, 128), 128, 0, s>>>(nC, Lc.rp.get(), Lc.ci.get(), Lc.val.get(), Lc.diag.get(), g.cinv.get());
+        k_dense_coarse<<<grid_for(32LL * nC, 128), 128, 0, s>>>(nC, 32, Lc.rp.get(), Lc.ci.get(), Lc.val.get(), Lc.diag.get(), g.cinv.get());
         const int G = std::max(1, std::min(sms, nC));
         const int wmax = (nC + G - 1) / G;
         if (wmax > kGjgMaxStrip) throw Fail{CICY_E_INTERNAL, "multigrid: dense coarsest too large for this GPU"};
