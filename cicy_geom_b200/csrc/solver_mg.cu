@@ -1580,7 +1580,7 @@ __global__ void k_cagg(const int32_t* __restrict__ nnz, const int32_t* __restric
 // Smoothed level-1 prolongator (hierarchies of the clustered kernel).
 //
 // Why: with piecewise-constant aggregates below the chain level the V-cycle is weak on
-// the chain graph, whose junction conductances span five orders of magnitude.  Smoothing
+// a sparse chain graph (smoothing_pays), whose junction conductances span five orders of magnitude.  Smoothing
 // the first pairwise prolongator once, Q = (I - w D^-1 A_1) P with D the l1-Jacobi
 // diagonal and w = 4/3, takes a real-resistor pass of the 25k-CNT network from ~90 to
 // ~35 PCG iterations and its unit pass from 54 to 39.  Then A_2 = Q^T A_1 Q, the
@@ -2281,6 +2281,18 @@ void coarsen(MgWork& g, int l, int nc, cudaStream_t s, int64_t& launches) {
     CICY_LAUNCH_CHECK();
 }
 
+// Whether a chain graph of `rows` and `entries` takes the smoothed prolongator.  Smoothing a
+// level whose rows have d couplings gives the next level about d^2 couplings a row, so it pays
+// only on sparse chain graphs: whole path in ms, smoothed against piecewise constant, by couplings
+// per chain (unit and real pass): 2.3, 2.5: 20.7 / 29.2 (48.9k CNTs, 8 um); 2.4, 2.6: 12.7 / 12.9
+// (25k, 6 um); 2.8, 3.0: 11.5 / 12.5 (15.1k, 4.5 um); 3.2, 3.4: 13.7 / 12.2 (23.9k, 5 um); 3.8, 3.9:
+// 42.6 / 13.4 (16.3k, 4 um); 5.3, 5.4: 28.3 / 15.9 (24.4k, 4 um); 5.7, 5.8: 60.9 / 27.5 (47.7k, 5 um).
+// Small graphs are bound by the phases' latency, not by their entries: 6.3k chains of 3.5-3.7
+// couplings 9.1 / 8.4, 7.2k chains 8.9 / 8.9, but 8.5k chains of 3.9-4.1 couplings 10.8 / 9.2.
+bool smoothing_pays(int rows, int entries) {
+    return 10LL * entries < 31LL * rows || (rows <= 8192 && 10LL * entries < 37LL * rows);
+}
+
 // Pairwise aggregates of level l; returns their number and sets the level's entry count.
 int pairwise(MgWork& g, int l, cudaStream_t s, int64_t& launches) {
     MgWork::Lvl& F = g.L[l];
@@ -2353,6 +2365,7 @@ void build_mg_hierarchy(SolverWork& w, const SolverSystem& sys, cudaStream_t s, 
         if (g.L[C].n <= dense_cap || C + 1 >= kMgMaxLevels) break;
         const int nc2 = pairwise(g, C, s, launches);
         tr.mark("mg.pairwise");
+        if (C == 1) g.smooth = smooth && smoothing_pays(g.L[1].n, g.L[1].nnz);
         if (nc2 > 0.9 * g.L[C].n) break;
         nc = nc2;
     }
@@ -2451,6 +2464,16 @@ void build_mg_hierarchy(SolverWork& w, const SolverSystem& sys, cudaStream_t s, 
     CICY_CUDA(cudaStreamSynchronize(s));
     g.levels = C + 1;
     CICY_LAUNCH_CHECK();
+    if (trace_enabled())
+        for (int l = 0; l <= C; l++) {
+            int nz = 0, rr = 0, pq = 0;
+            if (g.L[l].rp_ptr) cudaMemcpy(&nz, g.L[l].rp_ptr + g.L[l].n, 4, cudaMemcpyDeviceToHost);
+            if (g.fused && l >= 1 && l < C) {
+                cudaMemcpy(&rr, g.L[l].rr_ptr.get() + g.L[l + 1].n, 4, cudaMemcpyDeviceToHost);
+                cudaMemcpy(&pq, g.L[l].pq_ptr.get() + g.L[l].n, 4, cudaMemcpyDeviceToHost);
+            }
+            std::fprintf(stderr, "[cicy] mg level %d rows %d entries %d restriction %d prolongation %d\n", l, g.L[l].n, nz, rr, pq);
+        }
 }
 
 bool mg_fused_path(int n, bool allow_cluster) { return !(allow_cluster && n <= kMgClusterMaxRows); }
