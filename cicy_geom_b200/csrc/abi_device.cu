@@ -69,7 +69,7 @@ cicy_status cicy_ctx_create(cicy_ctx** out, int device) {
         c.status.ensure(1);
         CICY_CUDA(cudaMemsetAsync(c.status.get(), 0, sizeof(int), c.stream));
         c.i32_scalar.ensure(8);
-        c.i64_scalar.ensure(8);
+        c.words.create();
     });
     if (s != CICY_OK) {
         delete ctx;

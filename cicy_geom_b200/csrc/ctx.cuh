@@ -18,6 +18,25 @@ struct GridGeom {
     long long total;
 };
 
+// Pinned host words the device writes totals to (mapped: the device uses the same address), so a
+// size is read by waiting for the stream instead of by a copy to pageable memory as well.
+// Registering a page costs about 2.5 ms, so contexts share pages of 32 slots (stage_clusters.cu);
+// a page is freed with its last slot, but for one that is kept for the next context.
+enum HostWord : int { W_READ = 0, W_STATUS = 1, W_NODES = 2, W_NNZ = 3, W_RESID = 4 /* two */, W_COUNT = 16 };
+int64_t* host_words_take();
+void host_words_return(int64_t* slot);
+struct HostWords {
+    int64_t* host = nullptr;
+    int64_t* dev = nullptr;
+    HostWords() = default;
+    HostWords(const HostWords&) = delete;
+    HostWords& operator=(const HostWords&) = delete;
+    void create() { host = dev = host_words_take(); }
+    ~HostWords() {
+        if (host) host_words_return(host);
+    }
+};
+
 // One assembled DEA system kept for copy-out and for the backbone/current steps.
 struct DeaSystem {
     int cluster = -1, pass = -2;  // pass -1: unit resistors; 0,1,2: real, along x,y,z
@@ -120,7 +139,7 @@ struct Ctx {
     DBuf<uint32_t> slot_q, slot_sorted;
     DBuf<int> status;      // device status word (DevErr)
     DBuf<int32_t> i32_scalar;  // small device scalars for totals
-    DBuf<int64_t> i64_scalar;
+    HostWords words;
 
     // ---- contacts / labels ----
     int n_raw = 0, n_uc = 0, n_labels = 0, n_junc = 0, n_perc = 0;
@@ -153,25 +172,26 @@ struct Ctx {
     std::vector<DeaSystem*> systems;
     std::vector<DeaSystem*> sys_pool;  // systems of earlier runs, reused
     DBuf<int32_t> lmm;         // node of each point in the current solve (-1 none)
-    DBuf<int32_t> cnt_nodes, cnt_node_base, cnt_fresh, claim;
+    DBuf<int32_t> cnt_fresh, claim, chain_cnt;
+    DBuf<int64_t> node_cnt, node_base;  // per CNT of the cluster: new nodes (low half), resistors (high half); their scan
     DBuf<int32_t> e_n1, e_n2, e_op;
     DBuf<double> e_g;
-    DBuf<int32_t> work_i32a, work_i32b, work_i32c;
-    DBuf<double> work_f64a;
+    // assembly by rows: resistors per free node, their keys and positions, the row's couplings and lengths
+    DBuf<int32_t> row_cnt, row_ptr, row_pos, row_col;
+    DBuf<uint64_t> row_key;
+    DBuf<double> row_val;
+    DBuf<int64_t> row_len, row_ofs;
+    DBuf<int32_t> work_i32a;
     RadixScratch rs;
     RadixScratch rs_side;  // sorts issued on `side`
     DBuf<int32_t> scan_tmp32;
     DBuf<int64_t> scan_tmp64;
     // CG scratch
     DBuf<int32_t> cg_rp, cg_ci;
-    DBuf<double> cg_val, cg_minv, cg_x, cg_r, cg_p, cg_q, cg_z, cg_w, cg_s, cg_part;
-    DBuf<unsigned int> barrier;
+    DBuf<double> cg_val, cg_x;
     DBuf<double> cg_scal;
-    DBuf<long long> cg_iters;
-    // assembly / backbone scratch
-    DBuf<uint64_t> dkey, stage_keys;
-    DBuf<uint32_t> dval;
-    DBuf<double> runval, vef, cur_out, bterm;
+    // backbone scratch
+    DBuf<double> vef, cur_out, bterm;
     DBuf<int32_t> bvalid;
     DBuf<int32_t> eb, ee, alive, alive_scan, tmp_list;
     DBuf<unsigned long long> imax;

@@ -8,6 +8,10 @@ namespace {
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
+// Up to this many tiles (4.2 M items) a scan takes two launches: its blocks add up the earlier
+// tiles' sums themselves (at most 8 KB each from L2) instead of waiting for a one-block launch
+// in between (3.2-5.5 us); beyond, the quadratic reads would cost more than that launch.
+constexpr int kScanTilesMax = 2048;
 
 template <class T>
 __device__ T block_exclusive_sum(T v, T* smem_warp, T& block_total) {
@@ -71,9 +75,22 @@ __global__ void k_scan_blocks(T* bsum, int nb, T* total) {
     if (threadIdx.x == 0 && total) *total = carry;
 }
 
-template <class T>
-__global__ void k_scan_apply(const T* in, T* out, int n, const T* __restrict__ bsum) {
+// kSums: bsum holds the tiles' sums and every block adds up those before its own (at most
+// kScanTilesMax of them, read from L2); else bsum is already scanned.
+template <class T, bool kSums>
+__global__ void k_scan_apply(const T* in, T* out, int n, const T* __restrict__ bsum, T* total) {
     __shared__ T sw[33];
+    __shared__ T before;
+    if constexpr (kSums) {
+        T a = 0, tot;
+        for (int i = threadIdx.x; i < (int)blockIdx.x; i += kScanThreads) a += bsum[i];
+        block_exclusive_sum<T>(a, sw, tot);
+        if (threadIdx.x == 0) before = tot;
+        __syncthreads();
+    } else {
+        if (threadIdx.x == 0) before = bsum[blockIdx.x];
+        __syncthreads();
+    }
     long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
     T v[kScanItems];
     T s = 0;
@@ -84,13 +101,14 @@ __global__ void k_scan_apply(const T* in, T* out, int n, const T* __restrict__ b
         s += v[i];
     }
     T tot;
-    T ex = block_exclusive_sum<T>(s, sw, tot) + bsum[blockIdx.x];
+    T ex = block_exclusive_sum<T>(s, sw, tot) + before;
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) {
         long long j = base + i;
         if (j < n) out[j] = ex;
         ex += v[i];
     }
+    if (kSums && total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = before + tot;
 }
 
 // Scans of at most kScanSmallMax items in one launch: each of 1,024 threads holds a contiguous
@@ -135,9 +153,14 @@ void exclusive_scan_impl(const T* in, T* out, int n, T* total, DBuf<T>& tmp, cud
     int nb = ceil_div(n, kScanTile);
     tmp.ensure(nb + 1);
     k_scan_reduce<T><<<nb, kScanThreads, 0, s>>>(in, n, tmp.get());
-    k_scan_blocks<T><<<1, 1024, 0, s>>>(tmp.get(), nb, total);
-    k_scan_apply<T><<<nb, kScanThreads, 0, s>>>(in, out, n, tmp.get());
-    launches += 3;
+    if (nb <= kScanTilesMax) {
+        k_scan_apply<T, true><<<nb, kScanThreads, 0, s>>>(in, out, n, tmp.get(), total);
+        launches += 2;
+    } else {
+        k_scan_blocks<T><<<1, 1024, 0, s>>>(tmp.get(), nb, total);
+        k_scan_apply<T, false><<<nb, kScanThreads, 0, s>>>(in, out, n, tmp.get(), total);
+        launches += 3;
+    }
     CICY_LAUNCH_CHECK();
 }
 

@@ -1484,41 +1484,6 @@ __global__ void __launch_bounds__(kSmThreads) k_mg_pcg_sm(MgArgs a, MgSmArgs sa)
     }
 }
 
-// Exclusive scan of n ints in one CTA (the setup's arrays are short enough):
-// each thread scans a contiguous chunk; out may alias in; *total gets the sum.
-__global__ void __launch_bounds__(1024) k_scan_single(const int32_t* in, int32_t* out, int n, int32_t* total) {
-    __shared__ int32_t part[1024];
-    const int t = threadIdx.x, T = blockDim.x;
-    const int ch = (n + T - 1) / T;
-    const int lo = min(n, t * ch), hi = min(n, lo + ch);
-    int32_t s = 0;
-    for (int i = lo; i < hi; i++) s += in[i];
-    part[t] = s;
-    __syncthreads();
-    for (int o = 1; o < T; o <<= 1) {  // Hillis-Steele inclusive scan of the chunk sums
-        const int32_t v = t >= o ? part[t - o] : 0;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
-    }
-    int32_t run = part[t] - s;
-    for (int i = lo; i < hi; i++) {
-        const int32_t v = in[i];
-        out[i] = run;
-        run += v;
-    }
-    if (t == T - 1 && total) *total = part[T - 1];
-}
-
-void scan_small(const int32_t* in, int32_t* out, int n, int32_t* total, MgWork& g, cudaStream_t s, int64_t& launches) {
-    if (n <= (1 << 20)) {
-        k_scan_single<<<1, 1024, 0, s>>>(in, out, n, total);
-        launches++;
-    } else {
-        exclusive_scan_i32(in, out, n, total, g.scan_tmp, s, launches);
-    }
-}
-
 // Members of level-0 aggregates (chain blocks: consecutive rows).
 __global__ void k_members_contig(int n, int nc, const int32_t* __restrict__ agg, int32_t* __restrict__ mptr, int32_t* __restrict__ midx) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -2098,7 +2063,7 @@ long long gather_product(MgWork& g, int nrows, const RowSrc& S, const RowMat& B,
     CICY_CUDA(cudaMemsetAsync(nlist, 0, sizeof(int32_t) * kGrTiers, s));
     k_gather_len<<<grid_for(8LL * nrows), 256, 0, s>>>(nrows, 8, S, B, w.seg.get(), w.longr.get(), nlist);
     launches++;
-    scan_small(w.seg.get(), w.seg.get(), nrows + 1, g.total.get(), g, s, launches);
+    exclusive_scan_i32(w.seg.get(), w.seg.get(), nrows + 1, g.total.get(), g.scan_tmp, s, launches);
     bool global_tier = cand > kGrBigCap;  // some row may have more terms than a CTA's shared memory holds
     if (cand < 0) {
         int h[1 + kGrTiers];
@@ -2123,7 +2088,7 @@ long long gather_product(MgWork& g, int nrows, const RowSrc& S, const RowMat& B,
     if (two) launch_gather<true>(nrows, S, B, O, global_tier, s, launches);
     else launch_gather<false>(nrows, S, B, O, global_tier, s, launches);
     optr.ensure(nrows + 1);
-    scan_small(w.ulen.get(), optr.get(), nrows + 1, nullptr, g, s, launches);
+    exclusive_scan_i32(w.ulen.get(), optr.get(), nrows + 1, nullptr, g.scan_tmp, s, launches);
     ocol.ensure(cap);
     oval.ensure(cap);
     if (two) oval2->ensure(cap);
@@ -2159,7 +2124,7 @@ void coarsen_smoothed(MgWork& g, int nc, cudaStream_t s, int64_t& launches) {
     g.flag.ensure(nc + 1);
     CICY_CUDA(cudaMemsetAsync(g.flag.get(), 0, sizeof(int32_t) * (nc + 1), s));
     k_col_count<<<grid_for(n), 256, 0, s>>>(n, w.tp.get(), w.tc.get(), g.flag.get());
-    scan_small(g.flag.get(), w.qtp.get(), nc + 1, nullptr, g, s, launches);
+    exclusive_scan_i32(g.flag.get(), w.qtp.get(), nc + 1, nullptr, g.scan_tmp, s, launches);
     CICY_CUDA(cudaMemsetAsync(g.flag.get(), 0, sizeof(int32_t) * (nc + 1), s));
     k_col_place<<<grid_for(n), 256, 0, s>>>(n, w.tp.get(), w.tc.get(), w.qv.get(), w.qtp.get(), g.flag.get(), w.qti.get(), w.qtv.get());
     k_seg_sort<<<grid_for((long long)nc * 32, kGrWarps * 32), kGrWarps * 32, 0, s>>>(nc, w.qtp.get(), w.qti.get(), w.qtv.get());
@@ -2224,7 +2189,7 @@ void coarsen(MgWork& g, int l, int nc, cudaStream_t s, int64_t& launches) {
         g.flag.ensure(nc + 1);
         CICY_CUDA(cudaMemsetAsync(g.flag.get(), 0, sizeof(int32_t) * (nc + 1), s));
         k_member_count<<<grid_for(nf), 256, 0, s>>>(nf, F.agg.get(), g.flag.get());
-        scan_small(g.flag.get(), F.mptr.get(), nc + 1, nullptr, g, s, launches);
+        exclusive_scan_i32(g.flag.get(), F.mptr.get(), nc + 1, nullptr, g.scan_tmp, s, launches);
         CICY_CUDA(cudaMemsetAsync(g.flag.get(), 0, sizeof(int32_t) * (nc + 1), s));
         k_member_place<<<grid_for(nf), 256, 0, s>>>(nf, F.agg.get(), F.mptr.get(), g.flag.get(), F.midx.get());
         k_member_sort<<<grid_for(nc), 256, 0, s>>>(nc, F.mptr.get(), F.midx.get());
@@ -2251,7 +2216,7 @@ void coarsen(MgWork& g, int l, int nc, cudaStream_t s, int64_t& launches) {
     // restriction rows of level l (l >= 1) and its column aggregates; the clustered kernel
     // (g.fused) reads the fused rows instead of P^T A_l and the coarse column aggregates
     if (l >= 1) {
-        scan_small(F.ra_ptr.get(), F.ra_ptr.get(), nc + 1, nullptr, g, s, launches);
+        exclusive_scan_i32(F.ra_ptr.get(), F.ra_ptr.get(), nc + 1, nullptr, g.scan_tmp, s, launches);
         if (!g.fused) {
             F.ra_col.ensure(std::max(nnz + nf, 1));
             F.ra_val.ensure(std::max(nnz + nf, 1));
@@ -2314,7 +2279,7 @@ int pairwise(MgWork& g, int l, cudaStream_t s, int64_t& launches) {
     k_join<<<grid_for(n), 256, 0, s>>>(n, g.mate.get(), g.best.get(), g.rep.get());
     k_is_rep<<<grid_for(n), 256, 0, s>>>(n, g.rep.get(), g.flag.get());
     launches += 4;
-    scan_small(g.flag.get(), g.pos.get(), n, g.total.get(), g, s, launches);
+    exclusive_scan_i32(g.flag.get(), g.pos.get(), n, g.total.get(), g.scan_tmp, s, launches);
     F.agg.ensure(n + 1);
     k_agg_ids<<<grid_for(n), 256, 0, s>>>(n, g.rep.get(), g.pos.get(), F.agg.get());
     launches++;

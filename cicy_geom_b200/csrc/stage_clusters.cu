@@ -2,6 +2,7 @@
 // labelling, junction compression, elements, percolation (device).
 #include <algorithm>
 #include <cmath>
+#include <mutex>
 
 #include "ctx.cuh"
 #include "trace.cuh"
@@ -444,17 +445,63 @@ Ctx::~Ctx() {
     delete hy;
 }
 
+namespace {
+struct WordPages {
+    static constexpr int kSlots = 32;
+    struct Page {
+        int64_t* p;
+        uint32_t used;
+    };
+    std::mutex m;
+    std::vector<Page> pages;
+};
+WordPages& word_pages() {
+    static WordPages* w = new WordPages;  // not destroyed: a context may outlive static objects
+    return *w;
+}
+}  // namespace
+
+int64_t* host_words_take() {
+    WordPages& w = word_pages();
+    std::lock_guard<std::mutex> lock(w.m);
+    for (auto& g : w.pages)
+        for (int k = 0; k < WordPages::kSlots; k++)
+            if (!(g.used >> k & 1)) {
+                g.used |= 1u << k;
+                return g.p + (size_t)k * W_COUNT;
+            }
+    w.pages.reserve(w.pages.size() + 1);
+    int64_t* p = nullptr;
+    CICY_CUDA(cudaHostAlloc(&p, sizeof(int64_t) * W_COUNT * WordPages::kSlots, cudaHostAllocMapped | cudaHostAllocPortable));
+    w.pages.push_back(WordPages::Page{p, 1u});
+    return p;
+}
+
+void host_words_return(int64_t* slot) {
+    WordPages& w = word_pages();
+    std::lock_guard<std::mutex> lock(w.m);
+    for (size_t i = 0; i < w.pages.size(); i++) {
+        WordPages::Page& g = w.pages[i];
+        if (slot < g.p || slot >= g.p + (size_t)W_COUNT * WordPages::kSlots) continue;
+        g.used &= ~(1u << ((slot - g.p) / W_COUNT));
+        if (!g.used && w.pages.size() > 1) {
+            cudaFreeHost(g.p);
+            w.pages.erase(w.pages.begin() + i);
+        }
+        return;
+    }
+}
+
 int32_t read_i32(Ctx& c, const int32_t* dptr) {
-    int32_t v = 0;
-    CICY_CUDA(cudaMemcpyAsync(&v, dptr, sizeof(v), cudaMemcpyDeviceToHost, c.stream));
+    CICY_CUDA(cudaMemcpyAsync(c.words.host + W_READ, dptr, sizeof(int32_t), cudaMemcpyDeviceToHost, c.stream));
     CICY_CUDA(cudaStreamSynchronize(c.stream));
-    return v;
+    return *reinterpret_cast<const int32_t*>(c.words.host + W_READ);
 }
 
 void check_status(Ctx& c, const char* where) {
-    int st = 0;
-    CICY_CUDA(cudaMemcpyAsync(&st, c.status.get(), sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    CICY_CUDA(cudaMemcpyAsync(c.words.host + W_STATUS, c.status.get(), sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     CICY_CUDA(cudaStreamSynchronize(c.stream));
+    const int st = *reinterpret_cast<const int*>(c.words.host + W_STATUS);
     if (st == DEV_OK) return;
     CICY_CUDA(cudaMemsetAsync(c.status.get(), 0, sizeof(int), c.stream));
     if (st == DEV_TIMEOUT) throw Fail{CICY_E_TIMEOUT, std::string(where) + ": a bounded device wait gave up"};
@@ -515,7 +562,6 @@ void upload_network(Ctx& c, const cicy_network& n) {
     c.bpts_idx.ensure(std::max(c.h_bpts_ptr[6], 1));
     c.status.ensure(1);
     c.i32_scalar.ensure(8);
-    c.i64_scalar.ensure(8);
     auto up = [&](void* d, const void* h, size_t bytes) {
         if (bytes) CICY_CUDA(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s));
     };

@@ -37,19 +37,31 @@ int boundaries_of_family(int family, int out[6]) {
     return len[family];
 }
 
-// Per-CNT element ranges of the cluster being solved: [eb, ee) into elem_idx.
+// Per-CNT element ranges of the cluster being solved: [eb, ee) into elem_idx (empty, with the
+// status set, when the CNT has no element), and its end points' claims reset.
 __global__ void k_cluster_ranges(int n, const int32_t* __restrict__ members, const int32_t* __restrict__ cur_lo,
-                                 const int32_t* __restrict__ cur_hi, int32_t* __restrict__ eb, int32_t* __restrict__ ee,
-                                 int* status) {
+                                 const int32_t* __restrict__ cur_hi, const int32_t* __restrict__ elem, int32_t* __restrict__ eb,
+                                 int32_t* __restrict__ ee, int32_t* __restrict__ claim, int* status) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int c = members[i];
         int lo = cur_lo[c], hi = cur_hi[c];
+        // LM_matrix_for_cnts: "There is a CNT with not enough points to form an element"
+        if (lo < 0 || hi - lo + 1 <= 1) {
+            atomicCAS(status, 0, (int)DEV_INPUT);
+            eb[i] = ee[i] = 0;
+            continue;
+        }
         eb[i] = lo;
         ee[i] = hi + 1;
-        // LM_matrix_for_cnts: "There is a CNT with not enough points to form an element"
-        if (lo < 0 || hi - lo + 1 <= 1) atomicCAS(status, 0, (int)DEV_INPUT);
+        claim[elem[lo]] = 0x7fffffff;
+        claim[elem[hi]] = 0x7fffffff;
     }
 }
+
+// Points of the prescribed faces: node k for face list k (a point on two of them belongs to the later one).
+struct FaceRuns {
+    int n, b[6], e[6];
+};
 
 __global__ void k_lmm_face(int b, int e, const int32_t* __restrict__ bpts, int node, int32_t* lmm) {
     for (int i = b + blockIdx.x * blockDim.x + threadIdx.x; i < e; i += gridDim.x * blockDim.x) lmm[bpts[i]] = node;
@@ -63,43 +75,52 @@ __global__ void k_lmm_face(int b, int e, const int32_t* __restrict__ bpts, int n
 // reuses it.  Here the CNTs run in parallel, so each shared end point is first
 // claimed by the smallest cluster position (claim[P] = min i), and only the
 // claimant counts and numbers it.
-__global__ void k_claim_init(int n, const int32_t* __restrict__ eb, const int32_t* __restrict__ ee, const int32_t* __restrict__ elem,
-                             int32_t* __restrict__ claim) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        claim[elem[eb[i]]] = 0x7fffffff;
-        claim[elem[ee[i] - 1]] = 0x7fffffff;
-    }
-}
-
 __global__ void k_claim(int n, const int32_t* __restrict__ eb, const int32_t* __restrict__ ee, const int32_t* __restrict__ elem,
-                        int32_t* __restrict__ claim) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+                        int32_t* __restrict__ claim, FaceRuns f, const int32_t* __restrict__ bpts, int32_t* __restrict__ lmm) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    for (int i = t; i < n; i += step) {
+        if (ee[i] <= eb[i]) continue;
         atomicMin(&claim[elem[eb[i]]], i);
         atomicMin(&claim[elem[ee[i] - 1]], i);
     }
+    for (int k = 0; k < f.n; k++)
+        for (int i = f.b[k] + t; i < f.e[k]; i += step) atomicMax(&lmm[bpts[i]], k);
 }
 
-// new[i]: bit 0 first point numbered by CNT i, bit 1 last point numbered by CNT i
+// Per CNT: new nodes (low half) and resistors between consecutive elements (high half; one when
+// both ends of a three-point element list lie on the same prescribed face), for one scan of both.
+// fresh[i]: bit 0 first point numbered by CNT i, bit 1 last point numbered by CNT i.
 __global__ void k_node_counts(int n, const int32_t* __restrict__ eb, const int32_t* __restrict__ ee,
                               const int32_t* __restrict__ elem, const int32_t* __restrict__ lmm, const int32_t* __restrict__ claim,
-                              int32_t* __restrict__ cnt, int32_t* __restrict__ fresh) {
+                              int64_t* __restrict__ cnt, int32_t* __restrict__ fresh) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int b = eb[i], e = ee[i];
         int m = e - b;
+        if (m < 2) {
+            cnt[i] = 0;
+            fresh[i] = 0;
+            continue;
+        }
         const int P0 = elem[b], P1 = elem[e - 1];
         const bool f0 = lmm[P0] < 0 && claim[P0] == i;
         const bool f1 = lmm[P1] < 0 && claim[P1] == i && P1 != P0;
-        cnt[i] = (f0 ? 1 : 0) + (m - 2) + (f1 ? 1 : 0);
+        const bool three = m == 3 && lmm[P0] >= 0 && lmm[P0] == lmm[P1];
+        cnt[i] = (int64_t)((f0 ? 1 : 0) + (m - 2) + (f1 ? 1 : 0)) | ((int64_t)(three ? 1 : m - 1) << 32);
         fresh[i] = (f0 ? 1 : 0) | (f1 ? 2 : 0);
     }
 }
 
 __global__ void k_node_assign(int n, int reserved, const int32_t* __restrict__ eb, const int32_t* __restrict__ ee,
-                              const int32_t* __restrict__ elem, const int32_t* __restrict__ base, const int32_t* __restrict__ fresh,
-                              int32_t* lmm) {
+                              const int32_t* __restrict__ elem, const int64_t* __restrict__ cnt, const int64_t* __restrict__ base,
+                              const int32_t* __restrict__ fresh, int32_t* lmm, int32_t* __restrict__ chain_start,
+                              int32_t* __restrict__ chain_len) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int b = eb[i], e = ee[i];
-        int node = reserved + base[i];
+        const int first = (int)(uint32_t)base[i];
+        // free nodes of each CNT are one consecutive range: the chains of the block preconditioner
+        chain_start[i] = first;
+        chain_len[i] = (int)(uint32_t)cnt[i];
+        int node = reserved + first;
         if (fresh[i] & 1) lmm[elem[b]] = node++;
         for (int k = b + 1; k < e - 1; k++) lmm[elem[k]] = node++;
         if (fresh[i] & 2) lmm[elem[e - 1]] = node++;
@@ -129,25 +150,36 @@ __device__ __forceinline__ double cnt_volume(int P1, int P2, double radius, cons
     return length * kPI * radius * radius;
 }
 
-__global__ void k_cnt_edge_counts(int n, const int32_t* __restrict__ eb, const int32_t* __restrict__ ee,
-                                  const int32_t* __restrict__ elem, const int32_t* __restrict__ lmm, int32_t* __restrict__ cnt) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int b = eb[i], m = ee[i] - b;
-        bool three = (m == 3) && lmm[elem[b]] == lmm[elem[b + 2]];
-        cnt[i] = three ? 1 : m - 1;
-    }
-}
-
-// Fill_2d_matrices_cnts + Three_points_in_element (Direct_Electrifying.cpp:489-608).
-__global__ void k_cnt_edges(int n, int r_flag, double rho, const int32_t* __restrict__ members, const int32_t* __restrict__ eb,
+// Fill_2d_matrices_cnts + Three_points_in_element (Direct_Electrifying.cpp:489-608), and, with
+// x0, Initial_guess_for_cnt_nodes (:1434-1470).  kEdgeLanes threads per CNT, one resistor each at
+// a time: a resistor's length is a serial sum over its points (upstream's order), and one thread
+// per CNT walked all of a CNT's ~100 points (both passes of the 25k-CNT network: 139 us, now 62 us).
+constexpr int kEdgeLanes = 8;
+struct GuessArgs {
+    double* x0;  // null: no initial guess
+    int axis;
+    double v_per_length, max_coord;
+};
+__global__ void k_cnt_edges(int n, int r_flag, int reserved, double rho, const int32_t* __restrict__ members, const int32_t* __restrict__ eb,
                             const int32_t* __restrict__ ee, const int32_t* __restrict__ elem, const int32_t* __restrict__ lmm,
-                            const int32_t* __restrict__ ofs, const double* __restrict__ radii, const double* __restrict__ x,
+                            const int64_t* __restrict__ base, const double* __restrict__ radii, const double* __restrict__ x,
                             const double* __restrict__ y, const double* __restrict__ z, int32_t* __restrict__ n1,
-                            int32_t* __restrict__ n2, int32_t* __restrict__ op, double* __restrict__ g) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int b = eb[i], m = ee[i] - b, o = ofs[i];
-        double r = radii[members[i]];
+                            int32_t* __restrict__ n2, int32_t* __restrict__ op, double* __restrict__ g, GuessArgs guess) {
+    const int lane = threadIdx.x % kEdgeLanes;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) / kEdgeLanes; i < n; i += gridDim.x * blockDim.x / kEdgeLanes) {
+        const int b = eb[i], m = ee[i] - b, o = (int)(base[i] >> 32);
+        if (m < 2) continue;
+        const double r = radii[members[i]];
+        if (guess.x0) {
+            for (int k = lane; k < m; k += kEdgeLanes) {
+                const int P = elem[b + k], node = lmm[P];
+                if (node < 2) continue;
+                const double c = guess.axis == 0 ? x[P] : guess.axis == 1 ? y[P] : z[P];
+                guess.x0[node - reserved] = guess.v_per_length * (guess.max_coord - c);
+            }
+        }
         if (m == 3 && lmm[elem[b]] == lmm[elem[b + 2]]) {
+            if (lane != 0) continue;
             double g1 = 1.0, g2 = 1.0;
             if (r_flag == 1) {
                 g1 = 1 / cnt_resistance(elem[b], elem[b + 1], r, rho, x, y, z);
@@ -159,7 +191,7 @@ __global__ void k_cnt_edges(int n, int r_flag, double rho, const int32_t* __rest
             g[o] = g1 + g2;
             continue;
         }
-        for (int k = 0; k < m - 1; k++) {
+        for (int k = lane; k < m - 1; k += kEdgeLanes) {
             int P1 = elem[b + k], P2 = elem[b + k + 1];
             double gi = r_flag ? 1 / cnt_resistance(P1, P2, r, rho, x, y, z) : 1.0;
             n1[o + k] = lmm[P1];
@@ -209,191 +241,140 @@ __global__ void k_junction_edges(int nj, int base, int r_flag, int reserved, int
     }
 }
 
-// Off-diagonal keys (row = max node, col = min node) and diagonal contributions.
-// Skipped edges get the key 1 << (2 bn) (off-diagonal) / 1 << bn (diagonal) and sort last.
-__global__ void k_edge_keys(int ne, int bn, const int32_t* __restrict__ n1, const int32_t* __restrict__ n2,
-                            const int32_t* __restrict__ op, uint64_t* __restrict__ okey, uint32_t* __restrict__ oval,
-                            uint64_t* __restrict__ dkey, uint32_t* __restrict__ dval) {
+// ---------------------------------------------------------------------------
+// Assembly by rows (Add_new_elements_to_2d_sparse_matrix, From_2d_to_1d_vectors,
+// Direct_Electrifying.cpp:1329-1394): every free node gets the list of its resistors by a
+// counting sort, orders the few it has by insertion and forms its own diagonal, right-hand side
+// and couplings, each in upstream's order.  A row has two to six resistors (a GNP point up to a
+// few hundred), so this replaces three radix sorts over all resistors (24 passes of five launches;
+// 0.48 + 0.30 ms per network of 25k CNTs) by seven launches that are bound by launch latency and
+// one pass over the resistors (0.07 ms).
+
+// Position of every resistor in the list of each of its free nodes (cnt zeroed before).
+__global__ void k_row_count(int ne, int reserved, const int32_t* __restrict__ n1, const int32_t* __restrict__ n2,
+                            const int32_t* __restrict__ op, int32_t* cnt, int32_t* __restrict__ pos) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += gridDim.x * blockDim.x) {
-        int a = n1[i], b = n2[i];
-        bool live = op[i] != OP_SKIP;
-        uint64_t hi = (uint64_t)max(a, b), lo = (uint64_t)min(a, b);
-        okey[i] = live ? ((hi << bn) | lo) : (1ull << (2 * bn));
-        oval[i] = (uint32_t)i;
-        dkey[2 * i] = live ? (uint64_t)a : (1ull << bn);
-        dval[2 * i] = (uint32_t)i;
-        dkey[2 * i + 1] = live ? (uint64_t)b : (1ull << bn);
-        dval[2 * i + 1] = (uint32_t)i;
+        if (op[i] == OP_SKIP) continue;
+        const int a = n1[i], b = n2[i];
+        if (a >= reserved) pos[2 * i] = atomicAdd(&cnt[a - reserved], 1);
+        if (b >= reserved && b != a) pos[2 * i + 1] = atomicAdd(&cnt[b - reserved], 1);
     }
 }
 
-// diagonal[node] += g in insertion order (Add_new_elements_to_2d_sparse_matrix et al.).
-// Only free nodes: the prescribed nodes' diagonal is dropped (From_2d_to_1d_vectors)
-// and their runs, one entry per boundary element, are the longest ones.
-__global__ void k_diag_reduce(int n2e, uint64_t skip, uint64_t reserved, const uint64_t* __restrict__ dkey, const uint32_t* __restrict__ dval,
-                              const double* __restrict__ g, double* __restrict__ diag_all) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n2e; i += gridDim.x * blockDim.x) {
-        uint64_t k = dkey[i];
-        if (k == skip || k < reserved) continue;
-        if (i > 0 && dkey[i - 1] == k) continue;
-        double s = 0;
-        for (int j = i; j < n2e && dkey[j] == k; j++) s += g[dval[j]];
-        diag_all[k] = s;
+// Row lists of (resistor << 32 | other node); unordered within a row.
+__global__ void k_row_place(int ne, int reserved, const int32_t* __restrict__ n1, const int32_t* __restrict__ n2,
+                            const int32_t* __restrict__ op, const int32_t* __restrict__ rptr, const int32_t* __restrict__ pos,
+                            uint64_t* __restrict__ key) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += gridDim.x * blockDim.x) {
+        if (op[i] == OP_SKIP) continue;
+        const int a = n1[i], b = n2[i];
+        if (a >= reserved) key[rptr[a - reserved] + pos[2 * i]] = ((uint64_t)(uint32_t)i << 32) | (uint32_t)b;
+        if (b >= reserved && b != a) key[rptr[b - reserved] + pos[2 * i + 1]] = ((uint64_t)(uint32_t)i << 32) | (uint32_t)a;
     }
 }
 
-// col_values[row][col]: overwrite / subtract in insertion order.
-__global__ void k_offdiag_reduce(int ne, uint64_t skip, const uint64_t* __restrict__ okey, const uint32_t* __restrict__ oval,
-                                 const int32_t* __restrict__ op, const double* __restrict__ g, int32_t* __restrict__ head,
-                                 double* __restrict__ runval) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += gridDim.x * blockDim.x) {
-        uint64_t k = okey[i];
-        bool h = (k != skip) && (i == 0 || okey[i - 1] != k);
-        head[i] = h ? 1 : 0;
-        if (!h) continue;
-        double v = 0;
-        for (int j = i; j < ne && okey[j] == k; j++) {
-            uint32_t e = oval[j];
-            if (op[e] == OP_OVERWRITE) v = -g[e];
-            else v = v - g[e];
+__device__ __forceinline__ void sort_short(uint64_t* k, int n) {  // Shell sort: insertion sort up to a few dozen keys
+    int gap = 1;
+    while (n > 32 && gap * 9 / 4 + 1 < n) gap = gap * 9 / 4 + 1;
+    for (;; gap = max(1, (gap - 1) * 4 / 9)) {
+        for (int i = gap; i < n; i++) {
+            const uint64_t v = k[i];
+            int j = i;
+            while (j >= gap && k[j - gap] > v) {
+                k[j] = k[j - gap];
+                j -= gap;
+            }
+            k[j] = v;
         }
-        runval[i] = v;
+        if (gap == 1) break;
     }
 }
 
-// From_2d_to_1d_vectors (Direct_Electrifying.cpp:1329-1394): split the unique
-// (row, col) entries of the free rows into the SSS lower block and the rhs.
-__global__ void k_sss_flags(int ne, int bn, int reserved, const uint64_t* __restrict__ okey, const int32_t* __restrict__ head,
-                            int32_t* __restrict__ lower_flag) {
-    const uint64_t mask = (1ull << bn) - 1;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += gridDim.x * blockDim.x) {
-        bool f = false;
-        if (head[i]) {
-            long long row = (long long)(okey[i] >> bn), col = (long long)(okey[i] & mask);
-            f = row >= reserved && col >= reserved;
+// One thread per free node r: diagonal (sum over its resistors in insertion order), then its
+// resistors by other node: the value of each coupling (overwrite / subtract in insertion order),
+// the right-hand side over the prescribed nodes ascending, R = R - K VEF, and the couplings to free
+// nodes compacted at the front of the row's segment (col, val).  len[r]: couplings below r (low half:
+// the SSS row) and entries of the full row with its diagonal (high half).
+constexpr int kRowLocal = 16;
+__global__ void k_row_build(int n, int reserved, const int32_t* __restrict__ rptr, uint64_t* __restrict__ key, const int32_t* __restrict__ op,
+                            const double* __restrict__ g, const double* __restrict__ vef, int32_t* __restrict__ col, double* __restrict__ val,
+                            int64_t* __restrict__ len, double* __restrict__ diag, double* __restrict__ b, int* status) {
+    uint64_t local[kRowLocal];
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+        const int s0 = rptr[r], L = rptr[r + 1] - s0;
+        const uint32_t self = (uint32_t)(r + reserved);
+        uint64_t* k = key + s0;
+        if (L <= kRowLocal) {
+            for (int i = 0; i < L; i++) local[i] = k[i];
+            k = local;
         }
-        lower_flag[i] = f ? 1 : 0;
-    }
-}
-
-__global__ void k_sss_fill(int ne, int bn, int reserved, const uint64_t* __restrict__ okey, const int32_t* __restrict__ lower_flag,
-                           const int32_t* __restrict__ lower_scan, const double* __restrict__ runval, int32_t* __restrict__ row_cnt,
-                           int32_t* __restrict__ col, double* __restrict__ val) {
-    const uint64_t mask = (1ull << bn) - 1;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += gridDim.x * blockDim.x) {
-        if (!lower_flag[i]) continue;
-        int row = (int)(okey[i] >> bn) - reserved, c = (int)(okey[i] & mask) - reserved;
-        int o = lower_scan[i];
-        col[o] = c;
-        val[o] = runval[i];
-        atomicAdd(&row_cnt[row], 1);
-    }
-}
-
-// rhs: R[i] = R[i] - K_ij * VEF[j] for reserved columns j, ascending j.
-__global__ void k_rhs(int ne, int bn, int reserved, const uint64_t* __restrict__ okey, const int32_t* __restrict__ head,
-                      const double* __restrict__ runval, const double* __restrict__ vef, double* __restrict__ b) {
-    const uint64_t mask = (1ull << bn) - 1;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += gridDim.x * blockDim.x) {
-        if (!head[i]) continue;
-        long long row = (long long)(okey[i] >> bn), col = (long long)(okey[i] & mask);
-        if (row < reserved || col >= reserved) continue;
-        // the first reserved-column entry of a row performs the row's ordered fold
-        bool first = true;
-        for (int j = i - 1; j >= 0; j--) {
-            if (!head[j]) continue;
-            long long r2 = (long long)(okey[j] >> bn);
-            if (r2 == row) first = false;
-            break;
+        sort_short(k, L);
+        double d = 0;
+        for (int i = 0; i < L; i++) {
+            const double gi = g[k[i] >> 32];
+            d += gi;
+            if ((uint32_t)k[i] == self) d += gi;
+            k[i] = (k[i] << 32) | (k[i] >> 32);
         }
-        if (!first) continue;
+        sort_short(k, L);
         double R = 0;
-        for (int j = i; j < ne; j++) {
-            if (!head[j]) continue;
-            long long r2 = (long long)(okey[j] >> bn), c2 = (long long)(okey[j] & mask);
-            if (r2 != row || c2 >= reserved) break;
-            R = R - runval[j] * vef[c2];
+        int u = 0, low = 0, twice = 0;
+        for (int i = 0; i < L;) {
+            const uint32_t o = (uint32_t)(k[i] >> 32);
+            double v = 0;
+            for (; i < L && (uint32_t)(k[i] >> 32) == o; i++) {
+                const uint32_t e = (uint32_t)k[i];
+                if (op[e] == OP_OVERWRITE) v = -g[e];
+                else v = v - g[e];
+            }
+            if ((int)o < reserved) {
+                R = R - v * vef[o];
+                continue;
+            }
+            col[s0 + u] = (int32_t)o - reserved;
+            val[s0 + u] = v;
+            u++;
+            low += o <= self ? 1 : 0;
+            twice += o == self ? 1 : 0;  // a resistor from a node to itself stands below and above the diagonal
         }
-        b[row - reserved] = R;
-    }
-}
-
-__global__ void k_diag_free(int n, int reserved, const double* __restrict__ diag_all, double* __restrict__ diag, int* status) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double d = diag_all[i + reserved];
-        diag[i] = d;
+        len[r] = (int64_t)low | ((int64_t)(u + twice + 1) << 32);
+        diag[r] = d;
+        b[r] = R;
         if (fabs(d) < kZero) atomicCAS(status, 0, (int)DEV_ZERO_DIAG);
+        if (r == n - 1) len[n] = 0;
     }
 }
 
-// Full symmetric CSR (diagonal + lower + upper) for the gather SpMV of the CG.
-__global__ void k_full_keys(int n, int m, int bn, const int32_t* __restrict__ rp, const int32_t* __restrict__ col,
-                            uint64_t* __restrict__ key, uint32_t* __restrict__ val) {
-    // entries: [0, n) diagonal, [n, n+m) lower (row, col), [n+m, n+2m) upper (col, row)
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n + 2 * m; i += gridDim.x * blockDim.x) {
-        uint64_t r, c;
-        if (i < n) {
-            r = c = (uint64_t)i;
-        } else {
-            int e = (i < n + m) ? i - n : i - n - m;
-            // row of lower entry e: binary search in rp
-            int lo = 0, hi = n;
-            while (hi - lo > 1) {
-                int mid = (lo + hi) >> 1;
-                if (rp[mid] <= e) lo = mid; else hi = mid;
+// SSS lower rows (upstream's format, for the getter) and the full symmetric CSR of the gather SpMV, columns ascending.
+__global__ void k_row_emit(int n, const int32_t* __restrict__ rptr, const int32_t* __restrict__ col, const double* __restrict__ val,
+                           const int64_t* __restrict__ ofs, const double* __restrict__ diag, int32_t* __restrict__ lrp,
+                           int32_t* __restrict__ lcol, double* __restrict__ lval, int32_t* __restrict__ frp, int32_t* __restrict__ fcol,
+                           double* __restrict__ fval) {
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r <= n; r += gridDim.x * blockDim.x) {
+        int lo = (int)(uint32_t)ofs[r], fo = (int)(ofs[r] >> 32);
+        lrp[r] = lo;
+        frp[r] = fo;
+        if (r == n) continue;
+        const int f_end = (int)(ofs[r + 1] >> 32);
+        bool placed = false;
+        for (int q = rptr[r]; fo < f_end; q++) {
+            const int c = (fo + (placed ? 0 : 1) < f_end) ? col[q] : n;  // the diagonal alone is left
+            if (!placed && c >= r) {
+                fcol[fo] = r;
+                fval[fo++] = diag[r];
+                placed = true;
+                if (c == n) break;
             }
-            uint64_t rr = (uint64_t)lo, cc = (uint64_t)col[e];
-            if (i < n + m) { r = rr; c = cc; } else { r = cc; c = rr; }
-        }
-        key[i] = (r << bn) | c;
-        val[i] = (uint32_t)i;
-    }
-}
-
-__global__ void k_full_fill(int n, int m, int bn, const uint64_t* __restrict__ key, const uint32_t* __restrict__ val,
-                            const double* __restrict__ diag, const double* __restrict__ lval, int32_t* __restrict__ rcnt,
-                            int32_t* __restrict__ fcol, double* __restrict__ fval, double* __restrict__ minv) {
-    const uint64_t mask = (1ull << bn) - 1;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n + 2 * m; i += gridDim.x * blockDim.x) {
-        uint32_t src = val[i];
-        int r = (int)(key[i] >> bn);
-        fcol[i] = (int)(key[i] & mask);
-        double v;
-        if ((int)src < n) {
-            v = diag[src];
-            minv[src] = 1 / diag[src];  // Jacobi_preconditioner (Direct_Electrifying.cpp:1662-1668)
-        } else {
-            int e = ((int)src < n + m) ? (int)src - n : (int)src - n - m;
-            v = lval[e];
-        }
-        fval[i] = v;
-        atomicAdd(&rcnt[r], 1);
-    }
-}
-
-// Initial_guess_for_cnt_nodes (Direct_Electrifying.cpp:1434-1470).
-__global__ void k_initial_guess(int n, int reserved, int family, double v_p_coord, double max_coord, const int32_t* __restrict__ eb,
-                                const int32_t* __restrict__ ee, const int32_t* __restrict__ elem, const int32_t* __restrict__ lmm,
-                                const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
-                                double* __restrict__ x0) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        for (int k = eb[i]; k < ee[i]; k++) {
-            int P = elem[k];
-            int node = lmm[P];
-            if (node >= 2) {
-                double c = family == 0 ? x[P] : family == 1 ? y[P] : z[P];
-                x0[node - reserved] = v_p_coord * (max_coord - c);
+            const double v = val[q];
+            if (c <= r) {
+                lcol[lo] = c;
+                lval[lo++] = v;
+            }
+            for (int t = 0; t < (c == r ? 2 : 1); t++) {
+                fcol[fo] = c;
+                fval[fo++] = v;
             }
         }
-    }
-}
-
-__global__ void k_spmv_residual(int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ v,
-                                const double* __restrict__ xin, const double* __restrict__ b, double* __restrict__ r) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double s = 0;
-        for (int k = rp[i]; k < rp[i + 1]; k++) s += v[k] * xin[ci[k]];
-        r[i] = b[i] - s;
     }
 }
 
@@ -835,65 +816,70 @@ DeaSystem* solve_dea(Ctx& c, const cicy_params& p, const SolveInput& in, DBuf<in
     try {
         eb.ensure(NM + 1);
         ee.ensure(NM + 1);
-        k_cluster_ranges<<<grid_for(NM), 256, 0, s>>>(NM, in.members, c.bb_lo.get(), c.bb_hi.get(), eb.get(), ee.get(), c.status.get());
-        c.launches++;
-        check_status(c, "LM_matrix_for_cnts");
+        c.claim.ensure(std::max(c.n_points, 1));
+        c.lmm.ensure(std::max(c.n_points, 1));
+        c.node_cnt.ensure(NM + 1);
+        c.node_base.ensure(NM + 1);
+        c.cnt_fresh.ensure(NM + 1);
+        c.chain_start.ensure(NM + 1);
+        c.chain_len.ensure(NM + 1);
         TraceSeq tr(s);
         // ---- LMM ----
-        c.lmm.ensure(std::max(c.n_points, 1));
+        k_cluster_ranges<<<grid_for(NM), 256, 0, s>>>(NM, in.members, c.bb_lo.get(), c.bb_hi.get(), c.elem_idx.get(), eb.get(), ee.get(),
+                                                      c.claim.get(), c.status.get());
         CICY_CUDA(cudaMemsetAsync(c.lmm.get(), 0xff, sizeof(int32_t) * std::max(c.n_points, 1), s));
+        FaceRuns faces{nbnd, {}, {}};
         for (int k = 0; k < nbnd; k++) {
-            int f = bnd[k];
-            int b = c.h_bpts_ptr[f], e = c.h_bpts_ptr[f + 1];
-            if (e > b) {
-                k_lmm_face<<<grid_for(e - b), 256, 0, s>>>(b, e, c.bpts_idx.get(), k, c.lmm.get());
-                c.launches++;
-            }
+            faces.b[k] = c.h_bpts_ptr[bnd[k]];
+            faces.e[k] = c.h_bpts_ptr[bnd[k] + 1];
         }
-        c.cnt_nodes.ensure(NM + 1);
-        c.cnt_node_base.ensure(NM + 1);
-        c.claim.ensure(std::max(c.n_points, 1));
-        c.cnt_fresh.ensure(NM + 1);
-        k_claim_init<<<grid_for(NM), 256, 0, s>>>(NM, eb.get(), ee.get(), c.elem_idx.get(), c.claim.get());
-        k_claim<<<grid_for(NM), 256, 0, s>>>(NM, eb.get(), ee.get(), c.elem_idx.get(), c.claim.get());
-        k_node_counts<<<grid_for(NM), 256, 0, s>>>(NM, eb.get(), ee.get(), c.elem_idx.get(), c.lmm.get(), c.claim.get(), c.cnt_nodes.get(),
+        k_claim<<<grid_for(NM), 256, 0, s>>>(NM, eb.get(), ee.get(), c.elem_idx.get(), c.claim.get(), faces, c.bpts_idx.get(), c.lmm.get());
+        k_node_counts<<<grid_for(NM), 256, 0, s>>>(NM, eb.get(), ee.get(), c.elem_idx.get(), c.lmm.get(), c.claim.get(), c.node_cnt.get(),
                                                    c.cnt_fresh.get());
-        exclusive_scan_i32(c.cnt_nodes.get(), c.cnt_node_base.get(), NM, c.i32_scalar.get(), c.scan_tmp32, s, c.launches);
-        k_node_assign<<<grid_for(NM), 256, 0, s>>>(NM, reserved, eb.get(), ee.get(), c.elem_idx.get(), c.cnt_node_base.get(),
-                                                   c.cnt_fresh.get(), c.lmm.get());
+        c.words.host[W_NODES] = 0;
+        if (NM > 0) exclusive_scan_i64(c.node_cnt.get(), c.node_base.get(), NM, c.words.dev + W_NODES, c.scan_tmp64, s, c.launches);
+        k_node_assign<<<grid_for(NM), 256, 0, s>>>(NM, reserved, eb.get(), ee.get(), c.elem_idx.get(), c.node_cnt.get(), c.node_base.get(),
+                                                   c.cnt_fresh.get(), c.lmm.get(), c.chain_start.get(), c.chain_len.get());
         c.launches += 4;
-        int nodes = reserved + read_i32(c, c.i32_scalar.get());
-        const int n_cnt_free = nodes - reserved;
+        check_status(c, "LM_matrix_for_cnts");  // also waits for the counts
+        const int n_cnt_free = (int)(uint32_t)c.words.host[W_NODES], n_cnt_edges = (int)(c.words.host[W_NODES] >> 32);
+        int nodes = reserved + n_cnt_free;
         const int n_gnp_nodes = in.gnp ? gnp_lmm(c, *in.gnp, bnd, nbnd, nodes) : 0;
         nodes += n_gnp_nodes;
-        // free nodes of each CNT are one consecutive range: the chains of the block preconditioner;
-        // each GNP point node is a chain of its own
+        // each GNP point node is a chain of its own, after the CNTs' chains
         const int NMc = NM + n_gnp_nodes;
-        c.chain_start.ensure(NMc + 1);
-        c.chain_len.ensure(NMc + 1);
-        if (NM > 0) {
-            CICY_CUDA(cudaMemcpyAsync(c.chain_start.get(), c.cnt_node_base.get(), sizeof(int32_t) * NM, cudaMemcpyDeviceToDevice, s));
-            CICY_CUDA(cudaMemcpyAsync(c.chain_len.get(), c.cnt_nodes.get(), sizeof(int32_t) * NM, cudaMemcpyDeviceToDevice, s));
-        }
         if (n_gnp_nodes > 0) {
+            c.chain_cnt.ensure(2 * (size_t)NM + 1);
+            CICY_CUDA(cudaMemcpyAsync(c.chain_cnt.get(), c.chain_start.get(), sizeof(int32_t) * NM, cudaMemcpyDeviceToDevice, s));
+            CICY_CUDA(cudaMemcpyAsync(c.chain_cnt.get() + NM, c.chain_len.get(), sizeof(int32_t) * NM, cudaMemcpyDeviceToDevice, s));
+            c.chain_start.ensure(NMc + 1);
+            c.chain_len.ensure(NMc + 1);
+            CICY_CUDA(cudaMemcpyAsync(c.chain_start.get(), c.chain_cnt.get(), sizeof(int32_t) * NM, cudaMemcpyDeviceToDevice, s));
+            CICY_CUDA(cudaMemcpyAsync(c.chain_len.get(), c.chain_cnt.get() + NM, sizeof(int32_t) * NM, cudaMemcpyDeviceToDevice, s));
             k_singleton_chains<<<grid_for(n_gnp_nodes), 256, 0, s>>>(n_gnp_nodes, NM, n_cnt_free, c.chain_start.get(), c.chain_len.get());
             c.launches++;
         }
         const int n = nodes - reserved;
         sys->nodes = nodes;
         tr.mark(r_flag ? "dea.real.lmm" : "dea.unit.lmm");
-        // ---- edges ----
-        k_cnt_edge_counts<<<grid_for(NM), 256, 0, s>>>(NM, eb.get(), ee.get(), c.elem_idx.get(), c.lmm.get(), c.cnt_nodes.get());
-        exclusive_scan_i32(c.cnt_nodes.get(), c.cnt_node_base.get(), NM, c.i32_scalar.get(), c.scan_tmp32, s, c.launches);
-        c.launches++;
-        const int n_cnt_edges = read_i32(c, c.i32_scalar.get());
+        // ---- resistors and initial guess ----
         const int n_gnp_edges = in.gnp ? gnp_prepare_edges(c, *in.gnp, r_flag) : 0;
         const int NE = n_cnt_edges + in.n_jlist + n_gnp_edges;
         c.e_n1.ensure(NE + 1); c.e_n2.ensure(NE + 1); c.e_op.ensure(NE + 1); c.e_g.ensure(NE + 1);
-        k_cnt_edges<<<grid_for(NM), 256, 0, s>>>(NM, r_flag, p.resistivity_cnt, in.members, eb.get(), ee.get(), c.elem_idx.get(), c.lmm.get(),
-                                               c.cnt_node_base.get(), c.radii.get(), c.x.get(), c.y.get(), c.z.get(), c.e_n1.get(),
-                                               c.e_n2.get(), c.e_op.get(), c.e_g.get());
+        sys->x0.ensure(std::max(n, 1));
+        c.cg_x.ensure(n + 1);
+        CICY_CUDA(cudaMemsetAsync(sys->x0.get(), 0, sizeof(double) * std::max(n, 1), s));
+        GuessArgs guess{nullptr, 0, 0, 0};
+        if (r_flag && reserved == 2) {
+            const cicy_cuboid& w = c.window;
+            const double Lw = in.family == 0 ? w.len_x : in.family == 1 ? w.len_y : w.len_z;
+            guess = GuessArgs{sys->x0.get(), in.family, p.applied_voltage / Lw, in.family == 0 ? w.max_x : in.family == 1 ? w.max_y : w.max_z};
+        }
+        k_cnt_edges<<<grid_for((long long)NM * kEdgeLanes), 256, 0, s>>>(
+            NM, r_flag, reserved, p.resistivity_cnt, in.members, eb.get(), ee.get(), c.elem_idx.get(), c.lmm.get(), c.node_base.get(),
+            c.radii.get(), c.x.get(), c.y.get(), c.z.get(), c.e_n1.get(), c.e_n2.get(), c.e_op.get(), c.e_g.get(), guess);
         c.launches++;
+        if (n > 0) CICY_CUDA(cudaMemcpyAsync(c.cg_x.get(), sys->x0.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
         if (in.n_jlist > 0) {
             k_junction_edges<<<grid_for(in.n_jlist), 256, 0, s>>>(in.n_jlist, n_cnt_edges, r_flag, reserved, p.junction_type,
                                                                 p.junction_resistance, p.C1, p.C2, in.jlist, c.j_p1.get(), c.j_n1.get(),
@@ -903,56 +889,41 @@ DeaSystem* solve_dea(Ctx& c, const cicy_params& p, const SolveInput& in, DBuf<in
         }
         if (in.gnp) gnp_fill_edges(c, *in.gnp, n_cnt_edges + in.n_jlist, r_flag, reserved, p);
         tr.mark(r_flag ? "dea.real.edges" : "dea.unit.edges");
-        // ---- sort-and-reduce assembly ----
-        const int bn = bits_for((uint64_t)std::max(nodes, 1));
-        const int ND = 2 * NE;
-        c.sort_k.ensure(std::max(ND, 2 * NE) + 2);
-        c.sort_v.ensure(std::max(ND, 2 * NE) + 2);
-        DBuf<uint64_t>& dkey = c.dkey;
-        DBuf<uint32_t>& dval = c.dval;
-        dkey.ensure(ND + 2);
-        dval.ensure(ND + 2);
-        k_edge_keys<<<grid_for(NE), 256, 0, s>>>(NE, bn, c.e_n1.get(), c.e_n2.get(), c.e_op.get(), c.sort_k.get(), c.sort_v.get(),
-                                               dkey.get(), dval.get());
-        c.launches++;
-        radix_sort_pairs(c.sort_k.get(), c.sort_v.get(), NE, 2 * bn + 1, c.rs, s, c.launches);
-        radix_sort_pairs(dkey.get(), dval.get(), ND, bn + 1, c.rs, s, c.launches);
-        tr.mark("asm.sorts");
-        c.work_f64a.ensure(std::max(nodes, NE) + 1);  // diag over all nodes
-        CICY_CUDA(cudaMemsetAsync(c.work_f64a.get(), 0, sizeof(double) * (nodes + 1), s));
-        k_diag_reduce<<<grid_for(ND), 256, 0, s>>>(ND, 1ull << bn, (uint64_t)reserved, dkey.get(), dval.get(), c.e_g.get(),
-                                                   c.work_f64a.get());
-        c.work_i32a.ensure(NE + 1);
-        c.work_i32b.ensure(NE + 1);
-        c.work_i32c.ensure(NE + 1);
-        c.runval.ensure(NE + 1);
-        k_offdiag_reduce<<<grid_for(NE), 256, 0, s>>>(NE, 1ull << (2 * bn), c.sort_k.get(), c.sort_v.get(), c.e_op.get(), c.e_g.get(), c.work_i32a.get(),
-                                                    c.runval.get());
-        tr.mark("asm.reduce");
-        k_sss_flags<<<grid_for(NE), 256, 0, s>>>(NE, bn, reserved, c.sort_k.get(), c.work_i32a.get(), c.work_i32b.get());
-        exclusive_scan_i32(c.work_i32b.get(), c.work_i32c.get(), NE, c.i32_scalar.get(), c.scan_tmp32, s, c.launches);
-        c.launches += 3;
-        const int m = read_i32(c, c.i32_scalar.get());
-        sys->nnz_lower = m;
-        sys->row_ptr.ensure(n + 1); sys->col.ensure(std::max(m, 1)); sys->val.ensure(std::max(m, 1));
-        sys->diag.ensure(std::max(n, 1)); sys->b.ensure(std::max(n, 1)); sys->x0.ensure(std::max(n, 1));
-        sys->volt.ensure(std::max(nodes, 1));
-        c.cnt_nodes.ensure(n + 1);
-        CICY_CUDA(cudaMemsetAsync(c.cnt_nodes.get(), 0, sizeof(int32_t) * (n + 1), s));
-        k_sss_fill<<<grid_for(NE), 256, 0, s>>>(NE, bn, reserved, c.sort_k.get(), c.work_i32b.get(), c.work_i32c.get(), c.runval.get(),
-                                              c.cnt_nodes.get(), sys->col.get(), sys->val.get());
-        exclusive_scan_i32(c.cnt_nodes.get(), sys->row_ptr.get(), n + 1, nullptr, c.scan_tmp32, s, c.launches);
-        tr.mark("asm.sss");
+        // ---- assembly by rows ----
         // Get_voltage_vector (Direct_Electrifying.cpp:1472-1500)
         std::vector<double> vef(reserved, 0.0);
         const double V = r_flag ? p.applied_voltage : (double)nodes;
         for (int i = 1; i < reserved; i++) vef[i] = vef[i - 1] + V;
         c.vef.ensure(8);
         CICY_CUDA(cudaMemcpyAsync(c.vef.get(), vef.data(), sizeof(double) * reserved, cudaMemcpyHostToDevice, s));
-        CICY_CUDA(cudaMemsetAsync(sys->b.get(), 0, sizeof(double) * std::max(n, 1), s));
-        k_rhs<<<grid_for(NE), 256, 0, s>>>(NE, bn, reserved, c.sort_k.get(), c.work_i32a.get(), c.runval.get(), c.vef.get(), sys->b.get());
-        k_diag_free<<<grid_for(n), 256, 0, s>>>(n, reserved, c.work_f64a.get(), sys->diag.get(), c.status.get());
-        c.launches += 3;
+        // every resistor is in at most two rows, so couplings number at most NE below the diagonal, n + 2 NE in the full rows
+        c.row_cnt.ensure(n + 1); c.row_ptr.ensure(n + 1); c.row_pos.ensure(2 * (size_t)NE + 1);
+        c.row_key.ensure(2 * (size_t)NE + 1); c.row_col.ensure(2 * (size_t)NE + 1); c.row_val.ensure(2 * (size_t)NE + 1);
+        c.row_len.ensure(n + 1); c.row_ofs.ensure(n + 1);
+        sys->row_ptr.ensure(n + 1); sys->col.ensure(NE + 1); sys->val.ensure(NE + 1);
+        sys->diag.ensure(std::max(n, 1)); sys->b.ensure(std::max(n, 1)); sys->volt.ensure(std::max(nodes, 1));
+        c.cg_rp.ensure(n + 1); c.cg_ci.ensure(n + 2 * (size_t)NE + 1); c.cg_val.ensure(n + 2 * (size_t)NE + 1);
+        CICY_CUDA(cudaMemsetAsync(c.row_cnt.get(), 0, sizeof(int32_t) * (n + 1), s));
+        if (n == 0) CICY_CUDA(cudaMemsetAsync(c.row_len.get(), 0, sizeof(int64_t), s));
+        k_row_count<<<grid_for(NE), 256, 0, s>>>(NE, reserved, c.e_n1.get(), c.e_n2.get(), c.e_op.get(), c.row_cnt.get(), c.row_pos.get());
+        exclusive_scan_i32(c.row_cnt.get(), c.row_ptr.get(), n + 1, nullptr, c.scan_tmp32, s, c.launches);
+        k_row_place<<<grid_for(NE), 256, 0, s>>>(NE, reserved, c.e_n1.get(), c.e_n2.get(), c.e_op.get(), c.row_ptr.get(), c.row_pos.get(),
+                                                 c.row_key.get());
+        k_row_build<<<grid_for(n, 128), 128, 0, s>>>(n, reserved, c.row_ptr.get(), c.row_key.get(), c.e_op.get(), c.e_g.get(), c.vef.get(),
+                                                     c.row_col.get(), c.row_val.get(), c.row_len.get(), sys->diag.get(), sys->b.get(),
+                                                     c.status.get());
+        exclusive_scan_i64(c.row_len.get(), c.row_ofs.get(), n + 1, c.words.dev + W_NNZ, c.scan_tmp64, s, c.launches);
+        k_row_emit<<<grid_for(n + 1), 256, 0, s>>>(n, c.row_ptr.get(), c.row_col.get(), c.row_val.get(), c.row_ofs.get(), sys->diag.get(),
+                                                   sys->row_ptr.get(), sys->col.get(), sys->val.get(), c.cg_rp.get(), c.cg_ci.get(),
+                                                   c.cg_val.get());
+        c.launches += 4;
+        // host copy of the chains, for cicy_get_chains
+        sys->h_chain_start.resize(NMc);
+        sys->h_chain_len.resize(NMc);
+        if (NMc > 0) {
+            CICY_CUDA(cudaMemcpyAsync(sys->h_chain_start.data(), c.chain_start.get(), sizeof(int32_t) * NMc, cudaMemcpyDeviceToHost, s));
+            CICY_CUDA(cudaMemcpyAsync(sys->h_chain_len.data(), c.chain_len.get(), sizeof(int32_t) * NMc, cudaMemcpyDeviceToHost, s));
+        }
         try {
             check_status(c, "Fill_sparse_stiffness_matrix");
         } catch (Fail& f) {
@@ -974,38 +945,9 @@ DeaSystem* solve_dea(Ctx& c, const cicy_params& p, const SolveInput& in, DBuf<in
             }
             throw;
         }
+        sys->nnz_lower = (int64_t)(uint32_t)c.words.host[W_NNZ];
+        const int NF = (int)(c.words.host[W_NNZ] >> 32);
         tr.mark(r_flag ? "dea.real.assembly" : "dea.unit.assembly");
-        // ---- full CSR for the CG ----
-        const int NF = n + 2 * m;
-        const int bnf = bits_for((uint64_t)std::max(n, 1));
-        c.sort_k.ensure(NF + 1);
-        c.sort_v.ensure(NF + 1);
-        c.cg_rp.ensure(n + 1); c.cg_ci.ensure(NF + 1); c.cg_val.ensure(NF + 1); c.cg_minv.ensure(n + 1);
-        k_full_keys<<<grid_for(NF), 256, 0, s>>>(n, m, bnf, sys->row_ptr.get(), sys->col.get(), c.sort_k.get(), c.sort_v.get());
-        radix_sort_pairs(c.sort_k.get(), c.sort_v.get(), NF, 2 * bnf, c.rs, s, c.launches);
-        CICY_CUDA(cudaMemsetAsync(c.cnt_nodes.get(), 0, sizeof(int32_t) * (n + 1), s));
-        k_full_fill<<<grid_for(NF), 256, 0, s>>>(n, m, bnf, c.sort_k.get(), c.sort_v.get(), sys->diag.get(), sys->val.get(), c.cnt_nodes.get(),
-                                               c.cg_ci.get(), c.cg_val.get(), c.cg_minv.get());
-        exclusive_scan_i32(c.cnt_nodes.get(), c.cg_rp.get(), n + 1, nullptr, c.scan_tmp32, s, c.launches);
-        c.launches += 2;
-        tr.mark(r_flag ? "dea.real.full_csr" : "dea.unit.full_csr");
-        // ---- initial guess and r0 ----
-        c.cg_x.ensure(n + 1); c.cg_r.ensure(n + 1); c.cg_z.ensure(n + 1); c.cg_p.ensure(n + 1); c.cg_q.ensure(n + 1);
-        CICY_CUDA(cudaMemsetAsync(sys->x0.get(), 0, sizeof(double) * std::max(n, 1), s));
-        if (r_flag && reserved == 2) {
-            const cicy_cuboid& w = c.window;
-            const double Lw = in.family == 0 ? w.len_x : in.family == 1 ? w.len_y : w.len_z;
-            const double maxc = in.family == 0 ? w.max_x : in.family == 1 ? w.max_y : w.max_z;
-            k_initial_guess<<<grid_for(NM), 256, 0, s>>>(NM, reserved, in.family, p.applied_voltage / Lw, maxc, eb.get(), ee.get(),
-                                                       c.elem_idx.get(), c.lmm.get(), c.x.get(), c.y.get(), c.z.get(), sys->x0.get());
-            c.launches++;
-        }
-        if (n > 0) {
-            k_spmv_residual<<<grid_for(n), 256, 0, s>>>(n, c.cg_rp.get(), c.cg_ci.get(), c.cg_val.get(), sys->x0.get(), sys->b.get(), c.cg_r.get());
-            CICY_CUDA(cudaMemcpyAsync(c.cg_x.get(), sys->x0.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-            c.launches++;
-        }
-        tr.mark(r_flag ? "dea.real.guess" : "dea.unit.guess");
         // ---- CG ----
         SolverSystem ss;
         ss.n = n;
@@ -1025,13 +967,6 @@ DeaSystem* solve_dea(Ctx& c, const cicy_params& p, const SolveInput& in, DBuf<in
             tr.mark(r_flag ? "dea.real.gnn" : "dea.unit.gnn");
         } else if (c.solver.preconditioner != CICY_PRECOND_JACOBI && n > 0) {
             kind = PRECOND_KIND_BLOCK;
-        }
-        // host copy of the chains, for cicy_get_chains
-        sys->h_chain_start.resize(NMc);
-        sys->h_chain_len.resize(NMc);
-        if (NMc > 0) {
-            CICY_CUDA(cudaMemcpyAsync(sys->h_chain_start.data(), c.chain_start.get(), sizeof(int32_t) * NMc, cudaMemcpyDeviceToHost, s));
-            CICY_CUDA(cudaMemcpyAsync(sys->h_chain_len.data(), c.chain_len.get(), sizeof(int32_t) * NMc, cudaMemcpyDeviceToHost, s));
         }
         PcgStats st;
         const double tol = (r_flag == 0 && p.tolerance_unit > 0) ? p.tolerance_unit : p.tolerance;
@@ -1057,41 +992,35 @@ DeaSystem* solve_dea(Ctx& c, const cicy_params& p, const SolveInput& in, DBuf<in
                 build_block_preconditioner(c.sw, ss, NMc, c.chain_start.get(), c.chain_len.get(), nullptr, nullptr, mixed, s, c.launches);
             pcg_solve(c.sw, ss, kind, mixed, tol, max_iter, c.num_sms, c.status.get(), s, c.launches, st, ew);
         }
-        check_status(c, "Solve_DEA_equations_CG_SSS");
         tr.mark(r_flag ? "dea.real.cg" : "dea.unit.cg");
-        // true FP64 residual |b - A x| / |b|
-        auto true_residual = [&]() {
-            double rb[2] = {0, 0};
-            if (n > 0) {
-                c.cg_scal.ensure(4);
-                CICY_CUDA(cudaMemsetAsync(c.cg_scal.get(), 0, sizeof(double) * 2, s));
-                k_true_residual<<<grid_for(n), 256, 0, s>>>(n, c.cg_rp.get(), c.cg_ci.get(), c.cg_val.get(), c.cg_x.get(), sys->b.get(),
-                                                          c.cg_scal.get());
-                c.launches++;
-                CICY_CUDA(cudaMemcpyAsync(rb, c.cg_scal.get(), sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
-                CICY_CUDA(cudaStreamSynchronize(s));
-            }
+        // true FP64 residual |b - A x| / |b| and the voltages of all nodes
+        auto finish = [&](const char* where) {
+            c.cg_scal.ensure(4);
+            CICY_CUDA(cudaMemsetAsync(c.cg_scal.get(), 0, sizeof(double) * 2, s));
+            k_true_residual<<<grid_for(n), 256, 0, s>>>(n, c.cg_rp.get(), c.cg_ci.get(), c.cg_val.get(), c.cg_x.get(), sys->b.get(),
+                                                      c.cg_scal.get());
+            k_voltages<<<grid_for(nodes), 256, 0, s>>>(nodes, reserved, c.vef.get(), c.cg_x.get(), sys->volt.get());
+            c.launches += 2;
+            double* rb = reinterpret_cast<double*>(c.words.host + W_RESID);
+            CICY_CUDA(cudaMemcpyAsync(rb, c.cg_scal.get(), sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
+            check_status(c, where);
             return rb[1] > 0 ? std::sqrt(rb[0] / rb[1]) : 0.0;
         };
-        double rel = true_residual();
+        double rel = finish("Solve_DEA_equations_CG_SSS");
         if (kind == PRECOND_KIND_SPAI && !(rel <= 10 * tol && st.iterations < max_iter)) {
             // the learned preconditioner did not reduce the residual: Jacobi-PCG from the initial guess
             const double seconds = st.seconds;
             CICY_CUDA(cudaMemcpyAsync(c.cg_x.get(), sys->x0.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
             pcg_solve(c.sw, ss, PRECOND_KIND_JACOBI, false, tol, max_iter, c.num_sms, c.status.get(), s, c.launches, st);
-            check_status(c, "Solve_DEA_equations_CG_SSS (Jacobi fallback)");
             st.seconds += seconds;
             sys->fallback = 1;
-            rel = true_residual();
+            rel = finish("Solve_DEA_equations_CG_SSS (Jacobi fallback)");
         }
         sys->cluster_solver = st.cluster;
         sys->mg_levels = st.levels;
         sys->seconds = st.seconds;
         sys->iterations = st.iterations;
         sys->restarts = st.restarts;
-        k_voltages<<<grid_for(nodes), 256, 0, s>>>(nodes, reserved, c.vef.get(), c.cg_x.get(), sys->volt.get());
-        c.launches++;
-        CICY_CUDA(cudaStreamSynchronize(s));
         sys->rel_residual = rel;
     } catch (...) {
         c.sys_pool.push_back(sys);

@@ -364,7 +364,6 @@ void generate_network_device(Ctx& c, const cicy_gen_params& g) {
     const PhiloxDev rng{(uint32_t)(g.seed & 0xffffffffu), (uint32_t)(g.seed >> 32)};
     c.clen.ensure(std::max(nc, 1));
     c.cstart.ensure(std::max(nc, 1) + 1);
-    c.i64_scalar.ensure(8);
     c.i32_scalar.ensure(8);
     c.status.ensure(1);
     c.radii.ensure(std::max(nc, 1));
