@@ -22,7 +22,7 @@ struct GridGeom {
 // size is read by waiting for the stream instead of by a copy to pageable memory as well.
 // Registering a page costs about 2.5 ms, so contexts share pages of 32 slots (stage_clusters.cu);
 // a page is freed with its last slot, but for one that is kept for the next context.
-enum HostWord : int { W_READ = 0, W_STATUS = 1, W_NODES = 2, W_NNZ = 3, W_RESID = 4 /* two */, W_COUNT = 16 };
+enum HostWord : int { W_READ = 0, W_STATUS = 1, W_NODES = 2, W_NNZ = 3, W_RESID = 4 /* two */, W_WIN = 8, W_COUNT = 16 };
 int64_t* host_words_take();
 void host_words_return(int64_t* slot);
 struct HostWords {
@@ -217,6 +217,7 @@ struct Ctx {
     DBuf<int32_t> win_prun, win_pparent, win_pnev, win_cs, win_cl, win_raw_p, win_raw_c;
     DBuf<int64_t> win_ev, win_pev;
     DBuf<double> win_rad;
+    DBuf<unsigned long long> gen_total;
 
     // ---- CNT-GNP contacts (cicy_gnp_cnt_contacts), indexed by contact-point number ----
     int n_mix = 0;

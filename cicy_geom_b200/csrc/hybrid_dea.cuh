@@ -954,7 +954,7 @@ void run_hybrid_electrical(Ctx& c, const cicy_hybrid_state& h, const cicy_params
                 const int nb = (int)(c.h_bcnt_ptr[b1 + 1] - c.h_bcnt_ptr[b1]);
                 c.bterm.ensure(2 * (size_t)std::max(nb, 1));
                 c.bvalid.ensure(2 * (size_t)std::max(nb, 1));
-                k_boundary_terms<<<grid_for(2 * nb), 128, 0, s>>>((int)c.h_bcnt_ptr[b1], (int)c.h_bcnt_ptr[b1 + 1], c.bcnt_idx.get(),
+                k_boundary_terms<<<grid_for(2LL * nb * kLanes, 128), 128, 0, s>>>((int)c.h_bcnt_ptr[b1], (int)c.h_bcnt_ptr[b1 + 1], c.bcnt_idx.get(),
                                                                  c.bb_lo.get(), c.bb_hi.get(), c.elem_idx.get(), c.lmm.get(), sr->volt.get(),
                                                                  c.radii.get(), p.resistivity_cnt, c.x.get(), c.y.get(), c.z.get(),
                                                                  c.bterm.get(), c.bvalid.get());

@@ -150,11 +150,48 @@ __device__ __forceinline__ double cnt_volume(int P1, int P2, double radius, cons
     return length * kPI * radius * radius;
 }
 
+// Length from P1 to P2 by kLanes threads (a power of two of one warp): each thread takes one
+// point's distance, then all add the kLanes distances in point order by shuffle, so the sum is
+// upstream's sequence of additions (a distance past P2 adds +0.0, which leaves a sum >= 0 as it
+// is).  One thread per CNT waited for ~100 dependent load-sqrt-add steps: the isolated CNTs'
+// volumes took 82 us on 509 CNTs (2 um), the backbone's 216 us, the boundary terms 55 us on the
+// 25k-CNT network; with 8 threads 18, 36 and 13 us.
+constexpr int kLanes = 8;
+struct LaneGroup {
+    int lane;
+    unsigned mask;
+    __device__ LaneGroup() : lane(threadIdx.x % kLanes), mask(((1u << kLanes) - 1) << ((threadIdx.x & 31) & ~(kLanes - 1))) {}
+    __device__ int first() const { return (blockIdx.x * blockDim.x + threadIdx.x) / kLanes; }
+    __device__ static int step() { return gridDim.x * blockDim.x / kLanes; }
+};
+__device__ __forceinline__ double group_length(const LaneGroup& gr, int P1, int P2, const double* __restrict__ x, const double* __restrict__ y,
+                                               const double* __restrict__ z) {
+    double length = 0;
+    for (int b = P1; b < P2; b += kLanes) {
+        const int i = b + gr.lane;
+        double d = 0;
+        if (i < P2) {
+            const double dx = x[i] - x[i + 1], dy = y[i] - y[i + 1], dz = z[i] - z[i + 1];
+            d = sqrt(dx * dx + dy * dy + dz * dz);
+        }
+#pragma unroll
+        for (int t = 0; t < kLanes; t++) length = length + __shfl_sync(gr.mask, d, t, kLanes);
+    }
+    return length;
+}
+__device__ __forceinline__ double group_resistance(const LaneGroup& gr, int P1, int P2, double radius, double rho, const double* __restrict__ x,
+                                                   const double* __restrict__ y, const double* __restrict__ z) {
+    return rho * group_length(gr, P1, P2, x, y, z) / (kPI * radius * radius);
+}
+__device__ __forceinline__ double group_volume(const LaneGroup& gr, int P1, int P2, double radius, const double* __restrict__ x,
+                                               const double* __restrict__ y, const double* __restrict__ z) {
+    return group_length(gr, P1, P2, x, y, z) * kPI * radius * radius;
+}
+
 // Fill_2d_matrices_cnts + Three_points_in_element (Direct_Electrifying.cpp:489-608), and, with
-// x0, Initial_guess_for_cnt_nodes (:1434-1470).  kEdgeLanes threads per CNT, one resistor each at
-// a time: a resistor's length is a serial sum over its points (upstream's order), and one thread
-// per CNT walked all of a CNT's ~100 points (both passes of the 25k-CNT network: 139 us, now 62 us).
-constexpr int kEdgeLanes = 8;
+// x0, Initial_guess_for_cnt_nodes (:1434-1470).  kLanes threads per CNT: resistor by resistor
+// together when the CNT has few (long) ones, else one resistor each (both passes of the 25k-CNT
+// network: 139 us with one thread per CNT, 62 us with one resistor per thread, 40 us so).
 struct GuessArgs {
     double* x0;  // null: no initial guess
     int axis;
@@ -165,13 +202,14 @@ __global__ void k_cnt_edges(int n, int r_flag, int reserved, double rho, const i
                             const int64_t* __restrict__ base, const double* __restrict__ radii, const double* __restrict__ x,
                             const double* __restrict__ y, const double* __restrict__ z, int32_t* __restrict__ n1,
                             int32_t* __restrict__ n2, int32_t* __restrict__ op, double* __restrict__ g, GuessArgs guess) {
-    const int lane = threadIdx.x % kEdgeLanes;
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) / kEdgeLanes; i < n; i += gridDim.x * blockDim.x / kEdgeLanes) {
+    const LaneGroup gr;
+    const int lane = gr.lane;
+    for (int i = gr.first(); i < n; i += LaneGroup::step()) {
         const int b = eb[i], m = ee[i] - b, o = (int)(base[i] >> 32);
         if (m < 2) continue;
         const double r = radii[members[i]];
         if (guess.x0) {
-            for (int k = lane; k < m; k += kEdgeLanes) {
+            for (int k = lane; k < m; k += kLanes) {
                 const int P = elem[b + k], node = lmm[P];
                 if (node < 2) continue;
                 const double c = guess.axis == 0 ? x[P] : guess.axis == 1 ? y[P] : z[P];
@@ -179,21 +217,25 @@ __global__ void k_cnt_edges(int n, int r_flag, int reserved, double rho, const i
             }
         }
         if (m == 3 && lmm[elem[b]] == lmm[elem[b + 2]]) {
-            if (lane != 0) continue;
             double g1 = 1.0, g2 = 1.0;
             if (r_flag == 1) {
-                g1 = 1 / cnt_resistance(elem[b], elem[b + 1], r, rho, x, y, z);
-                g2 = 1 / cnt_resistance(elem[b + 1], elem[b + 2], r, rho, x, y, z);
+                g1 = 1 / group_resistance(gr, elem[b], elem[b + 1], r, rho, x, y, z);
+                g2 = 1 / group_resistance(gr, elem[b + 1], elem[b + 2], r, rho, x, y, z);
             }
+            if (lane != 0) continue;
             n1[o] = lmm[elem[b]];
             n2[o] = lmm[elem[b + 1]];
             op[o] = OP_OVERWRITE;
             g[o] = g1 + g2;
             continue;
         }
-        for (int k = lane; k < m - 1; k += kEdgeLanes) {
+        const bool together = r_flag == 1 && m <= kLanes;
+        for (int k = together ? 0 : lane; k < m - 1; k += together ? 1 : kLanes) {
             int P1 = elem[b + k], P2 = elem[b + k + 1];
-            double gi = r_flag ? 1 / cnt_resistance(P1, P2, r, rho, x, y, z) : 1.0;
+            double gi = 1.0;
+            if (together) gi = 1 / group_resistance(gr, P1, P2, r, rho, x, y, z);
+            else if (r_flag) gi = 1 / cnt_resistance(P1, P2, r, rho, x, y, z);
+            if (together && lane != 0) continue;
             n1[o + k] = lmm[P1];
             n2[o + k] = lmm[P2];
             op[o + k] = OP_OVERWRITE;
@@ -547,8 +589,23 @@ __global__ void k_backbone_scan(int n, const int32_t* __restrict__ members, cons
 __global__ void k_backbone_volumes(int n, const int32_t* __restrict__ pts, const double* __restrict__ radii, const double* __restrict__ x,
                                    const double* __restrict__ y, const double* __restrict__ z, double* __restrict__ vol3,
                                    int32_t* __restrict__ kind) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        backbone_volumes(i, radii[pts[5 * i]], pts[5 * i + 1], pts[5 * i + 2], pts[5 * i + 3], pts[5 * i + 4], x, y, z, vol3, kind);
+    const LaneGroup gr;
+    for (int i = gr.first(); i < n; i += LaneGroup::step()) {
+        const int32_t* q = pts + 5 * (size_t)i;
+        const double r = radii[q[0]];
+        const int Ps = q[1], P1 = q[2], P2 = q[3], Pe = q[4];
+        const double before = group_volume(gr, Ps, P1 < 0 ? Pe : P1, r, x, y, z);
+        double run = 0, after = 0;
+        if (P1 >= 0) {
+            run = group_volume(gr, P1, P2 < 0 ? Pe : P2, r, x, y, z);
+            if (P2 >= 0) after = group_volume(gr, P2, Pe, r, x, y, z);
+        }
+        if (gr.lane != 0) continue;
+        vol3[3 * i] = before;
+        if (P1 >= 0) vol3[3 * i + 1] = run;
+        if (P1 >= 0 && P2 >= 0) vol3[3 * i + 2] = after;
+        kind[i] = P1 < 0 ? 0 : P2 < 0 ? 1 : 2;
+    }
 }
 
 // Volume members of Backbone_Network (acc: volumes_cnt[8], dead_branches[7], then the
@@ -634,11 +691,14 @@ __global__ void k_isolated_volumes(int n_inside, uint64_t end, const uint64_t* _
                                    const int32_t* __restrict__ cstart, const int32_t* __restrict__ clen, const double* __restrict__ radii,
                                    const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
                                    double* __restrict__ vol, int32_t* count) {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n_inside; p += gridDim.x * blockDim.x) {
+    const LaneGroup gr;
+    for (int p = gr.first(); p < n_inside; p += LaneGroup::step()) {
         if (key[p] >= end) continue;
         const int c = (int)cnt[p];
-        vol[p] = cnt_volume(cstart[c], cstart[c] + clen[c] - 1, radii[c], x, y, z);
-        atomicMax(count, p + 1);
+        const double v = group_volume(gr, cstart[c], cstart[c] + clen[c] - 1, radii[c], x, y, z);
+        if (gr.lane != 0) continue;
+        vol[p] = v;
+        if (p + 1 == n_inside || key[p + 1] >= end) *count = p + 1;  // the isolated CNTs are a prefix of the list
     }
 }
 
@@ -707,7 +767,8 @@ __global__ void k_boundary_terms(int b, int e, const int32_t* __restrict__ bcnt,
                                  const double* __restrict__ x, const double* __restrict__ y, const double* __restrict__ z,
                                  double* __restrict__ term, int32_t* __restrict__ valid) {
     const int m = 2 * (e - b);
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < m; t += gridDim.x * blockDim.x) {
+    const LaneGroup gr;
+    for (int t = gr.first(); t < m; t += LaneGroup::step()) {
         const int i = b + (t >> 1), side = t & 1;
         int ok = 0;
         double v = 0;
@@ -721,13 +782,13 @@ __global__ void k_boundary_terms(int b, int e, const int32_t* __restrict__ bcnt,
                 const int n2 = lmm[P2];
                 if (n2 >= 0) {
                     const double V = volt[n2] - volt[n1];
-                    const double Re = (P1 > P2) ? cnt_resistance(P2, P1, radii[c], rho, x, y, z)
-                                                : cnt_resistance(P1, P2, radii[c], rho, x, y, z);
+                    const double Re = group_resistance(gr, min(P1, P2), max(P1, P2), radii[c], rho, x, y, z);
                     v = V / Re;
                     ok = 1;
                 }
             }
         }
+        if (gr.lane != 0) continue;
         term[t] = v;
         valid[t] = ok;
     }
@@ -875,7 +936,7 @@ DeaSystem* solve_dea(Ctx& c, const cicy_params& p, const SolveInput& in, DBuf<in
             const double Lw = in.family == 0 ? w.len_x : in.family == 1 ? w.len_y : w.len_z;
             guess = GuessArgs{sys->x0.get(), in.family, p.applied_voltage / Lw, in.family == 0 ? w.max_x : in.family == 1 ? w.max_y : w.max_z};
         }
-        k_cnt_edges<<<grid_for((long long)NM * kEdgeLanes), 256, 0, s>>>(
+        k_cnt_edges<<<grid_for((long long)NM * kLanes), 256, 0, s>>>(
             NM, r_flag, reserved, p.resistivity_cnt, in.members, eb.get(), ee.get(), c.elem_idx.get(), c.lmm.get(), c.node_base.get(),
             c.radii.get(), c.x.get(), c.y.get(), c.z.get(), c.e_n1.get(), c.e_n2.get(), c.e_op.get(), c.e_g.get(), guess);
         c.launches++;
@@ -1086,7 +1147,7 @@ void run_electrical(Ctx& c, const cicy_params& p, cicy_result* out) {
                          c.rs_side, ss, c.launches);
         c.vol_iso.ensure(c.n_inside);
         CICY_CUDA(cudaMemsetAsync(c.i32_scalar.get() + 2, 0, sizeof(int32_t), ss));
-        k_isolated_volumes<<<grid_for(c.n_inside), 256, 0, ss>>>(c.n_inside, (uint64_t)(c.n_labels + 1) * (uint64_t)c.n_inside,
+        k_isolated_volumes<<<grid_for((long long)c.n_inside * kLanes), 256, 0, ss>>>(c.n_inside, (uint64_t)(c.n_labels + 1) * (uint64_t)c.n_inside,
                                                                  c.vol_key.get(), c.vol_cnt.get(), c.cstart.get(), c.clen.get(),
                                                                  c.radii.get(), c.x.get(), c.y.get(), c.z.get(), c.vol_iso.get(),
                                                                  c.i32_scalar.get() + 2);
@@ -1120,7 +1181,7 @@ void run_electrical(Ctx& c, const cicy_params& p, cicy_result* out) {
         // the volumes (read by no later stage of the step) beside the real-resistor pass
         CICY_CUDA(cudaEventRecord(c.ev_main, s));
         CICY_CUDA(cudaStreamWaitEvent(c.side, c.ev_main, 0));
-        k_backbone_volumes<<<grid_for(NM), 256, 0, c.side>>>(NM, c.bb_pts.get(), c.radii.get(), c.x.get(), c.y.get(), c.z.get(), c.vol3.get(),
+        k_backbone_volumes<<<grid_for((long long)NM * kLanes), 256, 0, c.side>>>(NM, c.bb_pts.get(), c.radii.get(), c.x.get(), c.y.get(), c.z.get(), c.vol3.get(),
                                                             c.vol_kind.get());
         k_volume_sum<<<1, kSumThreads, 0, c.side>>>(NM, c.h_family[k], c.vol3.get(), c.vol_kind.get(), c.vol_acc.get());
         CICY_CUDA(cudaEventRecord(c.ev_side, c.side));
@@ -1177,7 +1238,7 @@ void run_electrical(Ctx& c, const cicy_params& p, cicy_result* out) {
             const int nb = (int)(c.h_bcnt_ptr[b1 + 1] - c.h_bcnt_ptr[b1]);
             c.bterm.ensure(2 * (size_t)nb);
             c.bvalid.ensure(2 * (size_t)nb);
-            k_boundary_terms<<<grid_for(2 * nb), 128, 0, s>>>((int)c.h_bcnt_ptr[b1], (int)c.h_bcnt_ptr[b1 + 1], c.bcnt_idx.get(),
+            k_boundary_terms<<<grid_for(2LL * nb * kLanes, 128), 128, 0, s>>>((int)c.h_bcnt_ptr[b1], (int)c.h_bcnt_ptr[b1 + 1], c.bcnt_idx.get(),
                                                              c.bb_lo.get(), c.bb_hi.get(), c.elem_idx.get(), c.lmm.get(), sr->volt.get(),
                                                              c.radii.get(), p.resistivity_cnt, c.x.get(), c.y.get(), c.z.get(),
                                                              c.bterm.get(), c.bvalid.get());

@@ -132,83 +132,114 @@ struct TrimOut {
     int nev = 0;
 };
 
-// Trim_boundary_cnts for one CNT whose points are the run base .. base + n - 1.
-// Pieces (segment m >= 1) get flag -m on their points and a slot (start, end,
-// in shell 0); `allow_pieces` false (the pieces' own pass) makes a piece an error.
+// Add_cnt_segment_to_structure for the segment s0 .. e0 of the run at `base`.  Pieces (segment
+// m >= 1) get flag -m on their points and a slot (start, end, in shell 0); `allow_pieces` false
+// (the pieces' own pass) makes a piece an error.
+__host__ __device__ inline int add_segment(const WinGeom& g, const Pts& p, int base, int s0, int e0, int end_loc, bool allow_pieces, TrimOut& o,
+                                           int32_t* slots, int64_t* ev) {
+    int new_start = s0, new_end = e0;
+    int p_out_start = base + new_start;
+    const int sl = where_is(g, p, p_out_start);
+    if (sl != L_INSIDE) {
+        if (sl == L_OUTSIDE) substitute(g, p, base + new_start + 1, p_out_start);
+        if (dist(p, p_out_start, p_out_start + 1) - g.step_cutoff < kZero) {
+            p.copy(p_out_start + 1, p_out_start);
+            new_start++;
+            p_out_start++;
+        }
+        const int b = boundary_of(g, p, p_out_start);
+        if (b < 0) return WIN_NOT_AT_BOUNDARY;
+        if (o.nev >= kMaxEv) return WIN_CAPACITY;
+        ev[o.nev++] = pack_event(p_out_start, b, o.segments);
+    }
+    int p_out_end = base + new_end;
+    if (end_loc != L_INSIDE) {
+        if (end_loc == L_OUTSIDE) substitute(g, p, base + new_end - 1, p_out_end);
+        if (dist(p, p_out_end - 1, p_out_end) - g.step_cutoff < kZero) {
+            p.copy(p_out_end - 1, p_out_end);
+            new_end--;
+            p_out_end--;
+        }
+        const int b = boundary_of(g, p, p_out_end);
+        if (b < 0) return WIN_NOT_AT_BOUNDARY;
+        if (o.nev >= kMaxEv) return WIN_CAPACITY;
+        ev[o.nev++] = pack_event(p_out_end, b, o.segments);
+    }
+    if (o.segments == 0) {
+        o.first = new_start;
+        o.last = new_end;
+    } else {
+        if (!allow_pieces) return WIN_INTERNAL;
+        if (o.segments >= kMaxSeg) return WIN_CAPACITY;
+        int sh0 = 0;
+        for (int j = new_start; j <= new_end; j++) {
+            p.flag[base + j] = -o.segments;
+            sh0 |= in_shell0(g, p, base + j) ? 1 : 0;
+        }
+        int32_t* sl3 = slots + 3 * (o.segments - 1);
+        sl3[0] = base + new_start;
+        sl3[1] = base + new_end;
+        sl3[2] = sh0;
+    }
+    o.segments++;
+    return WIN_OK;
+}
+
+// Trim_boundary_cnts for one CNT whose points are the run base .. base + n - 1.  Upstream
+// visits the points one by one, but only a point outside that follows one that is not ends a
+// segment (two points outside in a row leave none between them and min_points >= 2), and the
+// points a segment moves are not looked at again as ends: the walk depends on the original
+// points' in/out bits alone.  TrimWalk takes them in blocks of 32 (bit k: point first + k is
+// outside), so a warp can find the bits in parallel.
+struct TrimWalk {
+    int start = 0;
+    bool start_out = false;  // the point at `start` is outside (else start = 0 and the first point is not)
+    bool prev_out = false;
+    int err = WIN_OK;
+
+    __host__ __device__ void block(const WinGeom& g, const Pts& p, int base, int first, uint32_t out, bool allow_pieces, TrimOut& o,
+                                   int32_t* slots, int64_t* ev) {
+        if (first == 0) {
+            start_out = prev_out = (out & 1u) != 0;
+        }
+        for (int k = first == 0 ? 1 : 0; k < 32 && err == WIN_OK; k++) {
+            if (!(out >> k)) {  // no more points outside in this block
+                prev_out = false;
+                return;
+            }
+            const bool now = (out >> k & 1u) != 0;
+            if (now) {
+                const int end = first + k;
+                if (!prev_out) {
+                    const int n_points = start_out ? end - start - 1 : end - start;
+                    if (n_points >= g.min_points) err = add_segment(g, p, base, start, end, L_OUTSIDE, allow_pieces, o, slots, ev);
+                }
+                start = end;
+                start_out = true;
+            }
+            prev_out = now;
+        }
+    }
+    // after the last block: last_loc is where the last point is
+    __host__ __device__ int finish(const WinGeom& g, const Pts& p, int base, int n, int last_loc, bool allow_pieces, TrimOut& o, int32_t* slots,
+                                   int64_t* ev) {
+        if (err != WIN_OK) return err;
+        if (last_loc != L_OUTSIDE && n - start >= g.min_points)
+            return add_segment(g, p, base, start, n - 1, n > 1 ? last_loc : L_INSIDE, allow_pieces, o, slots, ev);
+        return WIN_OK;
+    }
+};
+
 __host__ __device__ inline int trim_run(const WinGeom& g, const Pts& p, int base, int n, bool allow_pieces, TrimOut& o, int32_t* slots,
                                         int64_t* ev) {
-    int start = 0, end = 0, last_inside = 0;
-    int point_location = L_INSIDE;
-    const int first_loc = where_is(g, p, base);
-    // Add_cnt_segment_to_structure
-    auto add_segment = [&](int s0, int e0, int end_loc) -> int {
-        int new_start = s0, new_end = e0;
-        int p_out_start = base + new_start;
-        const int sl = where_is(g, p, p_out_start);
-        if (sl != L_INSIDE) {
-            if (sl == L_OUTSIDE) substitute(g, p, base + new_start + 1, p_out_start);
-            if (dist(p, p_out_start, p_out_start + 1) - g.step_cutoff < kZero) {
-                p.copy(p_out_start + 1, p_out_start);
-                new_start++;
-                p_out_start++;
-            }
-            const int b = boundary_of(g, p, p_out_start);
-            if (b < 0) return WIN_NOT_AT_BOUNDARY;
-            if (o.nev >= kMaxEv) return WIN_CAPACITY;
-            ev[o.nev++] = pack_event(p_out_start, b, o.segments);
-        }
-        int p_out_end = base + new_end;
-        if (end_loc != L_INSIDE) {
-            if (end_loc == L_OUTSIDE) substitute(g, p, base + new_end - 1, p_out_end);
-            if (dist(p, p_out_end - 1, p_out_end) - g.step_cutoff < kZero) {
-                p.copy(p_out_end - 1, p_out_end);
-                new_end--;
-                p_out_end--;
-            }
-            const int b = boundary_of(g, p, p_out_end);
-            if (b < 0) return WIN_NOT_AT_BOUNDARY;
-            if (o.nev >= kMaxEv) return WIN_CAPACITY;
-            ev[o.nev++] = pack_event(p_out_end, b, o.segments);
-        }
-        if (o.segments == 0) {
-            o.first = new_start;
-            o.last = new_end;
-        } else {
-            if (!allow_pieces) return WIN_INTERNAL;
-            if (o.segments >= kMaxSeg) return WIN_CAPACITY;
-            int sh0 = 0;
-            for (int j = new_start; j <= new_end; j++) {
-                p.flag[base + j] = -o.segments;
-                sh0 |= in_shell0(g, p, base + j) ? 1 : 0;
-            }
-            int32_t* sl3 = slots + 3 * (o.segments - 1);
-            sl3[0] = base + new_start;
-            sl3[1] = base + new_end;
-            sl3[2] = sh0;
-        }
-        o.segments++;
-        return WIN_OK;
-    };
-    for (int j = 1; j < n; j++) {
-        point_location = where_is(g, p, base + j);
-        if (point_location != L_OUTSIDE) {
-            last_inside = j;
-        } else {
-            end = j;
-            const int n_points = (start == 0 && first_loc != L_OUTSIDE) ? end - start : end - start - 1;
-            if (n_points >= g.min_points) {
-                const int e = add_segment(start, end, point_location);
-                if (e) return e;
-            }
-            start = j;
-        }
+    TrimWalk w;
+    const int last_loc = where_is(g, p, base + n - 1);
+    for (int first = 0; first < n; first += 32) {
+        uint32_t out = 0;
+        for (int k = 0; k < 32 && first + k < n; k++) out |= (uint32_t)(where_is(g, p, base + first + k) == L_OUTSIDE) << k;
+        w.block(g, p, base, first, out, allow_pieces, o, slots, ev);
     }
-    if (last_inside == n - 1 && (last_inside - start + 1) >= g.min_points) {
-        end = n - 1;
-        const int e = add_segment(start, end, point_location);
-        if (e) return e;
-    }
-    return WIN_OK;
+    return w.finish(g, p, base, n, last_loc, allow_pieces, o, slots, ev);
 }
 
 // Window 0 and the shell geometry: Geom_sample::update_observation_window_geometry(0, ...)
