@@ -207,7 +207,7 @@ cicy_status cicy_network_to_conductance(cicy_ctx* ctx, const cicy_params* p, cic
         cudaEvent_t ev[4];
         for (auto& e : ev) CICY_CUDA(cudaEventCreate(&e));
         CICY_CUDA(cudaEventRecord(ev[0], c.stream));
-        cicy::run_contact_grid(c, *p);
+        cicy::run_contact_grid(c, *p, false);
         CICY_CUDA(cudaEventRecord(ev[1], c.stream));
         cicy::run_clusters(c, *p);
         CICY_CUDA(cudaEventRecord(ev[2], c.stream));

@@ -22,7 +22,7 @@ struct GridGeom {
 // size is read by waiting for the stream instead of by a copy to pageable memory as well.
 // Registering a page costs about 2.5 ms, so contexts share pages of 32 slots (stage_clusters.cu);
 // a page is freed with its last slot, but for one that is kept for the next context.
-enum HostWord : int { W_READ = 0, W_STATUS = 1, W_NODES = 2, W_NNZ = 3, W_RESID = 4 /* two */, W_WIN = 8, W_COUNT = 16 };
+enum HostWord : int { W_READ = 0, W_STATUS = 1, W_NODES = 2, W_NNZ = 3, W_RESID = 4 /* two */, W_WIN = 8, W_CLU = 16, W_COUNT = 32 };
 int64_t* host_words_take();
 void host_words_return(int64_t* slot);
 struct HostWords {
@@ -125,6 +125,7 @@ struct Ctx {
 
     // ---- network (device) ----
     int n_points = 0, n_cnts = 0, n_inside = 0, n_trav = 0;
+    double r_max = 0;  // largest CNT radius
     cicy_cuboid window{};
     DBuf<double> x, y, z, radii;
     DBuf<int32_t> flag, cstart, clen, inside, trav_off, trav_pt;
@@ -135,7 +136,8 @@ struct Ctx {
     // ---- grid ----
     GridGeom grid{};
     int n_slots = 0;
-    DBuf<int32_t> region_cnt, region_ptr, region_cur, slot_region, seg_large;
+    DBuf<int32_t> region_cnt, region_ptr, slot_region, seg_large;
+    DBuf<char> trav_reg;  // int4, ushort4 each traversal point: its regions (-1: none), its arrival number in them
     DBuf<uint32_t> slot_q, slot_sorted;
     DBuf<int> status;      // device status word (DevErr)
     DBuf<int32_t> i32_scalar;  // small device scalars for totals
@@ -143,10 +145,8 @@ struct Ctx {
 
     // ---- contacts / labels ----
     int n_raw = 0, n_uc = 0, n_labels = 0, n_junc = 0, n_perc = 0;
-    DBuf<int32_t> raw_a, raw_b, raw_pa, raw_pb;
-    DBuf<double> raw_d;
-    DBuf<uint64_t> raw_key;
-    DBuf<int32_t> raw_count;
+    DBuf<char> con_raw, con_of_cnt, con_seg;  // arrays of the contact visits, of each CNT's share of them, of its contacts
+    DBuf<int32_t> clu_words;
     DBuf<uint64_t> sort_k;
     DBuf<uint32_t> sort_v;
     DBuf<int32_t> flags, flags_scan;
@@ -154,11 +154,10 @@ struct Ctx {
     DBuf<double> uc_d;
     DBuf<int32_t> parent, uf_root, labels, root_rank;
     DBuf<unsigned long long> minkey;
-    DBuf<int32_t> grp_start, junc_cnt, junc_ofs;
     DBuf<int32_t> j_p1, j_n1, j_p2, j_n2;
     DBuf<double> j_d;
     DBuf<int32_t> mark, mark_scan, elem_idx, has_junc;
-    DBuf<int32_t> face_bits, perc_bits, perc_index;
+    DBuf<int32_t> face_bits, perc_bits, perc_index, perc_fam;
     std::vector<int32_t> h_family;  // family of each percolated cluster
     DBuf<int32_t> clu_ptr, clu_idx, cj_ptr, cj_idx;          // percolated clusters (after percolation)
     std::vector<int32_t> h_clu_ptr, h_cj_ptr;
@@ -243,7 +242,8 @@ void upload_network(Ctx& c, const cicy_network& net);
 // Network construction on the device (stage_window.cu).
 void generate_network_device(Ctx& c, const cicy_gen_params& g);
 void extract_window_device(Ctx& c, const cicy_window_params& w);
-void run_contact_grid(Ctx& c, const cicy_params& p);
+// wait: return once the grid is complete (else the next stage reports its errors).
+void run_contact_grid(Ctx& c, const cicy_params& p, bool wait = true);
 void run_clusters(Ctx& c, const cicy_params& p);
 void run_electrical(Ctx& c, const cicy_params& p, cicy_result* out);
 // Clusters and percolation of a mixed CNT/GNP network (mixed_percolation.cu).

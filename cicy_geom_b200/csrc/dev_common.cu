@@ -77,8 +77,9 @@ __global__ void k_scan_blocks(T* bsum, int nb, T* total) {
 
 // kSums: bsum holds the tiles' sums and every block adds up those before its own (at most
 // kScanTilesMax of them, read from L2); else bsum is already scanned.
+// marked: with it, marked[out[j]] = j for every j whose input is not zero.
 template <class T, bool kSums>
-__global__ void k_scan_apply(const T* in, T* out, int n, const T* __restrict__ bsum, T* total) {
+__global__ void k_scan_apply(const T* in, T* out, int n, const T* __restrict__ bsum, T* total, int32_t* __restrict__ marked) {
     __shared__ T sw[33];
     __shared__ T before;
     if constexpr (kSums) {
@@ -105,7 +106,10 @@ __global__ void k_scan_apply(const T* in, T* out, int n, const T* __restrict__ b
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) {
         long long j = base + i;
-        if (j < n) out[j] = ex;
+        if (j < n) {
+            out[j] = ex;
+            if (marked && v[i] != T(0)) marked[ex] = (int32_t)j;
+        }
         ex += v[i];
     }
     if (kSums && total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = before + tot;
@@ -116,7 +120,7 @@ __global__ void k_scan_apply(const T* in, T* out, int n, const T* __restrict__ b
 constexpr int kScanSmallItems = 16;
 constexpr int kScanSmallMax = 1024 * kScanSmallItems;
 template <class T>
-__global__ void __launch_bounds__(1024) k_scan_small(const T* in, T* out, int n, T* total) {
+__global__ void __launch_bounds__(1024) k_scan_small(const T* in, T* out, int n, T* total, int32_t* __restrict__ marked) {
     __shared__ T sw[33];
     const int ch = (n + 1023) / 1024;
     const int lo = min(n, (int)threadIdx.x * ch), hi = min(n, lo + ch);
@@ -133,19 +137,20 @@ __global__ void __launch_bounds__(1024) k_scan_small(const T* in, T* out, int n,
     for (int i = 0; i < kScanSmallItems; i++)
         if (lo + i < hi) {
             out[lo + i] = ex;
+            if (marked && v[i] != T(0)) marked[ex] = lo + i;
             ex += v[i];
         }
     if (threadIdx.x == 0 && total) *total = tot;
 }
 
 template <class T>
-void exclusive_scan_impl(const T* in, T* out, int n, T* total, DBuf<T>& tmp, cudaStream_t s, int64_t& launches) {
+void exclusive_scan_impl(const T* in, T* out, int n, T* total, DBuf<T>& tmp, cudaStream_t s, int64_t& launches, int32_t* marked = nullptr) {
     if (n <= 0) {
         if (total) CICY_CUDA(cudaMemsetAsync(total, 0, sizeof(T), s));
         return;
     }
     if (n <= kScanSmallMax) {
-        k_scan_small<T><<<1, 1024, 0, s>>>(in, out, n, total);
+        k_scan_small<T><<<1, 1024, 0, s>>>(in, out, n, total, marked);
         launches++;
         CICY_LAUNCH_CHECK();
         return;
@@ -154,11 +159,11 @@ void exclusive_scan_impl(const T* in, T* out, int n, T* total, DBuf<T>& tmp, cud
     tmp.ensure(nb + 1);
     k_scan_reduce<T><<<nb, kScanThreads, 0, s>>>(in, n, tmp.get());
     if (nb <= kScanTilesMax) {
-        k_scan_apply<T, true><<<nb, kScanThreads, 0, s>>>(in, out, n, tmp.get(), total);
+        k_scan_apply<T, true><<<nb, kScanThreads, 0, s>>>(in, out, n, tmp.get(), total, marked);
         launches += 2;
     } else {
         k_scan_blocks<T><<<1, 1024, 0, s>>>(tmp.get(), nb, total);
-        k_scan_apply<T, false><<<nb, kScanThreads, 0, s>>>(in, out, n, tmp.get(), total);
+        k_scan_apply<T, false><<<nb, kScanThreads, 0, s>>>(in, out, n, tmp.get(), total, marked);
         launches += 3;
     }
     CICY_LAUNCH_CHECK();
@@ -234,31 +239,32 @@ __global__ void k_radix_scatter(const uint64_t* __restrict__ kin, const uint32_t
 }
 
 // ---------------- segmented sort ----------------
-__global__ void k_segsort_warp(const int32_t* __restrict__ ptr, int n_seg, const uint32_t* __restrict__ keys,
-                               uint32_t* __restrict__ out, int32_t* large_list, int32_t* large_count, int* status) {
-    const int lane = threadIdx.x & 31;
-    long long wg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long sgi = wg; sgi < n_seg; sgi += nw) {
-        int b = ptr[sgi], e = ptr[sgi + 1], len = e - b;
-        if (len <= 1) {
-            if (len == 1 && lane == 0) out[b] = keys[b];
-            continue;
-        }
-        if (len > 32) {
+// Eight threads per segment: segments are grid regions of three points on average, and a warp for
+// each left most lanes idle (1.7 M regions: 114 us, now 80 us).  Each key's rank is the number of
+// smaller keys of its segment; seg_of gets the segment of every slot.
+constexpr int kSegLanes = 8;
+constexpr int kSegSmall = 32;
+__global__ void k_segsort_small(const int32_t* __restrict__ ptr, int n_seg, const uint32_t* __restrict__ keys, uint32_t* __restrict__ out,
+                                int32_t* __restrict__ seg_of, int32_t* large_list, int32_t* large_count, int* status) {
+    const int lane = threadIdx.x % kSegLanes;
+    const long long step = (long long)gridDim.x * blockDim.x / kSegLanes;
+    for (long long sgi = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / kSegLanes; sgi < n_seg; sgi += step) {
+        const int b = ptr[sgi], len = ptr[sgi + 1] - b;
+        if (len > kSegSmall) {
             if (lane == 0) {
                 if (len > kSegSortMax) atomicCAS(status, 0, (int)DEV_CAPACITY);
                 else large_list[atomicAdd(large_count, 1)] = (int32_t)sgi;
             }
+            for (int i = lane; i < len; i += kSegLanes) seg_of[b + i] = (int32_t)sgi;
             continue;
         }
-        uint32_t k = lane < len ? keys[b + lane] : 0xffffffffu;
-        int rank = 0;
-        for (int t = 0; t < len; t++) {
-            uint32_t o = __shfl_sync(0xffffffffu, k, t);
-            rank += (o < k) ? 1 : 0;
+        for (int i = lane; i < len; i += kSegLanes) {
+            const uint32_t k = keys[b + i];
+            int rank = 0;
+            for (int t = 0; t < len; t++) rank += keys[b + t] < k ? 1 : 0;
+            out[b + rank] = k;
+            seg_of[b + i] = (int32_t)sgi;
         }
-        if (lane < len) out[b + rank] = k;
     }
 }
 
@@ -286,6 +292,11 @@ __global__ void k_segsort_block(const int32_t* __restrict__ ptr, const uint32_t*
 void exclusive_scan_i32(const int32_t* in, int32_t* out, int n, int32_t* total, DBuf<int32_t>& tmp, cudaStream_t s,
                         int64_t& launches) {
     exclusive_scan_impl<int32_t>(in, out, n, total, tmp, s, launches);
+}
+
+void exclusive_scan_flags_i32(const int32_t* in, int32_t* out, int n, int32_t* total, int32_t* marked, DBuf<int32_t>& tmp, cudaStream_t s,
+                              int64_t& launches) {
+    exclusive_scan_impl<int32_t>(in, out, n, total, tmp, s, launches, marked);
 }
 
 void exclusive_scan_i64(const int64_t* in, int64_t* out, int n, int64_t* total, DBuf<int64_t>& tmp, cudaStream_t s,
@@ -407,12 +418,12 @@ void radix_sort_pairs(uint64_t* keys, uint32_t* vals, int n, int bits, RadixScra
     }
 }
 
-void segmented_sort_u32(const int32_t* ptr, int n_seg, const uint32_t* keys, uint32_t* out, int32_t* large_list,
+void segmented_sort_u32(const int32_t* ptr, int n_seg, const uint32_t* keys, uint32_t* out, int32_t* seg_of, int32_t* large_list,
                         int32_t* large_count, int* status, cudaStream_t s, int64_t& launches) {
     if (n_seg <= 0) return;
     CICY_CUDA(cudaMemsetAsync(large_count, 0, sizeof(int32_t), s));
-    int blocks = std::min(ceil_div((long long)n_seg * 32, 256), 148 * 16);
-    k_segsort_warp<<<blocks, 256, 0, s>>>(ptr, n_seg, keys, out, large_list, large_count, status);
+    int blocks = std::min(ceil_div((long long)n_seg * kSegLanes, 256), 148 * 16);
+    k_segsort_small<<<blocks, 256, 0, s>>>(ptr, n_seg, keys, out, seg_of, large_list, large_count, status);
     k_segsort_block<<<148 * 2, 256, 0, s>>>(ptr, keys, out, large_list, large_count);
     launches += 2;
     CICY_LAUNCH_CHECK();

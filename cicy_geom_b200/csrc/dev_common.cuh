@@ -77,12 +77,29 @@ struct DBuf {
     T* get() const { return p; }
 };
 
+// Several arrays in one allocation (an allocation costs a new context's first pass 10-20 us): take
+// the arrays of Carver{} for the size, then those of Carver{base}, in the same order.
+struct Carver {
+    char* base = nullptr;
+    size_t at = 0;
+    template <class T>
+    T* take(size_t n) {
+        at = (at + 255) & ~(size_t)255;
+        T* r = base ? reinterpret_cast<T*>(base + at) : nullptr;
+        at += n * sizeof(T);
+        return r;
+    }
+};
+
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 // ---------------------------------------------------------------------------
 // Exclusive scan of int32 counts (out may alias in). `total` (device) gets the sum.
 void exclusive_scan_i32(const int32_t* in, int32_t* out, int n, int32_t* total, DBuf<int32_t>& tmp, cudaStream_t s,
                         int64_t& launches);
+// The same over 0/1 flags, with the list of the flagged positions: marked[out[j]] = j.
+void exclusive_scan_flags_i32(const int32_t* in, int32_t* out, int n, int32_t* total, int32_t* marked, DBuf<int32_t>& tmp, cudaStream_t s,
+                              int64_t& launches);
 // Exclusive scan of int64 values.
 void exclusive_scan_i64(const int64_t* in, int64_t* out, int n, int64_t* total, DBuf<int64_t>& tmp, cudaStream_t s,
                         int64_t& launches);
@@ -98,10 +115,11 @@ struct RadixScratch {
 void radix_sort_pairs(uint64_t* keys, uint32_t* vals, int n, int bits, RadixScratch& rs, cudaStream_t s, int64_t& launches);
 
 // Sorts each segment [ptr[i], ptr[i+1]) of `keys` ascending (keys unique within a
-// segment) into `out`, carrying nothing else: out holds the sorted keys.
+// segment) into `out`, carrying nothing else: out holds the sorted keys; seg_of[j] = the
+// segment of position j.
 // Segments longer than kSegSortMax set the capacity flag in *status.
 constexpr int kSegSortMax = 8192;
-void segmented_sort_u32(const int32_t* ptr, int n_seg, const uint32_t* keys, uint32_t* out, int32_t* large_list,
+void segmented_sort_u32(const int32_t* ptr, int n_seg, const uint32_t* keys, uint32_t* out, int32_t* seg_of, int32_t* large_list,
                         int32_t* large_count, int* status, cudaStream_t s, int64_t& launches);
 
 int bits_for(uint64_t max_value);

@@ -458,6 +458,7 @@ void generate_network_device(Ctx& c, const cicy_gen_params& g) {
     c.n_inside = 0;
     c.n_trav = 0;
     c.window = g.sample;
+    c.r_max = nc > 0 ? std::fmax(0.0, g.radius) : 0;
     c.h_bcnt_ptr.assign(7, 0);
     c.h_bpts_ptr.assign(7, 0);
     c.bcnt_ptr.ensure(7); c.bpts_ptr.ensure(7);
