@@ -445,6 +445,253 @@ __global__ void __launch_bounds__(kClusterThreads) k_pcg_cluster(ClusterArgs a) 
     cl.sync();  // no CTA exits while others may still access its shared memory
 }
 
+// ---------------------------------------------------------------------------
+// Jacobi-PCG in the registers of one to eight CTAs.
+//
+// A Jacobi iteration of a few thousand rows is bound by its two reductions, and between 16 CTAs
+// each costs a wide cluster barrier and a round of remote stores: 3.6 us an iteration whatever the
+// size.  Here a thread owns up to eight rows, with their r, q, p, x, 1/diag and matrix entries in
+// registers (kCtaWidth of them; one row in a hundred has more, read from memory), and every CTA's
+// shared memory holds z of all rows, which their owners write there.  Two barriers an iteration: one
+// publishes the partials of p.q, one those of r.r and r.z together with the new z.  Every warp adds
+// the partials in the same order, so no scalar is broadcast and all CTAs decide alike.  Same
+// recurrence, stopping test and restarts as k_pcg_cluster.
+//
+// Iterations on one CTA: 0.7 us at 130 rows, 0.97 at 810, 1.15 at 1,500 (512 threads: 0.95, 1.09,
+// 1.31; 1,024: 1.6-2.5: fewer warps to add up, and with several rows a thread the loads of z
+// overlap).  A system takes the fewest CTAs whose registers hold it, but four from 3,073 rows: two
+// take 1.75 us at 2,500 rows (four 1.95) and 2.3 at 3,500 (four 2.1).  Four take 2.55 at 5,600, eight
+// 3.7-4.0 at 10,000 rows; the 16-CTA kernel 3.5, 3.6, 3.7 and 4.6.  Above kCtaMax that one is
+// faster (15,500 rows: 5.1 us, eight CTAs 5.6).
+constexpr int kCtaThreads = 256;
+constexpr int kCtaWidth = 5;
+constexpr int kCtaMax = kCtaThreads * 6 * 8;
+
+struct CtaArgs {
+    int n;
+    const int32_t *rp, *ci;
+    const double *val, *b, *diag;
+    double* x;
+    double tol;
+    long long max_iter;
+    int max_restarts;
+    double* stats;
+};
+
+template <int R, int C>
+__global__ void __launch_bounds__(kCtaThreads, 1) k_pcg_cta(CtaArgs a) {
+    constexpr int T = kCtaThreads, W = kCtaWidth, S = C * T / 32;
+    static_assert((S & (S - 1)) == 0 && S <= 64, "total");
+    extern __shared__ __align__(16) double zs[];  // z of all rows
+    __shared__ double slot[3][S];
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = C > 1 ? cl.block_rank() : 0, t = threadIdx.x, n = a.n;
+    auto row = [&](int j) { return (j * C + rank) * T + t; };
+    auto sync = [&]() {
+        if constexpr (C > 1) cl.sync();
+        else __syncthreads();
+    };
+    double* zr[C];  // the other CTAs' z
+#pragma unroll
+    for (int c = 0; c < C; c++) zr[c] = C > 1 ? cl.map_shared_rank(zs, (rank + c) % C) : zs;
+    auto put = [&](int j, double z) {
+        if (row(j) < n) {
+#pragma unroll
+            for (int c = 0; c < C; c++) zr[c][row(j)] = z;
+        }
+    };
+    // Sums over all CTAs: partials by warp_sum into everyone's slots, then, after the barrier, all warps alike.
+    double* const slot_r = C > 1 ? cl.map_shared_rank(&slot[0][0], t & (C - 1)) : &slot[0][0];
+    auto store = [&](int k, double v) {
+        v = warp_sum(v);                                         // lane 0's
+        if constexpr (C > 1) v = __shfl_sync(0xffffffffu, v, 0);  // lane c writes CTA c's slot
+        if ((t & 31) < C) slot_r[k * S + rank * (T / 32) + (t >> 5)] = v;
+    };
+    auto total = [&](int k) {
+        double v = slot[k][t & (S < 32 ? S - 1 : 31)];
+        if constexpr (S > 32) v += slot[k][32 + (t & 31)];
+#pragma unroll
+        for (int o = (S < 32 ? S : 32) / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    };
+    double v[R][W], r[R], p[R], q[R], x[R], ip[R];
+    uint32_t col[R][(W + 1) / 2];  // two 16-bit columns a word
+    unsigned tail = 0;             // rows with more than kCtaWidth entries
+#pragma unroll
+    for (int j = 0; j < R; j++) {
+        const int i = row(j);
+        const bool in = i < n;
+        const int k0 = in ? a.rp[i] : 0, len = in ? a.rp[i + 1] - k0 : 0;
+        if (len > W) tail |= 1u << j;
+#pragma unroll
+        for (int h = 0; h < (W + 1) / 2; h++) col[j][h] = 0;
+#pragma unroll
+        for (int k = 0; k < W; k++) {
+            v[j][k] = k < len ? a.val[k0 + k] : 0.0;
+            const uint32_t c = k < len ? a.ci[k0 + k] : in ? i : 0;
+            col[j][k / 2] |= c << (16 * (k & 1));
+        }
+        x[j] = in ? a.x[i] : 0.0;
+        ip[j] = in ? 1.0 / a.diag[i] : 0.0;
+        r[j] = p[j] = q[j] = 0;
+    }
+    // row j of A zs
+    auto product = [&](int j) {
+        double w = 0;
+#pragma unroll
+        for (int k = 0; k < W; k++) w += v[j][k] * zs[(col[j][k / 2] >> (16 * (k & 1))) & 0xffffu];
+        if (tail >> j & 1)
+            for (int k = a.rp[row(j)] + W; k < a.rp[row(j) + 1]; k++) w += a.val[k] * zs[a.ci[k]];
+        return w;
+    };
+    sync();  // every CTA of the cluster runs: its shared memory can be written
+    // r = b - A x, z = r / diag, and the partials of r.r and r.z
+    auto residual = [&]() {
+#pragma unroll
+        for (int j = 0; j < R; j++) put(j, x[j]);
+        sync();
+#pragma unroll
+        for (int j = 0; j < R; j++) r[j] = row(j) < n ? a.b[row(j)] - product(j) : 0.0;
+        sync();
+        double rr = 0, rz = 0;
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const double z = r[j] * ip[j];
+            put(j, z);
+            rr += r[j] * r[j];
+            rz += r[j] * z;
+        }
+        store(0, rr);
+        store(1, rz);
+        sync();
+    };
+    residual();
+    double rr = total(0), rz = total(1);
+    const double R0 = a.tol * sqrt(rr), R0sq = R0 * R0;
+    double beta = 0;
+    long long k = 0;
+    int restarts = 0;
+    bool fresh = true;
+    while (true) {
+        // ---- A: w = A z, q = w + beta q, p = z + beta p, partial p.q
+        double pq = 0;
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const double w = product(j), z = r[j] * ip[j];
+            q[j] = fresh ? w : w + beta * q[j];
+            p[j] = fresh ? z : z + beta * p[j];
+            pq += p[j] * q[j];
+        }
+        store(2, pq);
+        sync();  // the partials of p.q; zs and the slots of r.r, r.z have been read
+        const double alpha = rz / total(2);
+        fresh = false;
+        k++;
+        // ---- B: r -= alpha q, z = r / diag, x += alpha p, partials r.r, r.z
+        double rr_l = 0, rz_l = 0;
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            r[j] -= alpha * q[j];
+            const double z = r[j] * ip[j];
+            put(j, z);
+            rr_l += r[j] * r[j];
+            rz_l += r[j] * z;
+        }
+        store(0, rr_l);
+        store(1, rz_l);
+#pragma unroll
+        for (int j = 0; j < R; j++) x[j] += alpha * p[j];
+        sync();  // z and the partials; the slots of p.q have been read
+        rr = total(0);
+        const double rz_new = total(1);
+        beta = rz_new / rz;
+        rz = rz_new;
+        if (rr <= R0sq) {
+            if (restarts >= a.max_restarts) break;
+            sync();           // every slot has been read
+            residual();       // FP64 true residual
+            rr = total(0);
+            rz = total(1);
+            restarts++;
+            if (rr <= R0sq) break;
+            fresh = true;
+        }
+        if (k >= a.max_iter) break;
+    }
+#pragma unroll
+    for (int j = 0; j < R; j++)
+        if (row(j) < n) a.x[row(j)] = x[j];
+    if (rank == 0 && t == 0) {
+        a.stats[0] = (double)k;
+        a.stats[1] = rr;
+        a.stats[2] = sqrt(R0sq);
+        a.stats[3] = (double)restarts;
+    }
+}
+
+// Launches `solve` between two events, waits and reads its statistics.
+template <class F>
+void timed_solve(SolverWork& w, cudaStream_t s, int64_t& launches, PcgStats& st, F solve) {
+    cudaEvent_t e0, e1;
+    CICY_CUDA(cudaEventCreate(&e0));
+    CICY_CUDA(cudaEventCreate(&e1));
+    CICY_CUDA(cudaEventRecord(e0, s));
+    solve();
+    CICY_CUDA(cudaEventRecord(e1, s));
+    launches++;
+    double hs[4];
+    CICY_CUDA(cudaMemcpyAsync(hs, w.stats.get(), sizeof(hs), cudaMemcpyDeviceToHost, s));
+    CICY_CUDA(cudaStreamSynchronize(s));
+    float ms = 0;
+    cudaEventElapsedTime(&ms, e0, e1);
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    st.iterations = (long long)hs[0];
+    st.restarts = (int)hs[3];
+    st.seconds = ms * 1e-3;
+    st.cluster = true;
+}
+
+template <int R, int C>
+void launch_pcg_cta(const CtaArgs& a, cudaStream_t s, PcgStats& st) {
+    CICY_CUDA(cudaFuncSetAttribute(k_pcg_cta<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(double) * kCtaThreads * R * C));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(kCtaThreads);
+    cfg.dynamicSmemBytes = sizeof(double) * a.n;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = C > 1 ? 1 : 0;
+    CICY_CUDA(cudaLaunchKernelEx(&cfg, k_pcg_cta<R, C>, a));
+    st.ctas = C;
+}
+
+void pcg_solve_cta(SolverWork& w, const SolverSystem& sys, double tol, long long max_iter, cudaStream_t s, int64_t& launches, PcgStats& st) {
+    w.stats.ensure(4);
+    const CtaArgs a{sys.n, sys.rp, sys.ci, sys.val, sys.b, sys.diag, sys.x, tol, max_iter, 24, w.stats.get()};
+    timed_solve(w, s, launches, st, [&] {
+        switch (ceil_div(sys.n, kCtaThreads)) {
+            case 1: return launch_pcg_cta<1, 1>(a, s, st);
+            case 2: return launch_pcg_cta<2, 1>(a, s, st);
+            case 3: return launch_pcg_cta<3, 1>(a, s, st);
+            case 4: return launch_pcg_cta<4, 1>(a, s, st);
+            case 5: return launch_pcg_cta<5, 1>(a, s, st);
+            case 6: return launch_pcg_cta<6, 1>(a, s, st);
+            case 7: case 8: return launch_pcg_cta<8, 1>(a, s, st);
+            case 9: case 10: case 11: case 12: return launch_pcg_cta<6, 2>(a, s, st);
+            case 13: case 14: case 15: case 16: return launch_pcg_cta<4, 4>(a, s, st);
+            case 17: case 18: case 19: case 20: case 21: case 22: case 23: case 24: return launch_pcg_cta<6, 4>(a, s, st);
+            case 25: case 26: case 27: case 28: case 29: case 30: case 31: case 32: return launch_pcg_cta<8, 4>(a, s, st);
+            default: return launch_pcg_cta<6, 8>(a, s, st);
+        }
+    });
+}
+
 }  // namespace
 
 bool pcg_solve_cluster(SolverWork& w, const SolverSystem& sys, bool block_precond, const float* node_scale,
@@ -455,6 +702,10 @@ bool pcg_solve_cluster(SolverWork& w, const SolverSystem& sys, bool block_precon
     st = PcgStats{};
     if (n <= 0) return true;
     if (n < 4 * C || n >= (1 << 16) * C / 2) return false;
+    if (!block_precond && n <= kCtaMax) {
+        pcg_solve_cta(w, sys, tol, max_iter, s, launches, st);
+        return true;
+    }
     static int attr_state = 0;  // 0 unknown, 1 ok, -1 unsupported
     if (attr_state == 0) {
         cudaError_t e1 = cudaFuncSetAttribute(k_pcg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -567,25 +818,8 @@ bool pcg_solve_cluster(SolverWork& w, const SolverSystem& sys, bool block_precon
         return false;
     }
     tr.mark("cluster.occupancy");
-    cudaEvent_t e0, e1;
-    CICY_CUDA(cudaEventCreate(&e0));
-    CICY_CUDA(cudaEventCreate(&e1));
-    CICY_CUDA(cudaEventRecord(e0, s));
-    CICY_CUDA(cudaLaunchKernelEx(&cfg, k_pcg_cluster, a));
-    CICY_CUDA(cudaEventRecord(e1, s));
-    launches++;
-    double hs[4];
-    CICY_CUDA(cudaMemcpyAsync(hs, w.stats.get(), sizeof(hs), cudaMemcpyDeviceToHost, s));
-    CICY_CUDA(cudaStreamSynchronize(s));
-    float ms = 0;
-    cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    st.iterations = (long long)hs[0];
-    st.restarts = (int)hs[3];
-    st.seconds = ms * 1e-3;
+    timed_solve(w, s, launches, st, [&] { CICY_CUDA(cudaLaunchKernelEx(&cfg, k_pcg_cluster, a)); });
     st.ctas = C;
-    st.cluster = true;
     return true;
 }
 
