@@ -161,6 +161,45 @@ __global__ void k_block_inverse(int nb, int n, const int32_t* __restrict__ blk_r
     }
 }
 
+// LDL^T factors of each preconditioner block: lfac[k] (multiplier of row k-1,
+// 0 at a block start; one 0 past the last row) and ipiv[k] = 1/pivot; Jacobi blocks have lfac = 0.
+// Learned scalings as in k_block_inverse.
+__global__ void k_block_factors(int nb, int n, const int32_t* __restrict__ blk_row, const int32_t* __restrict__ rp,
+                                const int32_t* __restrict__ ci, const double* __restrict__ v, const double* __restrict__ diag,
+                                const float* __restrict__ node_scale, const float* __restrict__ edge_scale,
+                                double* __restrict__ lfac, double* __restrict__ ipiv) {
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
+        const int r0 = blk_row[b];
+        const int m = ((b + 1 < nb) ? blk_row[b + 1] : n) - r0;
+        double e_prev = 0, piv_prev = 0;
+        bool singular = false;
+        for (int k = 0; k < m; k++) {
+            const int i = r0 + k;
+            double e = 0;
+            if (k + 1 < m)
+                for (int kk = rp[i]; kk < rp[i + 1]; kk++)
+                    if (ci[kk] == i + 1) { e = v[kk]; break; }
+            double coup = fabs(e) + fabs(e_prev);
+            double s = node_scale ? (double)node_scale[i] : 1.0;
+            double d = coup + s * (diag[i] - coup);
+            if (edge_scale && k + 1 < m) e *= (double)edge_scale[i];
+            double l = (k == 0) ? 0.0 : e_prev / piv_prev;
+            double piv = d - l * e_prev;
+            singular |= !(piv > 1e-13 * fabs(d));
+            lfac[i] = l;
+            ipiv[i] = 1.0 / piv;
+            e_prev = e;
+            piv_prev = piv;
+        }
+        if (b == nb - 1) lfac[n] = 0.0;
+        if (singular)  // a CNT decoupled from the rest of the system: diagonal instead
+            for (int k = 0; k < m; k++) {
+                lfac[r0 + k] = 0.0;
+                ipiv[r0 + k] = 1.0 / diag[r0 + k];
+            }
+    }
+}
+
 // CTA row ranges that never split a block: CTA b starts at the first block start
 // at or after b * n / nb.
 __global__ void k_cta_rows(int nb_cta, int n, const int32_t* __restrict__ is_start, int32_t* __restrict__ cta_row) {
@@ -441,9 +480,9 @@ __global__ void k_mixed_prep(int n, const int32_t* __restrict__ rp, const int32_
 }  // namespace
 
 // ---------------------------------------------------------------------------
-void build_block_preconditioner(SolverWork& w, const SolverSystem& sys, int nchains, const int32_t* chain_start,
-                                const int32_t* chain_len, const float* node_scale, const float* edge_scale, bool mixed,
-                                cudaStream_t s, int64_t& launches) {
+// Preconditioner blocks from the chains: starts, row of each block, their number.
+static int build_blocks(SolverWork& w, const SolverSystem& sys, int nchains, const int32_t* chain_start, const int32_t* chain_len,
+                        cudaStream_t s, int64_t& launches) {
     const int n = sys.n;
     w.total.ensure(2);
     w.is_start.ensure(n + 1);
@@ -455,9 +494,33 @@ void build_block_preconditioner(SolverWork& w, const SolverSystem& sys, int ncha
     CICY_CUDA(cudaMemcpyAsync(&nblk, w.total.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
     CICY_CUDA(cudaStreamSynchronize(s));
     w.blk_row.ensure(nblk + 1);
+    k_block_fill<<<grid_for(n), 256, 0, s>>>(n, w.is_start.get(), w.start_scan.get(), w.blk_row.get());
+    launches += 2;
+    w.n_blocks = nblk;
+    return nblk;
+}
+
+void launch_block_factors(SolverWork& w, const SolverSystem& sys, int nblk, const float* node_scale, const float* edge_scale, cudaStream_t s) {
+    w.lfac.ensure(sys.n + 1);
+    w.ipiv.ensure(sys.n);
+    k_block_factors<<<grid_for(nblk, 128), 128, 0, s>>>(nblk, sys.n, w.blk_row.get(), sys.rp, sys.ci, sys.val, sys.diag, node_scale, edge_scale,
+                                                       w.lfac.get(), w.ipiv.get());
+}
+
+void build_block_factors(SolverWork& w, const SolverSystem& sys, int nchains, const int32_t* chain_start, const int32_t* chain_len,
+                         cudaStream_t s, int64_t& launches) {
+    launch_block_factors(w, sys, build_blocks(w, sys, nchains, chain_start, chain_len, s, launches), nullptr, nullptr, s);
+    launches++;
+    CICY_LAUNCH_CHECK();
+}
+
+void build_block_preconditioner(SolverWork& w, const SolverSystem& sys, int nchains, const int32_t* chain_start,
+                                const int32_t* chain_len, const float* node_scale, const float* edge_scale, bool mixed,
+                                cudaStream_t s, int64_t& launches) {
+    const int n = sys.n;
+    const int nblk = build_blocks(w, sys, nchains, chain_start, chain_len, s, launches);
     w.blk_msq.ensure(nblk + 1);
     w.blk_off.ensure(nblk + 1);
-    k_block_fill<<<grid_for(n), 256, 0, s>>>(n, w.is_start.get(), w.start_scan.get(), w.blk_row.get());
     k_block_sizes<<<grid_for(nblk), 256, 0, s>>>(nblk, n, w.blk_row.get(), w.blk_msq.get());
     exclusive_scan_i32(w.blk_msq.get(), w.blk_off.get(), nblk, w.total.get(), w.scan_tmp, s, launches);
     // the blocks' m^2 entries sum to at most kBlockMax per row: sized by that bound, no host read
@@ -470,9 +533,8 @@ void build_block_preconditioner(SolverWork& w, const SolverSystem& sys, int ncha
     k_block_inverse<<<grid_for(nblk, 128), 128, 0, s>>>(nblk, n, w.blk_row.get(), w.blk_off.get(), sys.rp, sys.ci, sys.val, sys.diag,
                                                        node_scale, edge_scale, w.tinv.get(), mixed ? w.tinv32.get() : nullptr,
                                                        w.row_off.get(), w.row_base.get(), w.row_m.get());
-    launches += 4;
+    launches += 2;
     CICY_LAUNCH_CHECK();
-    w.n_blocks = nblk;
 }
 
 void pcg_solve(SolverWork& w, const SolverSystem& sys, int precond, bool mixed, double tol, long long max_iter, int num_sms,

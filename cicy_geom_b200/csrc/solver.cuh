@@ -103,7 +103,6 @@ struct MgWork {
         // r_l, P^T A_l on z_l) and prolongation-smoother rows of level l (A_l on z_l and on P zc)
         DBuf<int32_t> rr_ptr, rr_col, pq_ptr, pq_col;
         DBuf<double> rr_val, pq_val;
-        DBuf<double> r_cl, z_cl, zf_cl;  // per-cluster copies of the levels each cluster solves alone
     };
     std::vector<Lvl> L;
     std::vector<MgLevel> host_lv;
@@ -124,7 +123,6 @@ struct MgWork {
     bool dense = false;
     bool fused = false;  // fused rows built (build_mg_hierarchy with fused = true)
     bool smooth = true;  // with fused: level 1's prolongator smoothed (coarsen_smoothed)
-    DBuf<int32_t> cl_fail;
     DBuf<unsigned char> sec_lv;  // device descriptors of the clustered kernel
 };
 
@@ -179,6 +177,10 @@ void build_block_preconditioner(SolverWork& w, const SolverSystem& sys, int ncha
                                 const int32_t* chain_len, const float* node_scale, const float* edge_scale, bool mixed,
                                 cudaStream_t s, int64_t& launches);
 
+// The blocks and their LDL^T factors alone (the multigrid grid kernel's smoother).
+void build_block_factors(SolverWork& w, const SolverSystem& sys, int nchains, const int32_t* chain_start, const int32_t* chain_len,
+                         cudaStream_t s, int64_t& launches);
+void launch_block_factors(SolverWork& w, const SolverSystem& sys, int nblk, const float* node_scale, const float* edge_scale, cudaStream_t s);
 void launch_block_marks(int nchains, const int32_t* chain_start, const int32_t* chain_len, int32_t* is_start, cudaStream_t s);
 void launch_block_fill(int n, const int32_t* is_start, const int32_t* start_scan, int32_t* blk_row, cudaStream_t s);
 void launch_cta_rows(int nb_cta, int n, const int32_t* is_start, int32_t* cta_row, cudaStream_t s);

@@ -47,44 +47,6 @@ __device__ __forceinline__ int owner_of(const int32_t* __restrict__ cta_row, int
     return lo;
 }
 
-// LDL^T factors of each preconditioner block: lfac[k] (multiplier of row k-1,
-// 0 at a block start) and ipiv[k] = 1/pivot; Jacobi blocks have lfac = 0.
-// Learned scalings as in k_block_inverse (solver.cu).
-__global__ void k_block_factors(int nb, int n, const int32_t* __restrict__ blk_row, const int32_t* __restrict__ rp,
-                                const int32_t* __restrict__ ci, const double* __restrict__ v, const double* __restrict__ diag,
-                                const float* __restrict__ node_scale, const float* __restrict__ edge_scale,
-                                double* __restrict__ lfac, double* __restrict__ ipiv) {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-        const int r0 = blk_row[b];
-        const int m = ((b + 1 < nb) ? blk_row[b + 1] : n) - r0;
-        double e_prev = 0, piv_prev = 0;
-        bool singular = false;
-        for (int k = 0; k < m; k++) {
-            const int i = r0 + k;
-            double e = 0;
-            if (k + 1 < m)
-                for (int kk = rp[i]; kk < rp[i + 1]; kk++)
-                    if (ci[kk] == i + 1) { e = v[kk]; break; }
-            double coup = fabs(e) + fabs(e_prev);
-            double s = node_scale ? (double)node_scale[i] : 1.0;
-            double d = coup + s * (diag[i] - coup);
-            if (edge_scale && k + 1 < m) e *= (double)edge_scale[i];
-            double l = (k == 0) ? 0.0 : e_prev / piv_prev;
-            double piv = d - l * e_prev;
-            singular |= !(piv > 1e-13 * fabs(d));
-            lfac[i] = l;
-            ipiv[i] = 1.0 / piv;
-            e_prev = e;
-            piv_prev = piv;
-        }
-        if (singular)  // a CNT decoupled from the rest of the system: diagonal instead
-            for (int k = 0; k < m; k++) {
-                lfac[r0 + k] = 0.0;
-                ipiv[r0 + k] = 1.0 / diag[r0 + k];
-            }
-    }
-}
-
 // Per CTA: first preconditioner block and first non-zero.
 __global__ void k_cta_stats(int C, const int32_t* __restrict__ cta_row, const int32_t* __restrict__ rp, int nblk,
                             const int32_t* __restrict__ blk_row, int32_t* __restrict__ out) {
@@ -731,10 +693,7 @@ bool pcg_solve_cluster(SolverWork& w, const SolverSystem& sys, bool block_precon
     CICY_CUDA(cudaStreamSynchronize(s));
     w.blk_row.ensure(nblk + 1);
     launch_block_fill(n, w.is_start.get(), w.start_scan.get(), w.blk_row.get(), s);
-    w.lfac.ensure(n);
-    w.ipiv.ensure(n);
-    k_block_factors<<<grid_for(nblk, 128), 128, 0, s>>>(nblk, n, w.blk_row.get(), sys.rp, sys.ci, sys.val, sys.diag, node_scale,
-                                                       edge_scale, w.lfac.get(), w.ipiv.get());
+    launch_block_factors(w, sys, nblk, node_scale, edge_scale, s);
     w.cta_row.ensure(C + 1);
     launch_cta_rows(C, n, w.is_start.get(), w.cta_row.get(), s);
     w.cta_stats.ensure(2 * (C + 1));

@@ -914,23 +914,31 @@ __global__ void __launch_bounds__(kMgClusterThreads) k_mg_batch(const MgArgs* __
 }
 
 // ---------------------------------------------------------------------------
-// Shared-memory-resident clustered grid kernel for systems above one cluster's size.
+// Shared-memory-resident grid kernel for systems above one cluster's size: one CTA per SM
+// (cooperative launch).
 //
-// The grid is K clusters of kSmCtas CTAs, one CTA per SM (cooperative launch).  Every
-// operator of the V-cycle is static during the solve, so each CTA copies once, at launch,
-// the rows it owns into shared memory: its level-0 rows (CSR, column aggregates, chain-block
-// inverses, aggregate ranges) with the CG vectors of those rows, and its share of the fused
-// restriction / prolongation rows of every coarse level.  A phase then costs one round trip
-// for the vector entries other CTAs wrote, plus its barrier, instead of three to six
-// dependent L2 round trips for indices, weights and vectors.  Levels lc .. coarsest (at most
-// kSmRows rows at lc) are solved by every cluster on its own copy of their vectors between
-// hardware cluster barriers (~0.3 us) instead of grid barriers (~1.1 us plus skew).  A row
-// set that does not fit the shared-memory budget is read from global memory instead.
-constexpr int kSmCtas = 8;          // CTAs per cluster (portable size)
+// An iteration is a dozen phases between grid barriers, each a gathered sparse product of a few
+// thousand entries a CTA, so it is bound by the latency of its dependent loads and barriers.  Every
+// operator of the V-cycle is static during the solve: each CTA copies once, at launch, the rows it
+// owns into shared memory (a set that does not fit the budget is read from global memory), and a
+// phase costs one round trip for the vector entries other CTAs wrote, plus its barrier.
+//
+// Rows of the coarse levels are dealt by their entries, not their number, and a CTA spreads the
+// entries over all its threads: products first, into shared memory, then the rows' sums.  With rows
+// dealt by number and two to 32 lanes a row the CTA holding a level's longest rows kept the others
+// waiting 2-10 us a phase.  The chain blocks are applied by their LDL^T factors, one thread a chain:
+// two values a row instead of the chain's length (which large systems read from L2), and no inverses
+// to set up (0.1-0.4 ms a network).
+//
+// An iteration of the 25k-CNT network's passes (64.7k, 28.4k rows) takes 44 and 40 us (57 and 47
+// with rows dealt by number and dense blocks), of a 47.7k-CNT / 5 um realisation (313k, 246k rows)
+// 86 and 90 us (160 and 123).  Measured and left: 1,024 threads (47, 43, 85, 88 us); one flag word a
+// CTA polled by a thread each instead of the counter (90 us); values stored with their iteration's
+// number and polled, without barriers (46, 41, 107, 98 us).
 constexpr int kSmThreads = 512;
-constexpr int kSmRows = 1000;       // largest level the clusters solve alone
-constexpr int kSmMaxClusters = 18;  // 144 CTAs
 constexpr int kSmBytes = 200 * 1024;
+constexpr int kSmProd = 4096;  // products of a phase held at once
+constexpr int kSmAux = kSmThreads;  // rows of a phase held at once
 
 struct MgSmLevel {
     int n;
@@ -945,25 +953,20 @@ struct MgSmLevel {
     double* r;
     double* z;
     double* zf;
-    int priv;      // bit 0: r and z per cluster (stride n), bit 1: zf per cluster
-    int rr_lanes;  // lanes per restriction row into l + 1 / per prolongation row of l (powers of two)
-    int pq_lanes;
 };
 
 struct MgSmArgs {
-    int lc;                  // first level the clusters solve alone (>= 1)
-    const MgSmLevel* lv;     // levels 0 .. coarsest
-    int* cl_fail;            // per cluster: a grid-barrier wait of one of its CTAs gave up
-    const int32_t* mptr0;    // level-0 aggregates (the chain blocks): first row of each, then n
-    int smem_bytes;          // dynamic shared memory of the launch
-    int grid_coarse;         // dense coarsest solved by all CTAs between grid barriers (lc = coarsest, no clusters)
+    const MgSmLevel* lv;   // levels 0 .. coarsest
+    const int32_t* mptr0;  // level-0 aggregates (the chain blocks): first row of each, then n
+    const double* lfac;    // LDL^T factors of the chain blocks (0 at a block's first row, and one 0 past the last row)
+    const double* ipiv;
+    int smem_bytes;        // dynamic shared memory of the launch
 };
 
 // Rows [lo, hi) of one fused operator.  ptr[i - lo] - sub and ptr[i - lo + 1] - sub bound the
-// entries of row i in col / val; agg and l1inv are indexed by i - lo.  Staged copies have
-// sub = 0; a set read from global memory points into the global arrays with sub = ptr[lo].
+// entries of row i in col / val; agg and l1inv are indexed by i - lo.  lanes: threads per row sum.
 struct SmRows {
-    int lo, hi, sub;
+    int lo, hi, sub, lanes;
     const int32_t* ptr;
     const int32_t* col;
     const double* val;
@@ -971,14 +974,13 @@ struct SmRows {
     const double* l1inv;
 };
 
-// The CTA's level-0 rows [lo, hi): CSR (entries ent_sub-based), column aggregates, chain-block
-// inverse rows (tinv, row offsets tofs-based, block bases lo-based), aggregates alo .. ahi with
-// their row ranges (lo-based), and the CG vectors of its rows (lo-based).
+// The CTA's level-0 rows [lo, hi): CSR (entries rp_sub-based), column aggregates, chain factors,
+// aggregates alo .. ahi with their row ranges (mptr_sub-based), and the CG vectors of its rows.
 struct SmL0 {
     int lo, hi, alo, ahi;
-    int rp_sub, roff_sub, rbase_sub, mptr_sub;
-    const int32_t *rp, *ci, *cagg, *roff, *rbase, *rm, *agg, *mptr;
-    const double *val, *tinv, *b;
+    int rp_sub, mptr_sub;
+    const int32_t *rp, *ci, *cagg, *agg, *mptr;
+    const double *val, *lf, *ip, *b, *l1;
     double *r, *x, *p, *q, *z, *z0, *w;
 };
 
@@ -988,7 +990,7 @@ struct SmPlan {
     SmRows Q[kMgMaxLevels];  // prolongation rows of level l
     int clo, chi;            // coarsest rows of this CTA (dense inverse rows)
     const double* cinv;      // its rows, (i - clo) * nC based
-    unsigned int used;
+    double *prod, *aux;
 };
 
 struct SmStage {  // one copy from global into shared memory
@@ -997,316 +999,244 @@ struct SmStage {  // one copy from global into shared memory
     int count, elem, rebase;  // elem 4: int32 (minus rebase), 8: double
 };
 
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+// Sum of v over all threads of the grid, between grid barriers (mg_sync): every CTA publishes its
+// partial before the barrier and adds up all of them, in the same order, after it.
+__device__ __forceinline__ bool sm_sum(const MgArgs& a, double* part, unsigned long long& target, double v, double* sm, int* s_ok, double& total) {
+    const int nb = gridDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    v = warp_sum(v);
+    if (lane == 0) sm[warp] = v;
+    __syncthreads();
+    if (warp == 0) {
+        v = warp_sum(lane < kSmThreads / 32 ? sm[lane] : 0.0);
+        if (lane == 0) part[blockIdx.x] = v;
+    }
+    if (!mg_sync(a.bar, target, a.err, s_ok, a.spin_limit)) return false;
+    v = warp_sum((int)threadIdx.x < nb ? __ldcg(&part[threadIdx.x]) : 0.0);
+    if (lane == 0) sm[32 + warp] = v;
+    __syncthreads();
+    total = 0;
+    for (int w = 0; w < (nb + 31) / 32; w++) total += sm[32 + w];
+    return true;
 }
 
-// Grid barrier (bounded).  A CTA whose wait gave up marks its cluster and carries on through
-// the iteration with the same control flow (its data are then stale, the device status says
-// why); sm_cluster_ok, once per iteration before the first data-dependent branch, lets every
-// CTA of a marked cluster leave together, so no cluster barrier ever waits on a CTA that has
-// returned and no CTA branches on partial sums another CTA of its cluster read differently.
-__device__ __forceinline__ void sm_sync(const MgArgs& a, int* cl_fail, unsigned long long& target, int cid, int* s_ok) {
-    if (!mg_sync(a.bar, target, a.err, s_ok, a.spin_limit) && threadIdx.x == 0) atomicExch(&cl_fail[cid], 1);
-}
-
-__device__ __forceinline__ bool sm_cluster_ok(const int* cl_fail, int cid) {
-    cluster_sync_all();
-    return __ldcg(&cl_fail[cid]) == 0;
-}
-
-// sum_k val[k] v(col[k]) with v(c) = v0[c] for c < n, else v1[c - n]; chunks of U entries
-// per lane (indices and weights first, vector entries second).
-template <int U>
-__device__ __forceinline__ double fused_dot(const int32_t* col, const double* val, int b, int e, int first, int step, int n,
-                                            const double* v0, const double* v1) {
-    double s = 0;
-    for (int k0 = b + first; k0 < e; k0 += U * step) {
-        int c[U];
-        double w[U], xv[U];
+// The CTA's part of one fused operator: out(row, sum, aux) for each of its rows, where sum is
+// sum_k val[k] v(col[k]) with v(c) = v0[c] for c < n, else v1[c - n], and aux the row's two values
+// of pre(row) (loaded with the entries).
+template <bool kAux, class Pre, class Out>
+__device__ __forceinline__ void sm_rows(const SmRows& R, double* prod, double* aux, int n, const double* v0, const double* v1, double* sm, Pre pre,
+                                        Out out) {
+    const int tid = threadIdx.x, nr = R.hi - R.lo;
+    for (int i0 = 0; i0 < nr;) {
+        const int e0 = R.ptr[i0] - R.sub;
+        int i1 = min(nr, i0 + kSmAux);
+        if (R.ptr[i1] - R.sub - e0 > kSmProd) {  // as many rows as fit, at least one
+            int lo = i0 + 1, hi = i1;
+            while (hi - lo > 1) {
+                const int m = (lo + hi) >> 1;
+                if (R.ptr[m] - R.sub - e0 <= kSmProd) lo = m; else hi = m;
+            }
+            i1 = lo;
+        }
+        const int E = R.ptr[i1] - R.sub - e0;
+        double2 t = make_double2(0, 0);
+        if (kAux && i0 + tid < i1) t = pre(i0 + tid);
+        double long_sum = 0;  // a row of more than kSmProd entries: one thread's share of it
+        for (int k0 = tid; k0 < E; k0 += 4 * kSmThreads) {
+            int c[4];
+            double w[4], x[4];
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int k = k0 + u * step;
-            c[u] = k < e ? col[k] : 0;
-            w[u] = k < e ? val[k] : 0.0;
+            for (int u = 0; u < 4; u++) {
+                const int k = k0 + u * kSmThreads;
+                c[u] = k < E ? R.col[e0 + k] : 0;
+                w[u] = k < E ? R.val[e0 + k] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) x[u] = k0 + u * kSmThreads < E ? (c[u] < n ? __ldcg(&v0[c[u]]) : __ldcg(&v1[c[u] - n])) : 0.0;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int k = k0 + u * kSmThreads;
+                if (E > kSmProd) long_sum += w[u] * x[u];
+                else if (k < E) prod[k] = w[u] * x[u];
+            }
+        }
+        if (kAux && i0 + tid < i1) {
+            aux[2 * tid] = t.x;
+            aux[2 * tid + 1] = t.y;
+        }
+        if (E > kSmProd) {
+            long_sum = warp_sum(long_sum);
+            if ((tid & 31) == 0) sm[tid >> 5] = long_sum;
+        }
+        __syncthreads();
+        if (E > kSmProd) {
+            if (tid == 0) {
+                double s = 0;
+                for (int w = 0; w < kSmThreads / 32; w++) s += sm[w];
+                out(i0, s, kAux ? aux[0] : 0.0, kAux ? aux[1] : 0.0);
+            }
+        } else {
+            const int lanes = R.lanes, gl = tid % lanes;
+            for (int i = i0 + tid / lanes; i < i1; i += kSmThreads / lanes) {
+                const int e = R.ptr[i + 1] - R.sub - e0;
+                double s = 0;
+                for (int k = R.ptr[i] - R.sub - e0 + gl; k < e; k += lanes) s += prod[k];
+                const unsigned mask = lanes >= 32 ? 0xffffffffu : (((1u << lanes) - 1) << ((tid & 31) & ~(lanes - 1)));
+                for (int o = lanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(mask, s, o, lanes);
+                if (gl == 0) out(i, s, kAux ? aux[2 * (i - i0)] : 0.0, kAux ? aux[2 * (i - i0) + 1] : 0.0);
+            }
+        }
+        i0 = i1;
+        if (i0 < nr) __syncthreads();
+    }
+}
+
+// One chain: w = (L D L^T)^-1 r over its rows [m0, m1) (r may be w).  lf is 0 at a chain's first
+// row, and lf[m1] (the next chain's first row) is readable.
+template <class Out>
+__device__ __forceinline__ void chain_solve(const double* r, const double* lf, const double* ip, double* w, int m0, int m1, Out out) {
+    double y = 0;
+    for (int k0 = m0; k0 < m1; k0 += 4) {
+        double rv[4], lv[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int k = min(k0 + u, m1 - 1);
+            rv[u] = r[k];
+            lv[u] = lf[k];
         }
 #pragma unroll
-        for (int u = 0; u < U; u++) xv[u] = (k0 + u * step < e) ? (c[u] < n ? __ldcg(&v0[c[u]]) : __ldcg(&v1[c[u] - n])) : 0.0;
-#pragma unroll
-        for (int u = 0; u < U; u++) s += w[u] * xv[u];
+        for (int u = 0; u < 4; u++)
+            if (k0 + u < m1) {
+                y = rv[u] - lv[u] * y;
+                w[k0 + u] = y;
+            }
     }
-    return s;
-}
-
-// Level-0 row gather: sum_q val[q] v(ci[q]) over entries [b, e), v(c) = vs[c - lo] for the
-// CTA's own rows [lo, hi) (shared memory), else the global vector vg; with zc, each entry also
-// adds zc[cagg[q]].  Chunks of U entries: indices and weights first, vector entries second.
-template <int U>
-__device__ __forceinline__ double own_dot(const int32_t* ci, const double* val, const int32_t* cagg, int b, int e, int lo, int hi,
-                                          const double* vs, const double* vg, const double* zc) {
-    double s = 0;
-    for (int q0 = b; q0 < e; q0 += U) {
-        int c[U], g[U];
-        double w[U], x[U];
+    y = 0;
+    for (int k0 = m1 - 1; k0 >= m0; k0 -= 4) {
+        double yv[4], lv[4];
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int q = q0 + u;
-            c[u] = q < e ? ci[q] : lo;
-            w[u] = q < e ? val[q] : 0.0;
-            g[u] = (zc && q < e) ? cagg[q] : 0;
+        for (int u = 0; u < 4; u++) {
+            const int k = max(k0 - u, m0);
+            yv[u] = w[k] * ip[k];
+            lv[u] = lf[k + 1];
         }
 #pragma unroll
-        for (int u = 0; u < U; u++) {
-            x[u] = (c[u] >= lo && c[u] < hi) ? vs[c[u] - lo] : __ldcg(&vg[c[u]]);
-            if (zc) x[u] += __ldcg(&zc[g[u]]);
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) s += w[u] * x[u];
-    }
-    return s;
-}
-
-// Sum of the nb per-CTA partials: one load per thread, then the CTA reduction.
-__device__ __forceinline__ double sm_sum_partials(const double* part, int nb, double* sm) {
-    double v = 0;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) v += __ldcg(&part[i]);
-    double r;
-    mg_reduce1(v, sm, r);
-    return r;
-}
-
-__device__ __forceinline__ double lanes_sum(double v, int lanes) {
-    const unsigned mask = lanes >= 32 ? 0xffffffffu : (((1u << lanes) - 1) << ((threadIdx.x & 31) & ~(lanes - 1)));
-    for (int o = lanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o, lanes);
-    return v;
-}
-
-// r_{l+1} = P^T (r_l - A_l z_l) and its l1-Jacobi smoothing on the rows of R.
-__device__ __forceinline__ void sm_restrict(const SmRows& R, int lanes, int nF, const double* rF, const double* zF, double* rG, double* zG,
-                                            bool smooth) {
-    const int grp = threadIdx.x / lanes, gl = threadIdx.x % lanes, ngrp = blockDim.x / lanes;
-    for (int J = R.lo + grp; J < R.hi; J += ngrp) {
-        const int j = J - R.lo;
-        double v = fused_dot<4>(R.col, R.val, R.ptr[j] - R.sub, R.ptr[j + 1] - R.sub, gl, lanes, nF, rF, zF);
-        v = lanes_sum(v, lanes);
-        if (gl == 0) {
-            rG[J] = v;
-            if (smooth) zG[J] = R.l1inv[j] * v;
-        }
+        for (int u = 0; u < 4; u++)
+            if (k0 - u >= m0) {
+                y = yv[u] - lv[u] * y;
+                out(k0 - u, y);
+            }
     }
 }
 
-// zp = z_l + P zc, zf_l = zp + D^-1 (r_l - A_l zp) on the rows of Q.
-__device__ __forceinline__ void sm_prolong(const SmRows& Q, int lanes, int nF, const double* rF, const double* zF, const double* zc, double* zf) {
-    const int grp = threadIdx.x / lanes, gl = threadIdx.x % lanes, ngrp = blockDim.x / lanes;
-    for (int I = Q.lo + grp; I < Q.hi; I += ngrp) {
-        const int i = I - Q.lo;
-        double zp = 0, rI = 0;
-        if (gl == 0) {
-            zp = __ldcg(&zF[I]) + __ldcg(&zc[Q.agg[i]]);
-            rI = __ldcg(&rF[I]);
-        }
-        double v = fused_dot<4>(Q.col, Q.val, Q.ptr[i] - Q.sub, Q.ptr[i + 1] - Q.sub, gl, lanes, nF, zF, zc);
-        v = lanes_sum(v, lanes);
-        if (gl == 0) zf[I] = zp + Q.l1inv[i] * (rI - v);
-    }
-}
+constexpr int kSmMaxStages = 16 + 7 * kMgMaxLevels;
 
-// Thread 0: place rows [lo, hi) of (ptr, col, val) plus optional per-row agg / l1inv into the
-// shared budget, or point at global memory; records the copies in st[] (returns their count).
-__device__ int sm_place_rows(SmRows& R, int lo, int hi, const int32_t* ptr, const int32_t* col, const double* val, const int32_t* agg,
-                             const double* l1inv, unsigned char* base, unsigned int cap, unsigned int& used, SmStage* st, int ns, int max_st) {
-    R.lo = lo;
-    R.hi = hi;
-    R.agg = agg ? agg + lo : nullptr;
-    R.l1inv = l1inv ? l1inv + lo : nullptr;
-    if (hi <= lo || !ptr) {
-        R.ptr = ptr ? ptr + lo : nullptr;
-        R.col = col;
-        R.val = val;
-        R.sub = 0;
-        return ns;
-    }
-    const int e0 = ptr[lo], e1 = ptr[hi], E = e1 - e0, nr = hi - lo;
-    auto al = [](unsigned int u) { return (u + 15u) & ~15u; };
-    unsigned int u = al(used);
-    const unsigned int o_ptr = u;
-    u = al(u + 4u * (nr + 1));
-    const unsigned int o_col = u;
-    u = al(u + 4u * E);
-    const unsigned int o_val = u;
-    u = al(u + 8u * E);
-    const unsigned int o_agg = u;
-    if (agg) u = al(u + 4u * nr);
-    const unsigned int o_l1 = u;
-    if (l1inv) u = al(u + 8u * nr);
-    if (u > cap || ns + 5 > max_st) {  // read from global memory
-        R.ptr = ptr + lo;
-        R.col = col + e0;
-        R.val = val + e0;
-        R.sub = e0;
-        return ns;
-    }
-    used = u;
-    R.ptr = reinterpret_cast<const int32_t*>(base + o_ptr);
-    R.col = reinterpret_cast<const int32_t*>(base + o_col);
-    R.val = reinterpret_cast<const double*>(base + o_val);
-    R.sub = 0;
-    st[ns++] = SmStage{base + o_ptr, ptr + lo, nr + 1, 4, e0};
-    st[ns++] = SmStage{base + o_col, col + e0, E, 4, 0};
-    st[ns++] = SmStage{base + o_val, val + e0, E, 8, 0};
-    if (agg) {
-        R.agg = reinterpret_cast<const int32_t*>(base + o_agg);
-        st[ns++] = SmStage{base + o_agg, agg + lo, nr, 4, 0};
-    }
-    if (l1inv) {
-        R.l1inv = reinterpret_cast<const double*>(base + o_l1);
-        st[ns++] = SmStage{base + o_l1, l1inv + lo, nr, 8, 0};
-    }
-    return ns;
-}
-
-constexpr int kSmMaxStages = 160;
-
-__global__ void __launch_bounds__(kSmThreads) k_mg_pcg_sm(MgArgs a, MgSmArgs sa) {
+__global__ void __launch_bounds__(kSmThreads, 1) k_mg_pcg_sm(MgArgs a, MgSmArgs sa) {
     extern __shared__ __align__(16) unsigned char sm_dyn[];
-    __shared__ double sm[72];
+    __shared__ double sm[64];
     __shared__ MgSmLevel lv[kMgMaxLevels];
     __shared__ SmPlan P;
     __shared__ SmStage st[kSmMaxStages];
-    __shared__ int n_st;
-    __shared__ int s_ok;
+    __shared__ int n_st, s_ok;
+    __shared__ int cut[kMgMaxLevels][4];
     __shared__ double rc[kMgDenseGridMax];
-    const int cta = blockIdx.x, nb = gridDim.x;
-    const int cid = cta / kSmCtas, crank = cta % kSmCtas;
-    const int C = a.levels - 1, Lc = sa.lc;
-    if (threadIdx.x < a.levels) {
-        MgSmLevel L = sa.lv[threadIdx.x];
-        if (L.priv & 1) {
-            L.r += (size_t)cid * L.n;
-            L.z += (size_t)cid * L.n;
+    const int cta = blockIdx.x, nb = gridDim.x, tid = threadIdx.x;
+    const int C = a.levels - 1;
+    if (tid < a.levels) lv[tid] = sa.lv[tid];
+    __syncthreads();
+    // ---- this CTA's rows of every level: an equal share of entries + 4 rows ----
+    if (tid < 4 * C && tid >= 4) {
+        const int l = tid >> 2, n = (tid & 2) ? lv[l].n : lv[l + 1].n, c = cta + (tid & 1);
+        const int32_t* ptr = (tid & 2) ? lv[l].pq_ptr : lv[l].rr_ptr;
+        const long long want = (ptr[n] + 4LL * n) * c / nb;
+        int lo = 0, hi = n;  // first row whose share starts at or after `want`
+        while (lo < hi) {
+            const int m = (lo + hi) >> 1;
+            if (ptr[m] + 4LL * m < want) lo = m + 1; else hi = m;
         }
-        if (L.priv & 2) L.zf += (size_t)cid * L.n;
-        lv[threadIdx.x] = L;
+        cut[l][tid & 3] = c == nb ? n : lo;
     }
     __syncthreads();
     // ---- placement (thread 0), then the copies (all threads) ----
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
         const unsigned int cap = (unsigned int)sa.smem_bytes;
         unsigned int used = 0;
         int ns = 0;
-        auto al = [](unsigned int u) { return (u + 15u) & ~15u; };
-        auto take = [&](unsigned int bytes) -> unsigned char* {
-            const unsigned int u = al(used);
+        auto take = [&](size_t bytes) -> unsigned char* {
+            const unsigned int u = (used + 15u) & ~15u;
             if (u + bytes > cap) return nullptr;
-            used = u + bytes;
+            used = u + (unsigned int)bytes;
             return sm_dyn + u;
+        };
+        // dst: the staged copy, or `src` itself when it does not fit
+        auto stage_i = [&](const int32_t*& dst, const int32_t* src, int count, int rebase) {
+            unsigned char* m = count > 0 ? take(4 * (size_t)count) : nullptr;
+            dst = m ? reinterpret_cast<const int32_t*>(m) : src;
+            if (m) st[ns++] = SmStage{m, src, count, 4, rebase};
+            return m != nullptr;
+        };
+        auto stage_d = [&](const double*& dst, const double* src, int count) {
+            unsigned char* m = count > 0 ? take(8 * (size_t)count) : nullptr;
+            dst = m ? reinterpret_cast<const double*>(m) : src;
+            if (m) st[ns++] = SmStage{m, src, count, 8, 0};
+        };
+        auto vec = [&](double* src, int count) {
+            unsigned char* m = count > 0 ? take(8 * (size_t)count) : nullptr;
+            return m ? reinterpret_cast<double*>(m) : src;
         };
         SmL0& L = P.l0;
         const MgLevel& G0 = a.lv[0];
         L.lo = a.cta_row[cta];
         L.hi = a.cta_row[cta + 1];
         const int nr = L.hi - L.lo;
-        // vectors of the own rows (x, r from global; the others are written before read)
-        double* vec = nr > 0 ? reinterpret_cast<double*>(take(8u * 7 * nr)) : nullptr;
-        if (vec) {
-            L.r = vec; L.x = vec + nr; L.p = vec + 2 * nr; L.q = vec + 3 * nr; L.z = vec + 4 * nr; L.z0 = vec + 5 * nr; L.w = vec + 6 * nr;
-            st[ns++] = SmStage{L.r, a.r + L.lo, nr, 8, 0};
-            st[ns++] = SmStage{L.x, a.x + L.lo, nr, 8, 0};
-        } else {
-            L.r = a.r + L.lo; L.x = a.x + L.lo; L.p = a.p + L.lo; L.q = a.q + L.lo; L.z = a.z + L.lo; L.z0 = a.z0 + L.lo; L.w = a.w + L.lo;
-        }
-        L.b = a.b + L.lo;
-        // CSR rows with their column aggregates
-        const int e0 = nr > 0 ? a.rp[L.lo] : 0, E = nr > 0 ? a.rp[L.hi] - e0 : 0;
-        unsigned char* m_rp = nr > 0 ? take(4u * (nr + 1)) : nullptr;
-        unsigned char* m_ci = m_rp ? take(4u * E) : nullptr;
-        unsigned char* m_cg = m_ci ? take(4u * E) : nullptr;
-        unsigned char* m_v = m_cg ? take(8u * E) : nullptr;
-        if (m_v) {
-            L.rp = reinterpret_cast<const int32_t*>(m_rp); L.rp_sub = 0;
-            L.ci = reinterpret_cast<const int32_t*>(m_ci);
-            L.cagg = reinterpret_cast<const int32_t*>(m_cg);
-            L.val = reinterpret_cast<const double*>(m_v);
-            st[ns++] = SmStage{m_rp, a.rp + L.lo, nr + 1, 4, e0};
-            st[ns++] = SmStage{m_ci, a.ci + e0, E, 4, 0};
-            st[ns++] = SmStage{m_cg, G0.cagg + e0, E, 4, 0};
-            st[ns++] = SmStage{m_v, a.val + e0, E, 8, 0};
-        } else {
-            L.rp = a.rp + L.lo; L.rp_sub = e0;
-            L.ci = a.ci + e0; L.cagg = G0.cagg + e0; L.val = a.val + e0;
-        }
-        // row -> aggregate, and the own aggregates' row ranges
+        P.prod = reinterpret_cast<double*>(take(8 * kSmProd));
+        P.aux = reinterpret_cast<double*>(take(16 * kSmAux));
+        // what every phase of level 0 reads: residual, smoothed vectors, chain factors and ranges
+        L.r = vec(a.r + L.lo, nr);
+        if (L.r != a.r + L.lo) st[ns++] = SmStage{L.r, a.r + L.lo, nr, 8, 0};
+        L.z0 = vec(a.z0 + L.lo, nr);
+        L.w = vec(a.w + L.lo, nr);
+        L.z = vec(a.z + L.lo, nr);
+        stage_d(L.lf, sa.lfac + L.lo, nr > 0 ? nr + 1 : 0);
+        stage_d(L.ip, sa.ipiv + L.lo, nr);
         L.alo = nr > 0 ? G0.agg[L.lo] : 0;
         L.ahi = nr > 0 ? G0.agg[L.hi - 1] + 1 : 0;
-        const int na = L.ahi - L.alo;
-        unsigned char* m_ag = nr > 0 ? take(4u * nr) : nullptr;
-        unsigned char* m_mp = m_ag ? take(4u * (na + 1)) : nullptr;
-        if (m_mp) {
-            L.agg = reinterpret_cast<const int32_t*>(m_ag);
-            L.mptr = reinterpret_cast<const int32_t*>(m_mp); L.mptr_sub = 0;
-            st[ns++] = SmStage{m_ag, G0.agg + L.lo, nr, 4, 0};
-            st[ns++] = SmStage{m_mp, sa.mptr0 + L.alo, na + 1, 4, L.lo};
-        } else {
-            L.agg = G0.agg + L.lo;
-            L.mptr = sa.mptr0 + L.alo; L.mptr_sub = L.lo;
-        }
-        // chain-block inverse rows (both smoother phases read them: before the coarse rows)
-        const int t0 = nr > 0 ? a.row_off[L.lo] : 0;
-        const int T = nr > 0 ? a.row_off[L.hi - 1] + a.row_m[L.hi - 1] - t0 : 0;
-        unsigned char* m_meta = nr > 0 && ns + 4 <= kSmMaxStages ? take(12u * nr) : nullptr;
-        unsigned char* m_t = m_meta ? take(8u * T) : nullptr;
-        if (m_t) {
-            L.roff = reinterpret_cast<const int32_t*>(m_meta); L.roff_sub = 0;
-            L.rbase = L.roff + nr; L.rbase_sub = 0;
-            L.rm = L.rbase + nr;
-            L.tinv = reinterpret_cast<const double*>(m_t);
-            st[ns++] = SmStage{m_meta, a.row_off + L.lo, nr, 4, t0};
-            st[ns++] = SmStage{m_meta + 4u * nr, a.row_base + L.lo, nr, 4, L.lo};
-            st[ns++] = SmStage{m_meta + 8u * nr, a.row_m + L.lo, nr, 4, 0};
-            st[ns++] = SmStage{m_t, a.tinv + t0, T, 8, 0};
-        } else {
-            L.roff = a.row_off + L.lo; L.roff_sub = t0;
-            L.rbase = a.row_base + L.lo; L.rbase_sub = L.lo;
-            L.rm = a.row_m + L.lo;
-            L.tinv = a.tinv + t0;
-        }
-        // coarse levels: grid rows below lc, cluster rows from lc on
-        auto lanes_for = [](long long entries, int rows) {
-            int ln = 2;
-            while (ln < 32 && (long long)ln * 4 * rows < entries) ln <<= 1;  // about one chunk of 4 entries per lane
-            return ln;
-        };
-        for (int l = 1; l < C; l++) {
-            MgSmLevel& F = lv[l];
-            const MgSmLevel& G = lv[l + 1];
-            F.rr_lanes = lanes_for(F.rr_ptr[G.n], G.n);
-            F.pq_lanes = lanes_for(F.pq_ptr[F.n], F.n);
-            const bool sec_r = l >= Lc, sec_q = l >= Lc;
-            const int n1 = G.n, n0 = F.n;
-            const int rlo = sec_r ? (int)((long long)n1 * crank / kSmCtas) : (int)((long long)n1 * cta / nb);
-            const int rhi = sec_r ? (int)((long long)n1 * (crank + 1) / kSmCtas) : (int)((long long)n1 * (cta + 1) / nb);
-            ns = sm_place_rows(P.R[l], rlo, rhi, F.rr_ptr, F.rr_col, F.rr_val, nullptr, G.l1inv, sm_dyn, cap, used, st, ns, kSmMaxStages);
-            const int qlo = sec_q ? (int)((long long)n0 * crank / kSmCtas) : (int)((long long)n0 * cta / nb);
-            const int qhi = sec_q ? (int)((long long)n0 * (crank + 1) / kSmCtas) : (int)((long long)n0 * (cta + 1) / nb);
-            ns = sm_place_rows(P.Q[l], qlo, qhi, F.pq_ptr, F.pq_col, F.pq_val, F.agg, F.l1inv, sm_dyn, cap, used, st, ns, kSmMaxStages);
-        }
-        const int nC = lv[C].n;
-        P.clo = sa.grid_coarse ? (int)((long long)nC * cta / nb) : (int)((long long)nC * crank / kSmCtas);
-        P.chi = sa.grid_coarse ? (int)((long long)nC * (cta + 1) / nb) : (int)((long long)nC * (crank + 1) / kSmCtas);
-        P.cinv = nullptr;
-        if (a.cinv) {
-            const int cr = P.chi - P.clo;
-            unsigned char* m_c = cr > 0 && ns < kSmMaxStages ? take(8u * cr * nC) : nullptr;
-            if (m_c) {
-                P.cinv = reinterpret_cast<const double*>(m_c);
-                st[ns++] = SmStage{m_c, a.cinv + (size_t)P.clo * nC, cr * nC, 8, 0};
-            } else {
-                P.cinv = a.cinv + (size_t)P.clo * nC;
+        stage_i(L.agg, G0.agg + L.lo, nr, 0);
+        L.mptr_sub = stage_i(L.mptr, sa.mptr0 + L.alo, nr > 0 ? L.ahi - L.alo + 1 : 0, L.lo) ? 0 : L.lo;
+        stage_d(L.l1, lv[1].l1inv + L.alo, L.ahi - L.alo);
+        const int ent0 = nr > 0 ? a.rp[L.lo] : 0, ent = nr > 0 ? a.rp[L.hi] - ent0 : 0;
+        L.rp_sub = stage_i(L.rp, a.rp + L.lo, nr > 0 ? nr + 1 : 0, ent0) ? 0 : ent0;
+        // coarse operators, the coarsest (most often waited for) first: row data, then entries
+        for (int l = C - 1; l >= 1; l--) {
+            for (int q = 0; q < 2; q++) {
+                SmRows& R = q ? P.Q[l] : P.R[l];
+                const MgSmLevel& F = lv[l];
+                const int32_t* ptr = q ? F.pq_ptr : F.rr_ptr;
+                R.lo = cut[l][2 * q];
+                R.hi = cut[l][2 * q + 1];
+                const int rows = R.hi - R.lo, e0 = ptr[R.lo], E = ptr[R.hi] - e0;
+                R.sub = stage_i(R.ptr, ptr + R.lo, rows > 0 ? rows + 1 : 0, e0) ? 0 : e0;
+                stage_d(R.l1inv, (q ? F.l1inv : lv[l + 1].l1inv) + R.lo, rows);
+                if (q) stage_i(R.agg, F.agg + R.lo, rows, 0);
+                stage_i(R.col, (q ? F.pq_col : F.rr_col) + e0, E, 0);
+                stage_d(R.val, (q ? F.pq_val : F.rr_val) + e0, E);
+                R.lanes = 32;
+                while (R.lanes > 2 && (R.lanes * rows > kSmThreads || R.lanes * rows > E)) R.lanes >>= 1;
             }
         }
-        P.used = used;
+        // level-0 matrix, the vectors only their own rows use, dense inverse rows
+        stage_i(L.ci, a.ci + ent0, ent, 0);
+        stage_d(L.val, a.val + ent0, ent);
+        stage_i(L.cagg, G0.cagg + ent0, ent, 0);
+        L.q = vec(a.q + L.lo, nr);
+        L.p = vec(a.p + L.lo, nr);
+        L.x = vec(a.x + L.lo, nr);
+        if (L.x != a.x + L.lo) st[ns++] = SmStage{L.x, a.x + L.lo, nr, 8, 0};
+        L.b = a.b + L.lo;
+        const int nC = lv[C].n;
+        P.clo = (int)((long long)nC * cta / nb);
+        P.chi = (int)((long long)nC * (cta + 1) / nb);
+        P.cinv = nullptr;
+        if (a.cinv) stage_d(P.cinv, a.cinv + (size_t)P.clo * nC, (P.chi - P.clo) * nC);
         n_st = ns;
     }
     __syncthreads();
@@ -1315,53 +1245,71 @@ __global__ void __launch_bounds__(kSmThreads) k_mg_pcg_sm(MgArgs a, MgSmArgs sa)
         if (S.elem == 8) {
             double* d = static_cast<double*>(S.dst);
             const double* g = static_cast<const double*>(S.src);
-            for (int i = threadIdx.x; i < S.count; i += blockDim.x) d[i] = g[i];
+            for (int i = tid; i < S.count; i += kSmThreads) d[i] = g[i];
         } else {
             int32_t* d = static_cast<int32_t*>(S.dst);
             const int32_t* g = static_cast<const int32_t*>(S.src);
-            for (int i = threadIdx.x; i < S.count; i += blockDim.x) d[i] = g[i] - S.rebase;
+            for (int i = tid; i < S.count; i += kSmThreads) d[i] = g[i] - S.rebase;
         }
     }
     __syncthreads();
     const SmL0& L = P.l0;
-    const int lo = L.lo, hi = L.hi;
-    // chain-block inverse row of own row li applied to a vector of own rows
-    auto block_row = [&](int li, const double* v) {
-        const int off = L.roff[li] - L.roff_sub, base = L.rbase[li] - L.rbase_sub, m = L.rm[li];
-        double s = 0;
-        for (int j = 0; j < m; j++) s += L.tinv[off + j] * v[base + j];
-        return s;
+    const int lo = L.lo, hi = L.hi, nr = hi - lo;
+    // out(row, sum) of own rows: sum_q val[q] v(ci[q]), v(c) = vs[c - lo] for the CTA's own rows (shared
+    // memory), else the global vector vg; with zc, each entry also adds zc[cagg[q]].  Four entries at
+    // a time: indices and weights first, vector entries second.
+    auto own_rows = [&](const double* vs, const double* vg, const double* zc, auto out) {
+        for (int li = tid; li < nr; li += kSmThreads) {
+            const int e = L.rp[li + 1] - L.rp_sub;
+            double s = 0;
+            for (int q0 = L.rp[li] - L.rp_sub; q0 < e; q0 += 4) {
+                int c[4], g[4];
+                double w[4], x[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int q = q0 + u;
+                    c[u] = q < e ? L.ci[q] : lo;
+                    w[u] = q < e ? L.val[q] : 0.0;
+                    g[u] = zc && q < e ? L.cagg[q] : -1;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    x[u] = (c[u] >= lo && c[u] < hi) ? vs[c[u] - lo] : __ldcg(&vg[c[u]]);
+                    if (g[u] >= 0) x[u] += __ldcg(&zc[g[u]]);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) s += w[u] * x[u];
+            }
+            out(li, s);
+        }
     };
-    auto row_b = [&](int li) { return L.rp[li] - L.rp_sub; };
+    auto chains = [&](const double* r, double* w, auto out) {  // one thread a chain
+        for (int j = tid; j < L.ahi - L.alo; j += kSmThreads)
+            chain_solve(r, L.lf, L.ip, w, L.mptr[j] - L.mptr_sub, L.mptr[j + 1] - L.mptr_sub, out);
+    };
     unsigned long long target = 0;
     double R0 = 0, rr = 0, rz = 0, beta = 0;
     long long k = 0;
     int restarts = 0;
     bool fresh = true;
     bool recursive = false;
-    double s0;
     while (true) {
         // ---- pre-smoother z0 = w M0^-1 r on own rows; r.r ----
         __syncthreads();
+        chains(L.r, L.w, [&](int li, double z) { L.z0[li] = a.omega0 * z; });
+        __syncthreads();
         double rr_l = 0;
-        for (int li = threadIdx.x; li < hi - lo; li += blockDim.x) {
-            const double z0 = a.omega0 * block_row(li, L.r);
-            L.z0[li] = z0;
-            a.z0[lo + li] = z0;
+        for (int li = tid; li < nr; li += kSmThreads) {
+            a.z0[lo + li] = L.z0[li];
             const double ri = L.r[li];
             rr_l += ri * ri;
         }
-        mg_reduce1(rr_l, sm, s0);
-        if (threadIdx.x == 0) a.partA[cta] = s0;
-        sm_sync(a, sa.cl_fail, target, cid, &s_ok);
-        if (!sa.grid_coarse && !sm_cluster_ok(sa.cl_fail, cid)) break;
-        rr = sm_sum_partials(a.partA, nb, sm);
+        if (!sm_sum(a, a.partA, target, rr_l, sm, &s_ok, rr)) return;
         if (k == 0 && !recursive && restarts == 0) R0 = a.tol * sqrt(rr);
         if (k > 0 && sqrt(rr) <= R0) {
             if (!recursive || restarts >= a.max_restarts) break;
             // the recursive residual met the test: replace it by the FP64 true residual
-            for (int li = threadIdx.x; li < hi - lo; li += blockDim.x)
-                L.r[li] = L.b[li] - own_dot<4>(L.ci, L.val, nullptr, row_b(li), row_b(li + 1), lo, hi, L.x, a.x, nullptr);
+            own_rows(L.x, a.x, nullptr, [&](int li, double s) { L.r[li] = L.b[li] - s; });
             restarts++;
             recursive = false;
             fresh = true;
@@ -1369,106 +1317,91 @@ __global__ void __launch_bounds__(kSmThreads) k_mg_pcg_sm(MgArgs a, MgSmArgs sa)
         }
         if (k >= a.max_iter) break;
         // ---- w = r - A z0; level 0 -> 1 over the own aggregates (the chain blocks) ----
+        own_rows(L.z0, a.z0, nullptr, [&](int li, double s) { L.w[li] = L.r[li] - s; });
+        __syncthreads();
         {
-            for (int li = threadIdx.x; li < hi - lo; li += blockDim.x)
-                L.w[li] = L.r[li] - own_dot<4>(L.ci, L.val, nullptr, row_b(li), row_b(li + 1), lo, hi, L.z0, a.z0, nullptr);
-            __syncthreads();
             const MgSmLevel& G = lv[1];
             const bool smooth = (C > 1) || a.cinv == nullptr;
-            for (int J = L.alo + threadIdx.x; J < L.ahi; J += blockDim.x) {
-                const int j = J - L.alo;
-                const int m0 = L.mptr[j] - L.mptr_sub, m1 = L.mptr[j + 1] - L.mptr_sub;
+            for (int j = tid; j < L.ahi - L.alo; j += kSmThreads) {
+                const int m1 = L.mptr[j + 1] - L.mptr_sub;
                 double v = 0;
-                for (int m = m0; m < m1; m++) v += L.w[m];
-                G.r[J] = v;
-                if (smooth) G.z[J] = G.l1inv[J] * v;
+                for (int m = L.mptr[j] - L.mptr_sub; m < m1; m++) v += L.w[m];
+                G.r[L.alo + j] = v;
+                if (smooth) G.z[L.alo + j] = L.l1[j] * v;
             }
-            sm_sync(a, sa.cl_fail, target, cid, &s_ok);
         }
-        // ---- restrictions l -> l + 1 grid-wide (1 <= l < lc) ----
-        for (int l = 1; l < Lc; l++) {
-            sm_restrict(P.R[l], lv[l].rr_lanes, lv[l].n, lv[l].r, lv[l].z, lv[l + 1].r, lv[l + 1].z, (l + 1 < C) || a.cinv == nullptr);
-            sm_sync(a, sa.cl_fail, target, cid, &s_ok);
+        if (!mg_sync(a.bar, target, a.err, &s_ok, a.spin_limit)) return;
+        // ---- r_{l+1} = P^T (r_l - A_l z_l) and its l1-Jacobi smoothing ----
+        for (int l = 1; l < C; l++) {
+            const SmRows& R = P.R[l];
+            const MgSmLevel& G = lv[l + 1];
+            const bool smooth = (l + 1 < C) || a.cinv == nullptr;
+            sm_rows<false>(R, P.prod, P.aux, lv[l].n, lv[l].r, lv[l].z, sm, [](int) { return make_double2(0, 0); },
+                    [&](int j, double v, double, double) {
+                        G.r[R.lo + j] = v;
+                        if (smooth) G.z[R.lo + j] = R.l1inv[j] * v;
+                    });
+            if (!mg_sync(a.bar, target, a.err, &s_ok, a.spin_limit)) return;
         }
-        // ---- levels lc .. coarsest: every cluster on its own copy ----
-        for (int l = Lc; l < C; l++) {
-            sm_restrict(P.R[l], lv[l].rr_lanes, lv[l].n, lv[l].r, lv[l].z, lv[l + 1].r, lv[l + 1].z, (l + 1 < C) || a.cinv == nullptr);
-            cluster_sync_all();
-        }
-        {
+        // ---- dense inverse of the coarsest level (r_C staged once), one warp per row; without one its correction is z ----
+        if (a.cinv) {
             const MgSmLevel& Cl = lv[C];
-            const int nC = Cl.n;
-            const int wpb = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-            if (a.cinv) {  // dense inverse of the coarsest level (r_C staged once), one warp per row
-                for (int j = threadIdx.x; j < nC; j += blockDim.x) rc[j] = __ldcg(&Cl.r[j]);
-                __syncthreads();
-                for (int i = P.clo + warp; i < P.chi; i += wpb) {
-                    const double* row = P.cinv + (size_t)(i - P.clo) * nC;
-                    double v = 0;
-                    for (int j = lane; j < nC; j += 32) v += row[j] * rc[j];
-                    v = warp_sum(v);
-                    if (lane == 0) Cl.zf[i] = v;
-                }
-            } else {  // l1-Jacobi only: the correction is the smoothed z
-                for (int i = P.clo + threadIdx.x; i < P.chi; i += blockDim.x) Cl.zf[i] = __ldcg(&Cl.z[i]);
+            const int nC = Cl.n, warp = tid >> 5, lane = tid & 31;
+            for (int j = tid; j < nC; j += kSmThreads) rc[j] = __ldcg(&Cl.r[j]);
+            __syncthreads();
+            for (int i = P.clo + warp; i < P.chi; i += kSmThreads / 32) {
+                const double* row = P.cinv + (size_t)(i - P.clo) * nC;
+                double v = 0;
+                for (int j = lane; j < nC; j += 32) v += row[j] * rc[j];
+                v = warp_sum(v);
+                if (lane == 0) Cl.zf[i] = v;
             }
-            if (sa.grid_coarse)
-                sm_sync(a, sa.cl_fail, target, cid, &s_ok);
-            else
-                cluster_sync_all();
+            if (!mg_sync(a.bar, target, a.err, &s_ok, a.spin_limit)) return;
         }
-        for (int l = C - 1; l >= Lc; l--) {
-            sm_prolong(P.Q[l], lv[l].pq_lanes, lv[l].n, lv[l].r, lv[l].z, lv[l + 1].zf, lv[l].zf);
-            cluster_sync_all();
-        }
-        // ---- prolongations lc - 1 .. 1 grid-wide ----
-        for (int l = Lc - 1; l >= 1; l--) {
-            sm_prolong(P.Q[l], lv[l].pq_lanes, lv[l].n, lv[l].r, lv[l].z, lv[l + 1].zf, lv[l].zf);
-            sm_sync(a, sa.cl_fail, target, cid, &s_ok);
+        // ---- zp = z_l + P zc, zf_l = zp + D^-1 (r_l - A_l zp) ----
+        for (int l = C - 1; l >= 1; l--) {
+            const SmRows& Q = P.Q[l];
+            const MgSmLevel& F = lv[l];
+            const double* zc = lv[l + 1].zf;
+            sm_rows<true>(Q, P.prod, P.aux, F.n, F.z, zc, sm,
+                    [&](int i) { return make_double2(__ldcg(&F.z[Q.lo + i]) + __ldcg(&zc[Q.agg[i]]), __ldcg(&F.r[Q.lo + i])); },
+                    [&](int i, double v, double zp, double r) { F.zf[Q.lo + i] = zp + Q.l1inv[i] * (r - v); });
+            if (!mg_sync(a.bar, target, a.err, &s_ok, a.spin_limit)) return;
         }
         // ---- level-0 post-smoother: z = z0 + P z1, z += w M0^-1 (r - A z); r.z ----
         {
             const double* zc = lv[1].zf;
-            for (int li = threadIdx.x; li < hi - lo; li += blockDim.x) {
-                const double zci = __ldcg(&zc[L.agg[li]]);
-                L.w[li] = L.r[li] - own_dot<4>(L.ci, L.val, L.cagg, row_b(li), row_b(li + 1), lo, hi, L.z0, a.z0, zc);
-                L.z[li] = L.z0[li] + zci;
-            }
+            for (int li = tid; li < nr; li += kSmThreads) L.z[li] = L.z0[li] + __ldcg(&zc[L.agg[li]]);
+            own_rows(L.z0, a.z0, zc, [&](int li, double s) { L.w[li] = L.r[li] - s; });
             __syncthreads();
-            double rz_l = 0;
-            for (int li = threadIdx.x; li < hi - lo; li += blockDim.x) {
-                const double zi = L.z[li] + a.omega0 * block_row(li, L.w);
-                L.z[li] = zi;
+            chains(L.w, L.w, [&](int li, double z) { L.z[li] += a.omega0 * z; });
+            __syncthreads();
+            double rz_l = 0, rz_new;
+            for (int li = tid; li < nr; li += kSmThreads) {
+                const double zi = L.z[li];
                 a.z[lo + li] = zi;
                 rz_l += L.r[li] * zi;
             }
-            mg_reduce1(rz_l, sm, s0);
-            if (threadIdx.x == 0) a.partB[cta] = s0;
-            sm_sync(a, sa.cl_fail, target, cid, &s_ok);
-            const double rz_new = sm_sum_partials(a.partB, nb, sm);
+            if (!sm_sum(a, a.partB, target, rz_l, sm, &s_ok, rz_new)) return;
             beta = fresh ? 0.0 : rz_new / rz;
             rz = rz_new;
         }
         // ---- q = A z + beta q, p = z + beta p; p.q ----
-        double pq_l = 0;
-        for (int li = threadIdx.x; li < hi - lo; li += blockDim.x) {
-            const double w = own_dot<4>(L.ci, L.val, nullptr, row_b(li), row_b(li + 1), lo, hi, L.z, a.z, nullptr);
+        double pq_l = 0, pq;
+        own_rows(L.z, a.z, nullptr, [&](int li, double w) {
             const double zi = L.z[li];
             const double qi = fresh ? w : w + beta * L.q[li];
             const double pi = fresh ? zi : zi + beta * L.p[li];
             L.q[li] = qi;
             L.p[li] = pi;
             pq_l += pi * qi;
-        }
-        mg_reduce1(pq_l, sm, s0);
-        if (threadIdx.x == 0) a.partA[nb + cta] = s0;
-        sm_sync(a, sa.cl_fail, target, cid, &s_ok);
-        const double pq = sm_sum_partials(a.partA + nb, nb, sm);
+        });
+        if (!sm_sum(a, a.partA + nb, target, pq_l, sm, &s_ok, pq)) return;
         fresh = false;
         k++;
         // ---- x += alpha p, r -= alpha q (x also to global: other CTAs read it for a true residual) ----
         const double alpha = rz / pq;
-        for (int li = threadIdx.x; li < hi - lo; li += blockDim.x) {
+        for (int li = tid; li < nr; li += kSmThreads) {
             const double xi = L.x[li] + alpha * L.p[li];
             L.x[li] = xi;
             a.x[lo + li] = xi;
@@ -1476,7 +1409,7 @@ __global__ void __launch_bounds__(kSmThreads) k_mg_pcg_sm(MgArgs a, MgSmArgs sa)
         }
         recursive = true;
     }
-    if (cta == 0 && threadIdx.x == 0) {
+    if (cta == 0 && tid == 0) {
         a.stats[0] = (double)k;
         a.stats[1] = rr;
         a.stats[2] = R0;
@@ -2479,64 +2412,24 @@ void pcg_solve_mg(SolverWork& w, const SolverSystem& sys, double tol, long long 
         cluster = cudaOccupancyMaxActiveClusters(&nclusters, (void*)k_mg_pcg<true>, &cfg) == cudaSuccess && nclusters >= 1;
         cudaGetLastError();
     }
-    // above one cluster's size: the shared-memory-resident clustered grid kernel (one CTA per
-    // SM, levels from lc on solved per cluster) when the fused rows exist and K clusters of
-    // kSmCtas can be co-resident
+    // above one cluster's size: the shared-memory-resident grid kernel, one CTA per SM
     bool sec = false;
-    const bool gridc = g.fused && g.dense;  // dense coarsest solved by all CTAs (no cluster levels)
-    int K = 0, nbg = 0;
-    cudaLaunchConfig_t scfg = {};
-    cudaLaunchAttribute sattr[2];
+    int nb = kMgClusterCtas;
     if (!cluster && g.fused && g.levels >= 2) {
         static int sm_state = 0;  // 0 unknown, 1 ok, -1 unsupported
         if (sm_state == 0) {
             sm_state = cudaFuncSetAttribute(k_mg_pcg_sm, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmBytes) == cudaSuccess ? 1 : -1;
             cudaGetLastError();
         }
-        if (sm_state > 0 && gridc) {
-            // dense coarsest on all CTAs: no clusters, one CTA per SM
-            int occ = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mg_pcg_sm, kSmThreads, kSmBytes) == cudaSuccess && occ >= 1) {
-                nbg = std::max(1, std::min({num_sms * occ, num_sms, ceil_div(n, 128)}));
-                scfg.gridDim = dim3(nbg);
-                scfg.blockDim = dim3(kSmThreads);
-                scfg.dynamicSmemBytes = kSmBytes;
-                scfg.stream = s;
-                sattr[0].id = cudaLaunchAttributeCooperative;
-                sattr[0].val.cooperative = 1;
-                scfg.attrs = sattr;
-                scfg.numAttrs = 1;
-                sec = true;
-            }
-            cudaGetLastError();
-        } else if (sm_state > 0) {
-            K = std::max(1, std::min({ceil_div(n, kSmCtas * kSmThreads), kSmMaxClusters, num_sms / kSmCtas}));
-            scfg.gridDim = dim3(K * kSmCtas);
-            scfg.blockDim = dim3(kSmThreads);
-            scfg.dynamicSmemBytes = kSmBytes;
-            scfg.stream = s;
-            sattr[0].id = cudaLaunchAttributeClusterDimension;
-            sattr[0].val.clusterDim.x = kSmCtas;
-            sattr[0].val.clusterDim.y = 1;
-            sattr[0].val.clusterDim.z = 1;
-            sattr[1].id = cudaLaunchAttributeCooperative;
-            sattr[1].val.cooperative = 1;
-            scfg.attrs = sattr;
-            scfg.numAttrs = 2;
-            int ncl = 0;
-            if (cudaOccupancyMaxActiveClusters(&ncl, (void*)k_mg_pcg_sm, &scfg) == cudaSuccess && ncl >= 1) {
-                K = std::min(K, ncl);
-                scfg.gridDim = dim3(K * kSmCtas);
-                sec = true;
-            }
-            cudaGetLastError();
+        int occ = 0;
+        if (sm_state > 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mg_pcg_sm, kSmThreads, kSmBytes) == cudaSuccess && occ >= 1) {
+            nb = std::max(1, std::min({num_sms, kSmThreads, ceil_div(n, 128)}));
+            sec = true;
         }
+        cudaGetLastError();
     }
     if (g.fused && !sec) throw Fail{CICY_E_INTERNAL, "multigrid: the clustered kernel cannot be launched for a hierarchy built for it"};
-    int nb = kMgClusterCtas;
-    if (sec) {
-        nb = gridc ? nbg : K * kSmCtas;
-    } else if (!cluster) {
+    if (!sec && !cluster) {
         int occ = 0;
         CICY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mg_pcg<false>, kMgThreads, 0));
         const int cap = std::max(1, occ) * num_sms;
@@ -2545,14 +2438,7 @@ void pcg_solve_mg(SolverWork& w, const SolverSystem& sys, double tol, long long 
     std::vector<MgSmLevel> hl;  // kept until the stream synchronisation below
     MgSmArgs sa{};
     if (sec) {
-        // levels lc .. coarsest per cluster: r and z above lc, zf from lc on, K copies each
         const int C = g.levels - 1;
-        int lc = C;
-        for (int l = 1; l <= C && !gridc; l++)
-            if (g.L[l].n <= kSmRows) {
-                lc = l;
-                break;
-            }
         hl.assign(C + 1, MgSmLevel{});
         for (int l = 0; l <= C; l++) {
             MgWork::Lvl& L = g.L[l];
@@ -2569,34 +2455,16 @@ void pcg_solve_mg(SolverWork& w, const SolverSystem& sys, double tol, long long 
                 d.agg = L.agg.get();
             }
             d.l1inv = L.l1inv.get();
-            if (l > lc) {
-                L.r_cl.ensure((size_t)K * L.n + 1);
-                L.z_cl.ensure((size_t)K * L.n + 1);
-                d.r = L.r_cl.get();
-                d.z = L.z_cl.get();
-                d.priv |= 1;
-            } else {
-                d.r = L.r.get();
-                d.z = L.z.get();
-            }
-            if (l >= lc && !gridc) {
-                L.zf_cl.ensure((size_t)K * L.n + 1);
-                d.zf = L.zf_cl.get();
-                d.priv |= 2;
-            } else {
-                d.zf = L.zf.get();
-            }
+            d.r = L.r.get();
+            d.z = L.z.get();
+            d.zf = l == C && !g.dense ? d.z : L.zf.get();
         }
         g.sec_lv.ensure(sizeof(MgSmLevel) * (C + 1));
         CICY_CUDA(cudaMemcpyAsync(g.sec_lv.get(), hl.data(), sizeof(MgSmLevel) * (C + 1), cudaMemcpyHostToDevice, s));
-        const int ncl = ceil_div(nb, kSmCtas);
-        g.cl_fail.ensure(ncl);
-        CICY_CUDA(cudaMemsetAsync(g.cl_fail.get(), 0, sizeof(int32_t) * ncl, s));
-        sa.lc = lc;
-        sa.grid_coarse = gridc ? 1 : 0;
         sa.lv = reinterpret_cast<const MgSmLevel*>(g.sec_lv.get());
-        sa.cl_fail = g.cl_fail.get();
         sa.mptr0 = g.L[0].mptr.get();
+        sa.lfac = w.lfac.get();
+        sa.ipiv = w.ipiv.get();
         sa.smem_bytes = kSmBytes;
     }
     w.cta_row.ensure(nb + 1);
@@ -2632,7 +2500,8 @@ void pcg_solve_mg(SolverWork& w, const SolverSystem& sys, double tol, long long 
     if (cluster) {
         CICY_CUDA(cudaLaunchKernelEx(&cfg, k_mg_pcg<true>, a));
     } else if (sec) {
-        CICY_CUDA(cudaLaunchKernelEx(&scfg, k_mg_pcg_sm, a, sa));
+        void* args[] = {&a, &sa};
+        CICY_CUDA(cudaLaunchCooperativeKernel((void*)k_mg_pcg_sm, dim3(nb), dim3(kSmThreads), args, kSmBytes, s));
     } else {
         void* args[] = {&a};
         CICY_CUDA(cudaLaunchCooperativeKernel((void*)k_mg_pcg<false>, dim3(nb), dim3(kMgThreads), args, 0, s));

@@ -40,3 +40,26 @@ def test_hub_rows_against_direct_solve(cuda_ok, degree):
     finally:
         bs.close()
     assert np.max(np.abs(x - sla.spsolve(A.tocsc(), b))) < 1e-10
+
+
+@pytest.mark.parametrize("spokes", [1400, 2200])
+def test_grid_kernel_with_long_rows(cuda_ok, spokes):
+    """A fan of CNTs on one end point through the grid kernel: coarse rows of hundreds of entries
+    (a CTA's phase in several batches) and, with 2,200 spokes, one of more than a batch holds.
+    Both preconditioners stop at 1e-13, as in the other comparisons of solvers."""
+    from test_gpu_assembly import fan_network
+
+    from cicy_geom_b200.device import Context
+    from cicy_geom_b200.network import NetworkConfig
+
+    cfg = NetworkConfig(side=1.0, n_cnts=spokes + 1, seed=0, tolerance=1e-13, tolerance_unit=1e-13, resistances=(1, 0, 0))
+    net, r = fan_network(spokes, cfg), {}
+    for pre in (0, 3):
+        with Context(0) as ctx:
+            ctx.set_solver(preconditioner=pre, cluster=False)
+            ctx.upload(net)
+            res = ctx.network_to_conductance(cfg.params())
+            assert all(s.rel_residual <= 1e-10 for s in res.solves[:res.n_solves])
+            r[pre], S = res.resistances[0], ctx.system(0)
+    assert (np.diff(S["row_ptr"]) + np.bincount(S["col_ind"], minlength=len(S["diag"]))).max() >= spokes
+    assert 0 < r[0] < 1e18 and abs(r[3] - r[0]) <= 1e-9 * r[0]
