@@ -181,51 +181,81 @@ __global__ void k_dense_coarse(int nc, int lanes, const int32_t* __restrict__ rp
 }
 
 // Blocked in-place Gauss-Jordan (32 pivots per block).  For pivot block b with the others o:
-// one warp inverts the Schur-complemented diagonal block D = S_bb pivot by pivot (dropping a
+// four warps invert the Schur-complemented diagonal block D = S_bb two pivots at a time (dropping a
 // variable whose pivot vanishes: its row and column of D^-1 are zero), then the CTA applies the
 // block step S_bo <- D^-1 S_bo, S_ob <- -S_ob D^-1, S_oo <- S_oo - S_ob D^-1 S_bo, S_bb <- D^-1:
 // the unblocked elimination's result with 4 barriers per block instead of 2 per pivot.
 constexpr int kGjBlock = 32;
 constexpr int kGjDS = kGjBlock + 1;  // row stride of a diagonal block in shared memory
 
-// The CTA's kGjThreads (512) threads: D <- D^-1 in place (32 x 32, row stride kGjDS; a smaller
-// block is padded with the identity, which stays decoupled); a variable whose pivot is not
-// above thr is dropped (its row and column of D^-1 are zero).  Thread t holds column t % 32 of
-// rows t / 32 and t / 32 + 16 in registers; each pivot's row and column go through shared
-// memory (fcol, frow), two barriers per pivot, so the pivot chain is a barrier, a division and
-// one FMA per step rather than a warp's serial sweep over the block.
 constexpr int kGjThreads = 512;
-__device__ __forceinline__ void gj_cta_invert(double* D, double* fcol, double* frow, double thr) {
-    static_assert(kGjThreads == 16 * kGjBlock, "two entries of the 32 x 32 block per thread");
-    const int t = threadIdx.x, j = t & 31, i0 = t >> 5, i1 = i0 + 16;
-    double a0 = D[i0 * kGjDS + j], a1 = D[i1 * kGjDS + j];
-    for (int k = 0; k < kGjBlock; k++) {
-        if (j == k) {
-            fcol[i0] = a0;
-            fcol[i1] = a1;
+
+// A 32 x 32 block inverted in place by the CTA's first four warps (kGjInvert threads): thread t holds
+// column t % 32 of rows 8 (t / 32) .. + 7 in a; a smaller block is padded with the identity, which
+// stays decoupled; a variable whose pivot is not above thr is dropped (its row and column of the
+// inverse are zero).  The chain of pivots bounds it, so two are taken at a time: the warp that holds
+// both rows inverts their 2 x 2 block (one division) and publishes the new rows, every thread in the
+// two columns its old entries (two banks in turn: one barrier a pair), and all update.  A block of
+// the grid Gauss-Jordan took 9.3 us with single pivots and 512 threads, 11 with one warp and shuffles.
+constexpr int kGjInvert = 128;
+struct GjBank {
+    double row[2][kGjBlock];   // new pivot rows
+    double2 col[kGjBlock];     // old pivot columns
+};
+__device__ __forceinline__ void gj_invert(double (&a)[8], GjBank (&bank)[2], double thr) {
+    const int w = threadIdx.x >> 5, j = threadIdx.x & 31;
+#pragma unroll 1
+    for (int q = 0; q < 4; q++) {  // the warp that holds the pivots
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+            const int k = 8 * q + 2 * h;
+            GjBank& B = bank[h & 1];
+            if (j == k)
+#pragma unroll
+                for (int e = 0; e < 8; e++) B.col[8 * w + e].x = a[e];
+            if (j == k + 1)
+#pragma unroll
+                for (int e = 0; e < 8; e++) B.col[8 * w + e].y = a[e];
+            if (w == q) {
+                const double u = a[2 * h], v = a[2 * h + 1];
+                const double p11 = __shfl_sync(0xffffffffu, u, k), p12 = __shfl_sync(0xffffffffu, u, k + 1);
+                const double p21 = __shfl_sync(0xffffffffu, v, k), p22 = __shfl_sync(0xffffffffu, v, k + 1);
+                const double det = p11 * p22 - p12 * p21;
+                double i11 = 0, i12 = 0, i21 = 0, i22 = 0;
+                if (p11 > thr && det > thr * p11) {  // det / p11: the second pivot after the first
+                    const double inv = 1.0 / det;
+                    i11 = p22 * inv;
+                    i12 = -p12 * inv;
+                    i21 = -p21 * inv;
+                    i22 = p11 * inv;
+                } else if (p11 > thr) {
+                    i11 = 1.0 / p11;
+                } else if (p22 > thr) {
+                    i22 = 1.0 / p22;
+                }
+                B.row[0][j] = j == k ? i11 : j == k + 1 ? i12 : i11 * u + i12 * v;
+                B.row[1][j] = j == k ? i21 : j == k + 1 ? i22 : i21 * u + i22 * v;
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            const double r0 = B.row[0][j], r1 = B.row[1][j];
+            const bool own = j == k || j == k + 1;
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                const double2 c = B.col[8 * w + e];
+                a[e] = (own ? 0.0 : a[e]) - c.x * r0 - c.y * r1;
+            }
+            if (w == q) {
+                a[2 * h] = r0;
+                a[2 * h + 1] = r1;
+            }
         }
-        if (i0 == k) frow[j] = a0;
-        if (i1 == k) frow[j] = a1;
-        __syncthreads();
-        const double p = frow[k];
-        if (!(p > thr)) {  // vanishing pivot: drop variable k (row k and column k)
-            if (i0 == k || j == k) a0 = 0.0;
-            if (i1 == k || j == k) a1 = 0.0;
-        } else {
-            const double dk = ((j == k) ? 1.0 : frow[j]) / p;  // the new pivot row
-            a0 = (i0 == k) ? dk : ((j == k) ? 0.0 : a0) - fcol[i0] * dk;
-            a1 = (i1 == k) ? dk : ((j == k) ? 0.0 : a1) - fcol[i1] * dk;
-        }
-        __syncthreads();
     }
-    D[i0 * kGjDS + j] = a0;
-    D[i1 * kGjDS + j] = a1;
-    __syncthreads();
 }
+static_assert(kGjInvert == 128 && kGjBlock == 32, "gj_invert: four warps of eight rows");
 
 __global__ void __launch_bounds__(kGjThreads) k_gauss_jordan(int n, double* __restrict__ M) {
     extern __shared__ double S[];  // n * n, then Cb (n x 32), Rb (32 x n), D (32 x 33), f (32)
-    __shared__ double gj_fcol[kGjBlock], gj_frow[kGjBlock];
+    __shared__ GjBank gj_bank[2];
     double* Cb = S + (size_t)n * n;
     double* Rb = Cb + (size_t)n * kGjBlock;
     double* D = Rb + (size_t)kGjBlock * n;
@@ -251,7 +281,15 @@ __global__ void __launch_bounds__(kGjThreads) k_gauss_jordan(int n, double* __re
         }
         for (int e = t; e < n * m; e += kGjThreads) Cb[(e / m) * kGjBlock + e % m] = S[(e / m) * n + b0 + e % m];
         __syncthreads();
-        gj_cta_invert(D, gj_fcol, gj_frow, thr);
+        if (t < kGjInvert) {
+            double a[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) a[e] = D[(8 * (t >> 5) + e) * kGjDS + (t & 31)];
+            gj_invert(a, gj_bank, thr);
+#pragma unroll
+            for (int e = 0; e < 8; e++) D[(8 * (t >> 5) + e) * kGjDS + (t & 31)] = a[e];
+        }
+        __syncthreads();
         // Rb = D^-1 S_bo (columns outside the block)
         for (int e = t; e < m * n; e += kGjThreads) {
             const int ii = e / n, jc = e % n;
@@ -435,146 +473,155 @@ __device__ __forceinline__ bool mg_sync(unsigned long long* bar, unsigned long l
 
 // Dense inverse of a coarsest level too large for one CTA: blocked Gauss-Jordan (32 pivots
 // per block, the drop rule and regularisation of k_gauss_jordan) over the whole grid, one
-// cooperative launch with one grid barrier per block.  CTA c keeps the column strip
-// [c0, c1) of the matrix in shared memory.  Block step b: every CTA reads the block's column
-// panel S[:, b] (global, double-buffered; the strips holding the panel's columns wrote it at
-// the end of step b - 1), inverts the diagonal block D = S_bb (one warp), and updates its own
-// columns j: outside the block R_j = D^-1 S_bj, S_ij -= S_ib R_j (rows outside), S_bj = R_j;
-// inside it S_ij = -S_ib (D^-1)_j (rows outside), S_bj = (D^-1)_j.  The products sum over the
-// block's pivots in order, as k_gauss_jordan's do.
+// cooperative launch with one grid barrier per block.  CTA (pr, pc) of a P x P grid keeps the tile
+// [r0, r1) x [c0, c1) of the matrix in registers.  Block step b: every CTA reads the diagonal block
+// D = S_bb, its rows' part of the column panel S[:, b] and its columns' part of the row panel
+// S[b, :] (global, double-buffered; the tiles that hold the panels wrote them at the end of step
+// b - 1), inverts D, forms X = D^-1 S_bj (columns of the block: D^-1) and updates its tile:
+// S_ij = (j in the block ? 0 : S_ij) - S_ib X_bj outside the block's rows, X in them.
+//
+// A block step is bound by the pivot chain, its panel reads and the barrier.  Column strips, one
+// per CTA, had every CTA read the whole column panel: 41 MB of L2 reads a block at 1,088 rows
+// against 7 MB so: with the pivots two at a time (gj_invert) 883 -> 611 us in all, 753 rows 510 -> 327.
 constexpr int kGjgThreads = 512;
-static_assert(kGjgThreads == kGjThreads, "gj_cta_invert runs on the whole CTA");
-constexpr int kMgDenseGridMax = 1280;  // largest dense coarsest (the grid Gauss-Jordan's strip budget)
-constexpr int kGjgMaxStrip = 10;       // columns per CTA strip (the launch uses at least n / 10 CTAs)
-static_assert(kMgDenseGridMax <= 3 * kGjgThreads, "the grid Gauss-Jordan updates three rows per thread");
+constexpr int kMgDenseGridMax = 1280;  // largest dense coarsest
+constexpr int kGjgTile = 112;          // largest tile edge: the CTA grid has at least n / 112 rows
 
-template <int W>
-__global__ void __launch_bounds__(kGjgThreads) k_gauss_jordan_grid(int n, double* __restrict__ M, double* __restrict__ panel,
+// RT, CT: tile rows / 32 and columns / 16 (thread t holds rows t / 16 + 32 a, columns t % 16 + 16 b).
+template <int RT, int CT>
+__global__ void __launch_bounds__(kGjgThreads) k_gauss_jordan_grid(int n, int P, double* __restrict__ M, double* __restrict__ panel,
                                                                    unsigned long long* bar, unsigned long long* dmax_bits, int* err,
                                                                    long long limit) {
-    extern __shared__ double gsm[];
+    constexpr int TR = 32 * RT, TC = 16 * CT;
+    extern __shared__ double gsm[];  // column panel part (32 x TR), row panel part (32 x TC), X (32 x TC)
+    double* const PI = gsm;
+    double* const RB = PI + kGjBlock * TR;
+    double* const X = RB + kGjBlock * TC;
     __shared__ double Dm[kGjBlock * kGjDS];
-    __shared__ double R[kGjBlock * W];  // the block rows' new values on the strip (rows past the block: 0)
-    __shared__ double gj_fcol[kGjBlock], gj_frow[kGjBlock];
+    __shared__ GjBank gj_bank[2];
     __shared__ int s_ok;
-    const int G = gridDim.x, t = threadIdx.x;
-    const int c0 = (int)((long long)n * blockIdx.x / G), c1 = (int)((long long)n * (blockIdx.x + 1) / G), w = c1 - c0;
-    double* S = gsm;  // the strip, column-major: S[jj * n + i] = M[i][c0 + jj]
+    const int t = threadIdx.x, ty = t >> 4, tx = t & 15;
+    const int pr = blockIdx.x / P, pc = blockIdx.x % P;
+    const int r0 = n * pr / P, nr = n * (pr + 1) / P - r0, c0 = n * pc / P, nc = n * (pc + 1) / P - c0;
+    const size_t half = (size_t)n * kGjBlock;  // panel: column panels 0, 1 (kk * n + i), row panels 0, 1 (kk * n + j)
+    double S[RT][CT];
+    double dm = 0;
+#pragma unroll
+    for (int a = 0; a < RT; a++)
+#pragma unroll
+        for (int b = 0; b < CT; b++) {
+            const int i = r0 + ty + 32 * a, j = c0 + tx + 16 * b;
+            const bool in = ty + 32 * a < nr && tx + 16 * b < nc;
+            double v = in ? M[(size_t)i * n + j] : 0.0;
+            if (in && i == j) {
+                dm = fmax(dm, fabs(v));
+                v *= (1.0 + 1e-8);
+            }
+            S[a][b] = v;
+        }
+    if (dm > 0) atomicMax(dmax_bits, (unsigned long long)__double_as_longlong(dm));  // non-negative: the bits order as the values
+    // the panels of block b0 from the tiles that hold them
+    auto publish = [&](int b0, int bank) {
+        const int m = min(kGjBlock, n - b0);
+#pragma unroll
+        for (int a = 0; a < RT; a++)
+#pragma unroll
+            for (int b = 0; b < CT; b++) {
+                if (ty + 32 * a >= nr || tx + 16 * b >= nc) continue;
+                const int i = r0 + ty + 32 * a, j = c0 + tx + 16 * b;
+                if (j >= b0 && j < b0 + m) panel[bank * half + (size_t)(j - b0) * n + i] = S[a][b];
+                if (i >= b0 && i < b0 + m) panel[(2 + bank) * half + (size_t)(i - b0) * n + j] = S[a][b];
+            }
+    };
+    publish(0, 0);
     unsigned long long target = 0;
-    // the strip, its regularised diagonal, and the largest diagonal (the drop threshold)
-    for (int e = t; e < n * w; e += kGjgThreads) {
-        const int i = e / w, jj = e % w;
-        double v = M[(size_t)i * n + c0 + jj];
-        if (i == c0 + jj) v *= (1.0 + 1e-8);
-        S[(size_t)jj * n + i] = v;
-    }
-    if (t == 0) {
-        double m = 0;
-        for (int jj = 0; jj < w; jj++) m = fmax(m, fabs(M[(size_t)(c0 + jj) * n + c0 + jj]));
-        atomicMax(dmax_bits, (unsigned long long)__double_as_longlong(m));  // non-negative: the bits order as the values
-    }
-    __syncthreads();
-    // panel of block 0 (columns 0 .. 31, column-major; columns past n are zero) from the strips holding them
-    for (int e = t; e < n * w; e += kGjgThreads) {
-        const int jj = e / n, i = e % n, j = c0 + jj;
-        if (j < kGjBlock) panel[(size_t)j * n + i] = S[e];
-    }
-    if (blockIdx.x == 0)
-        for (int e = n * n < kGjBlock * n ? n * n + t : kGjBlock * n; e < kGjBlock * n; e += kGjgThreads) panel[e] = 0.0;
     if (!mg_sync(bar, target, err, &s_ok, limit)) return;
     const double thr = 1e-12 * __longlong_as_double((long long)__ldcg(dmax_bits));
     const int nblk = (n + kGjBlock - 1) / kGjBlock;
     for (int bk = 0; bk < nblk; bk++) {
         const int b0 = bk * kGjBlock, m = min(kGjBlock, n - b0);
-        const double* P = panel + (size_t)(bk & 1) * n * kGjBlock;  // P[kk * n + i] = S[i][b0 + kk] (0 for kk >= m)
-        double* Pn = panel + (size_t)((bk + 1) & 1) * n * kGjBlock;
-        for (int e = t; e < kGjBlock * kGjBlock; e += kGjgThreads) {
-            const int c = e / kGjBlock, r = e % kGjBlock;
-            Dm[r * kGjDS + c] = (r < m && c < m) ? __ldcg(&P[(size_t)c * n + b0 + r]) : (r == c ? 1.0 : 0.0);
-        }
-        __syncthreads();
-        gj_cta_invert(Dm, gj_fcol, gj_frow, thr);
-        // X = the block rows' new values on the strip: D^-1 S_b,j outside the block, (D^-1)_j inside
-        for (int e = t; e < kGjBlock * W; e += kGjgThreads) {
-            const int ii = e / W, jj = e % W, j = c0 + jj;
-            double v = 0;
-            if (ii < m && jj < w) {
-                if (j >= b0 && j < b0 + m) {
-                    v = Dm[ii * kGjDS + (j - b0)];
-                } else {
-                    for (int kk = 0; kk < m; kk++) v += Dm[ii * kGjDS + kk] * S[(size_t)jj * n + b0 + kk];
+        const double* cp = panel + (bk & 1) * half;
+        const double* rp = panel + (2 + (bk & 1)) * half;
+        // four warps invert the diagonal block while the others fetch the panels
+        if (t < kGjInvert) {
+            double a[8];
+            const int w8 = 8 * (t >> 5), j = t & 31;
+#pragma unroll
+            for (int e = 0; e < 8; e++) a[e] = (w8 + e < m && j < m) ? __ldcg(&rp[(size_t)(w8 + e) * n + b0 + j]) : (w8 + e == j ? 1.0 : 0.0);
+            gj_invert(a, gj_bank, thr);
+#pragma unroll
+            for (int e = 0; e < 8; e++) Dm[(w8 + e) * kGjDS + j] = a[e];
+        } else {
+            constexpr int T = kGjgThreads - kGjInvert;
+            for (int e0 = t - kGjInvert; e0 < kGjBlock * (TR + TC); e0 += 4 * T) {
+                double v[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int e = e0 + u * T, f = e - kGjBlock * TR;
+                    v[u] = 0;
+                    if (f < 0) {
+                        if (e / TR < m && e % TR < nr) v[u] = __ldcg(&cp[(size_t)(e / TR) * n + r0 + e % TR]);
+                    } else if (f < kGjBlock * TC) {
+                        if (f / TC < m && f % TC < nc) v[u] = __ldcg(&rp[(size_t)(f / TC) * n + c0 + f % TC]);
+                    }
                 }
-            }
-            R[e] = v;
-        }
-        __syncthreads();
-        // rows: three per thread (t, t + 512, t + 1024); S_ij <- (j in the block ? 0 : S_ij) - sum_k S_ik X_kj,
-        // the sums over the block's pivots in order; the block's own rows take X
-        constexpr int RPT = 3;
-        int ri[RPT];
-        bool live[RPT], upd[RPT];
 #pragma unroll
-        for (int q = 0; q < RPT; q++) {
-            ri[q] = t + q * kGjgThreads;
-            live[q] = ri[q] < n;
-            upd[q] = live[q] && !(ri[q] >= b0 && ri[q] < b0 + m);
-        }
-        double acc[RPT][W];
-#pragma unroll
-        for (int q = 0; q < RPT; q++)
-#pragma unroll
-            for (int jj = 0; jj < W; jj++) acc[q][jj] = 0.0;
-#pragma unroll
-        for (int kc = 0; kc < kGjBlock; kc += 4) {
-            double ph[RPT][4];
-#pragma unroll
-            for (int q = 0; q < RPT; q++)
-#pragma unroll
-                for (int u = 0; u < 4; u++) ph[q][u] = upd[q] ? __ldcg(&P[(size_t)(kc + u) * n + ri[q]]) : 0.0;
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int jj = 0; jj < W; jj++) {
-                    const double x = R[(kc + u) * W + jj];
-#pragma unroll
-                    for (int q = 0; q < RPT; q++) acc[q][jj] += ph[q][u] * x;
-                }
-        }
-#pragma unroll
-        for (int q = 0; q < RPT; q++) {
-            if (!live[q]) continue;
-            const int i = ri[q];
-#pragma unroll
-            for (int jj = 0; jj < W; jj++) {
-                if (jj >= w) continue;
-                const int j = c0 + jj;
-                double v;
-                if (!upd[q]) {
-                    v = R[(i - b0) * W + jj];
-                } else {
-                    const double old = (j >= b0 && j < b0 + m) ? 0.0 : S[(size_t)jj * n + i];
-                    v = old - acc[q][jj];
-                }
-                S[(size_t)jj * n + i] = v;
+                for (int u = 0; u < 4; u++)
+                    if (e0 + u * T < kGjBlock * (TR + TC)) PI[e0 + u * T] = v[u];  // (the row panel's part follows the column panel's)
             }
         }
         __syncthreads();
-        // the next block's panel (columns past n zero) from the strips that hold its columns
+        {  // X: rows ty of the block (0 past it)
+            double x[CT] = {};
+#pragma unroll 8
+            for (int kk = 0; kk < kGjBlock; kk++) {
+                const double d = Dm[ty * kGjDS + kk];
+#pragma unroll
+                for (int b = 0; b < CT; b++) x[b] += d * RB[kk * TC + tx + 16 * b];
+            }
+#pragma unroll
+            for (int b = 0; b < CT; b++) {
+                const int jb = c0 + tx + 16 * b - b0;
+                X[ty * TC + tx + 16 * b] = ty >= m ? 0.0 : jb >= 0 && jb < m ? Dm[ty * kGjDS + jb] : x[b];
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < CT; b++) {
+            const int jb = c0 + tx + 16 * b - b0;
+            if (jb >= 0 && jb < m)
+#pragma unroll
+                for (int a = 0; a < RT; a++) S[a][b] = 0.0;
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int kk = 0; kk < kGjBlock; kk++) {
+            double pv[RT], xv[CT];
+#pragma unroll
+            for (int a = 0; a < RT; a++) pv[a] = PI[kk * TR + ty + 32 * a];
+#pragma unroll
+            for (int b = 0; b < CT; b++) xv[b] = X[kk * TC + tx + 16 * b];
+#pragma unroll
+            for (int a = 0; a < RT; a++)
+#pragma unroll
+                for (int b = 0; b < CT; b++) S[a][b] -= pv[a] * xv[b];
+        }
+#pragma unroll
+        for (int a = 0; a < RT; a++) {  // the block's own rows take X
+            const int ib = r0 + ty + 32 * a - b0;
+            if (ty + 32 * a < nr && ib >= 0 && ib < m)
+#pragma unroll
+                for (int b = 0; b < CT; b++) S[a][b] = X[ib * TC + tx + 16 * b];
+        }
         if (bk + 1 < nblk) {
-            const int nb0 = b0 + kGjBlock, nm = min(kGjBlock, n - nb0);
-            for (int e = t; e < n * w; e += kGjgThreads) {
-                const int jj = e / n, i = e % n, j = c0 + jj;
-                if (j >= nb0 && j < nb0 + nm) Pn[(size_t)(j - nb0) * n + i] = S[e];
-            }
-            if (blockIdx.x == 0)
-                for (int e = nm * n + t; e < kGjBlock * n; e += kGjgThreads) Pn[e] = 0.0;
+            publish(b0 + kGjBlock, (bk + 1) & 1);
+            if (!mg_sync(bar, target, err, &s_ok, limit)) return;
         }
-        if (!mg_sync(bar, target, err, &s_ok, limit)) return;
     }
-    for (int e = t; e < n * w; e += kGjgThreads) {
-        const int i = e / w, jj = e % w;
-        M[(size_t)i * n + c0 + jj] = S[(size_t)jj * n + i];
-    }
+#pragma unroll
+    for (int a = 0; a < RT; a++)
+#pragma unroll
+        for (int b = 0; b < CT; b++)
+            if (ty + 32 * a < nr && tx + 16 * b < nc) M[(size_t)(r0 + ty + 32 * a) * n + c0 + tx + 16 * b] = S[a][b];
 }
 
 // Cluster variant: the hardware cluster barrier (release/acquire at cluster
@@ -2226,6 +2273,13 @@ int pairwise(MgWork& g, int l, cudaStream_t s, int64_t& launches) {
 
 }  // namespace
 
+// Edge of the grid Gauss-Jordan's CTA grid: the largest square that is resident at once.
+int gj_grid(int sms) {
+    int P = 1;
+    while ((P + 1) * (P + 1) <= sms) P++;
+    return P;
+}
+
 // ---------------------------------------------------------------------------
 void build_mg_hierarchy(SolverWork& w, const SolverSystem& sys, cudaStream_t s, int64_t& launches, bool fused, bool smooth, int* status) {
     MgWork& g = w.mg;
@@ -2254,7 +2308,7 @@ void build_mg_hierarchy(SolverWork& w, const SolverSystem& sys, cudaStream_t s, 
         int dev = 0, sms = 0;
         CICY_CUDA(cudaGetDevice(&dev));
         CICY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        dense_cap = std::max(kMgDenseMax, std::min(kMgDenseGridMax, sms * kGjgMaxStrip));
+        dense_cap = std::max(kMgDenseMax, std::min(kMgDenseGridMax, gj_grid(sms) * kGjgTile));
     }
     for (int l = 0;; l++) {
         coarsen(g, l, nc, s, launches);
@@ -2285,7 +2339,7 @@ void build_mg_hierarchy(SolverWork& w, const SolverSystem& sys, cudaStream_t s, 
         CICY_CUDA(cudaGetDevice(&dev));
         CICY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         g.cinv.ensure((size_t)nC * nC);
-        g.gj_panel.ensure((size_t)2 * nC * kGjBlock);
+        g.gj_panel.ensure((size_t)4 * nC * kGjBlock);
         g.gj_sync.ensure(2);
         g.gj_err.ensure(1);
         CICY_CUDA(cudaMemsetAsync(g.gj_sync.get(), 0, sizeof(unsigned long long) * 2, s));
@@ -2296,31 +2350,25 @@ void build_mg_hierarchy(SolverWork& w, const SolverSystem& sys, cudaStream_t s, 
         }
         CICY_CUDA(cudaMemsetAsync(g.cinv.get(), 0, sizeof(double) * nC * nC, s));
         k_dense_coarse<<<grid_for(32LL * nC, 128), 128, 0, s>>>(nC, 32, Lc.rp.get(), Lc.ci.get(), Lc.val.get(), Lc.diag.get(), g.cinv.get());
-        const int G = std::max(1, std::min(sms, nC));
-        const int wmax = (nC + G - 1) / G;
-        if (wmax > kGjgMaxStrip) throw Fail{CICY_E_INTERNAL, "multigrid: dense coarsest too large for this GPU"};
-        const size_t smem = sizeof(double) * (size_t)nC * wmax;
-        void (*kern)(int, double*, double*, unsigned long long*, unsigned long long*, int*, long long) = nullptr;
-        switch (wmax) {
-            case 1: kern = k_gauss_jordan_grid<1>; break;
-            case 2: kern = k_gauss_jordan_grid<2>; break;
-            case 3: kern = k_gauss_jordan_grid<3>; break;
-            case 4: kern = k_gauss_jordan_grid<4>; break;
-            case 5: kern = k_gauss_jordan_grid<5>; break;
-            case 6: kern = k_gauss_jordan_grid<6>; break;
-            case 7: kern = k_gauss_jordan_grid<7>; break;
-            case 8: kern = k_gauss_jordan_grid<8>; break;
-            case 9: kern = k_gauss_jordan_grid<9>; break;
-            default: kern = k_gauss_jordan_grid<10>; break;
-        }
+        int P = gj_grid(sms);
+        const int tile = (nC + P - 1) / P;
+        if (tile > kGjgTile) throw Fail{CICY_E_INTERNAL, "multigrid: dense coarsest too large for this GPU"};
+        void (*kern)(int, int, double*, double*, unsigned long long*, unsigned long long*, int*, long long) = nullptr;
+        int edge[2];  // rows and columns of the kernel's tile
+        if (tile <= 32) kern = k_gauss_jordan_grid<1, 2>, edge[0] = 32, edge[1] = 32;
+        else if (tile <= 64) kern = k_gauss_jordan_grid<2, 4>, edge[0] = 64, edge[1] = 64;
+        else if (tile <= 80) kern = k_gauss_jordan_grid<3, 5>, edge[0] = 96, edge[1] = 80;
+        else if (tile <= 96) kern = k_gauss_jordan_grid<3, 6>, edge[0] = 96, edge[1] = 96;
+        else kern = k_gauss_jordan_grid<4, 7>, edge[0] = 128, edge[1] = 112;
+        const size_t smem = sizeof(double) * kGjBlock * (edge[0] + 2 * edge[1]);
         CICY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         double* M = g.cinv.get();
         double* panel = g.gj_panel.get();
         unsigned long long* bar = g.gj_sync.get();
         unsigned long long* dmax = g.gj_sync.get() + 1;
         long long limit = w.spin_limit;
-        void* args[] = {&nC, &M, &panel, &bar, &dmax, &err, &limit};
-        CICY_CUDA(cudaLaunchCooperativeKernel((void*)kern, dim3(G), dim3(kGjgThreads), args, smem, s));
+        void* args[] = {&nC, &P, &M, &panel, &bar, &dmax, &err, &limit};
+        CICY_CUDA(cudaLaunchCooperativeKernel((void*)kern, dim3(P * P), dim3(kGjgThreads), args, smem, s));
         launches += 2;
         g.dense = true;
     }
