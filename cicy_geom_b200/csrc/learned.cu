@@ -300,9 +300,13 @@ __global__ void k_edge_out(int n, const int32_t* __restrict__ rp, const int32_t*
 }
 
 // ---------------------------------------------------------------------------
-// Preconditioner pieces (FP64)
+// Preconditioner pieces (FP64).  The probe vectors of a group are handled by one launch each, probe
+// blockIdx.y at stride n: with a launch per probe and step, a training step of four probes was bound
+// by 290 launches of 3-4 us (3 um, 2 %: 2.12 ms a step, 1.45 so).
 __global__ void k_spmv(int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ v,
                        const double* __restrict__ x, double* __restrict__ y) {
+    x += (size_t)blockIdx.y * n;
+    y += (size_t)blockIdx.y * n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double s = 0;
         for (int k = rp[i]; k < rp[i + 1]; k++) s += v[k] * x[ci[k]];
@@ -310,13 +314,16 @@ __global__ void k_spmv(int n, const int32_t* __restrict__ rp, const int32_t* __r
     }
 }
 
+// out = T^-1 x, or (with add, which may be out) a T^-1 x + add.
 __global__ void k_tapply(int n, const double* __restrict__ tinv, const int32_t* __restrict__ off, const int32_t* __restrict__ base,
-                         const int32_t* __restrict__ m, const double* __restrict__ x, double* __restrict__ y) {
+                         const int32_t* __restrict__ m, const double* __restrict__ x, double a, const double* add, double* out) {
+    const size_t o0 = (size_t)blockIdx.y * n;
+    x += o0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double s = 0;
         const int o = off[i], b = base[i];
         for (int j = 0; j < m[i]; j++) s += tinv[o + j] * x[b + j];
-        y[i] = s;
+        out[o0 + i] = add ? a * s + add[o0 + i] : s;
     }
 }
 
@@ -324,6 +331,8 @@ __global__ void k_tapply(int n, const double* __restrict__ tinv, const int32_t* 
 __global__ void k_ew_apply(int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ v,
                            const float* __restrict__ w, const uint8_t* __restrict__ offb, const double* __restrict__ y,
                            double* __restrict__ u) {
+    y += (size_t)blockIdx.y * n;
+    u += (size_t)blockIdx.y * n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double s = 0;
         for (int k = rp[i]; k < rp[i + 1]; k++)
@@ -332,14 +341,12 @@ __global__ void k_ew_apply(int n, const int32_t* __restrict__ rp, const int32_t*
     }
 }
 
-// out = a x + y; out may be y (in-place updates), so neither is restrict-qualified.
-__global__ void k_axpy(int n, double a, const double* __restrict__ x, const double* y, double* out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = a * x[i] + y[i];
-}
-
-// Dot products r.q, r.r, q.q: per-CTA partials, then one thread sums them in order.
+// Dot products r.q, r.r, q.q: per-CTA partials, then one thread per probe sums them in order.
 __global__ void k_dots3(int n, const double* __restrict__ r, const double* __restrict__ q, double* __restrict__ part) {
     __shared__ double s[3][32];
+    r += (size_t)blockIdx.y * n;
+    q += (size_t)blockIdx.y * n;
+    part += (size_t)blockIdx.y * 3 * gridDim.x;
     double a = 0, b = 0, c = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         a += r[i] * q[i];
@@ -362,29 +369,44 @@ __global__ void k_dots3(int n, const double* __restrict__ r, const double* __res
     }
 }
 
-// loss of one probe and the coefficients of dL/dq = alpha r + beta q
-__global__ void k_probe_loss(int nb, const double* __restrict__ part, double* __restrict__ coef, double* __restrict__ loss) {
-    if (blockIdx.x || threadIdx.x) return;
-    double rq = 0, rr = 0, qq = 0;
-    for (int b = 0; b < nb; b++) { rq += part[3 * b]; rr += part[3 * b + 1]; qq += part[3 * b + 2]; }
-    const double den = rr * qq;
-    coef[0] = -2 * rq / den;
-    coef[1] = 2 * rq * rq / (den * qq);
-    loss[0] += 1 - rq * rq / den;
+// Losses of a group of probes (added to loss in order) and each probe's coefficients of
+// dL/dq = coef[2p] r + coef[2p + 1] q.
+constexpr int kProbeGroup = 8;
+__global__ void k_probe_loss(int probes, int nb, const double* __restrict__ part, double* __restrict__ coef, double* __restrict__ loss) {
+    __shared__ double l[kProbeGroup];
+    const int p = threadIdx.x;
+    if (p < probes) {
+        const double* q = part + (size_t)p * 3 * nb;
+        double rq = 0, rr = 0, qq = 0;
+        for (int b = 0; b < nb; b++) { rq += q[3 * b]; rr += q[3 * b + 1]; qq += q[3 * b + 2]; }
+        const double den = rr * qq;
+        coef[2 * p] = -2 * rq / den;
+        coef[2 * p + 1] = 2 * rq * rq / (den * qq);
+        l[p] = 1 - rq * rq / den;
+    }
+    __syncthreads();
+    if (p == 0)
+        for (int k = 0; k < probes; k++) loss[0] += l[k];
 }
 
 __global__ void k_combine(int n, const double* __restrict__ coef, const double* __restrict__ r, const double* __restrict__ q,
                           double* __restrict__ out) {
-    const double a = coef[0], b = coef[1];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = a * r[i] + b * q[i];
+    const size_t o = (size_t)blockIdx.y * n;
+    const double a = coef[2 * blockIdx.y], b = coef[2 * blockIdx.y + 1];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[o + i] = a * r[o + i] + b * q[o + i];
 }
 
-__global__ void k_dw(int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ v,
+// dw_k += the probes' derivatives, in their order.
+__global__ void k_dw(int n, int probes, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ v,
                      const uint8_t* __restrict__ offb, const double* __restrict__ lam, const double* __restrict__ y,
                      double* __restrict__ dw) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         for (int k = rp[i]; k < rp[i + 1]; k++)
-            if (offb[k]) dw[k] += lam[i] * (-v[k]) * y[ci[k]];
+            if (offb[k]) {
+                double d = dw[k];
+                for (int p = 0; p < probes; p++) d += lam[(size_t)p * n + i] * (-v[k]) * y[(size_t)p * n + ci[k]];
+                dw[k] = d;
+            }
 }
 
 __global__ void k_do(int nnz, double scale, const double* __restrict__ dw, const float* __restrict__ w, const uint8_t* __restrict__ offb,
@@ -617,40 +639,43 @@ void gnn_forward(GnnState& g, const float* P, cudaStream_t s, int64_t& launches)
     CICY_LAUNCH_CHECK();
 }
 
-// z = T^-1 r + T^-1 E_w T^-1 r; y keeps T^-1 r
-static void spai_apply(GnnState& g, const double* r, double* y, double* u, double* z, cudaStream_t s, int64_t& launches) {
+// z = T^-1 r + T^-1 E_w T^-1 r for `probes` vectors; y keeps T^-1 r
+static void spai_apply(GnnState& g, int probes, const double* r, double* y, double* u, double* z, cudaStream_t s, int64_t& launches) {
     const int n = g.n;
-    k_tapply<<<grid_for(n), 256, 0, s>>>(n, g.sw.tinv.get(), g.sw.row_off.get(), g.sw.row_base.get(), g.sw.row_m.get(), r, y);
-    k_ew_apply<<<grid_for(n), 256, 0, s>>>(n, g.rp, g.ci, g.val, g.w.get(), g.offb.get(), y, u);
-    k_tapply<<<grid_for(n), 256, 0, s>>>(n, g.sw.tinv.get(), g.sw.row_off.get(), g.sw.row_base.get(), g.sw.row_m.get(), u, z);
-    k_axpy<<<grid_for(n), 256, 0, s>>>(n, 1.0, y, z, z);
-    launches += 4;
+    const dim3 grid(grid_for(n), probes);
+    k_tapply<<<grid, 256, 0, s>>>(n, g.sw.tinv.get(), g.sw.row_off.get(), g.sw.row_base.get(), g.sw.row_m.get(), r, 1.0, nullptr, y);
+    k_ew_apply<<<grid, 256, 0, s>>>(n, g.rp, g.ci, g.val, g.w.get(), g.offb.get(), y, u);
+    k_tapply<<<grid, 256, 0, s>>>(n, g.sw.tinv.get(), g.sw.row_off.get(), g.sw.row_base.get(), g.sw.row_m.get(), u, 1.0, y, z);
+    launches += 3;
 }
 
 double gnn_loss_grad(GnnState& g, const float* P, int K, const double* probes, float* grad, cudaStream_t s, int64_t& launches) {
     const int n = g.n, nnz = g.nnz;
     gnn_forward(g, P, s, launches);
-    g.vr.ensure(n + 1); g.vy.ensure(n + 1); g.vu.ensure(n + 1); g.vz.ensure(n + 1); g.vq.ensure(n + 1);
-    g.vd.ensure(n + 1); g.vl.ensure(n + 1);
+    const size_t nv = (size_t)n * std::min(K, kProbeGroup) + 1;
+    g.vr.ensure(nv); g.vy.ensure(nv); g.vu.ensure(nv); g.vz.ensure(nv); g.vq.ensure(nv);
+    g.vd.ensure(nv); g.vl.ensure(nv);
     g.dw.ensure(nnz + 1);
     g.dout.ensure(nnz + 1);
     const int nbd = std::min(grid_for(n), 256);
-    g.part.ensure(3 * (size_t)nbd + 3);
-    g.coef.ensure(4);
+    g.part.ensure((size_t)kProbeGroup * 3 * nbd);
+    g.coef.ensure(2 * kProbeGroup + 2);
+    double* const loss = g.coef.get() + 2 * kProbeGroup;
     CICY_CUDA(cudaMemsetAsync(g.dw.get(), 0, sizeof(double) * (nnz + 1), s));
-    CICY_CUDA(cudaMemsetAsync(g.coef.get(), 0, sizeof(double) * 4, s));
-    for (int p = 0; p < K; p++) {
-        const double* u0 = probes + (size_t)p * n;
-        k_spmv<<<grid_for(n), 256, 0, s>>>(n, g.rp, g.ci, g.val, u0, g.vr.get());
-        spai_apply(g, g.vr.get(), g.vy.get(), g.vu.get(), g.vz.get(), s, launches);
-        k_spmv<<<grid_for(n), 256, 0, s>>>(n, g.rp, g.ci, g.val, g.vz.get(), g.vq.get());
-        k_dots3<<<nbd, 256, 0, s>>>(n, g.vr.get(), g.vq.get(), g.part.get());
-        k_probe_loss<<<1, 32, 0, s>>>(nbd, g.part.get(), g.coef.get(), g.coef.get() + 2);
-        k_combine<<<grid_for(n), 256, 0, s>>>(n, g.coef.get(), g.vr.get(), g.vq.get(), g.vd.get());  // dL/dq
-        k_spmv<<<grid_for(n), 256, 0, s>>>(n, g.rp, g.ci, g.val, g.vd.get(), g.vu.get());             // dL/dz
-        k_tapply<<<grid_for(n), 256, 0, s>>>(n, g.sw.tinv.get(), g.sw.row_off.get(), g.sw.row_base.get(), g.sw.row_m.get(), g.vu.get(),
-                                             g.vl.get());                                              // lambda
-        k_dw<<<grid_for(n), 256, 0, s>>>(n, g.rp, g.ci, g.val, g.offb.get(), g.vl.get(), g.vy.get(), g.dw.get());
+    CICY_CUDA(cudaMemsetAsync(loss, 0, sizeof(double), s));
+    for (int p = 0; p < K; p += kProbeGroup) {
+        const int np = std::min(kProbeGroup, K - p);
+        const dim3 grid(grid_for(n), np);
+        k_spmv<<<grid, 256, 0, s>>>(n, g.rp, g.ci, g.val, probes + (size_t)p * n, g.vr.get());
+        spai_apply(g, np, g.vr.get(), g.vy.get(), g.vu.get(), g.vz.get(), s, launches);
+        k_spmv<<<grid, 256, 0, s>>>(n, g.rp, g.ci, g.val, g.vz.get(), g.vq.get());
+        k_dots3<<<dim3(nbd, np), 256, 0, s>>>(n, g.vr.get(), g.vq.get(), g.part.get());
+        k_probe_loss<<<1, 32, 0, s>>>(np, nbd, g.part.get(), g.coef.get(), loss);
+        k_combine<<<grid, 256, 0, s>>>(n, g.coef.get(), g.vr.get(), g.vq.get(), g.vd.get());  // dL/dq
+        k_spmv<<<grid, 256, 0, s>>>(n, g.rp, g.ci, g.val, g.vd.get(), g.vu.get());             // dL/dz
+        k_tapply<<<grid, 256, 0, s>>>(n, g.sw.tinv.get(), g.sw.row_off.get(), g.sw.row_base.get(), g.sw.row_m.get(), g.vu.get(), 1.0,
+                                      nullptr, g.vl.get());  // lambda
+        k_dw<<<grid_for(n), 256, 0, s>>>(n, np, g.rp, g.ci, g.val, g.offb.get(), g.vl.get(), g.vy.get(), g.dw.get());
         launches += 8;
     }
     k_do<<<grid_for(nnz), 256, 0, s>>>(nnz, 1.0 / K, g.dw.get(), g.w.get(), g.offb.get(), g.dout.get());
@@ -677,26 +702,25 @@ double gnn_loss_grad(GnnState& g, const float* P, int K, const double* probes, f
     }
     k_layer0_bwd<<<warps_grid(n), 256, 0, s>>>(n, g.f.get(), g.A0.get(), dh, grad);
     launches++;
-    double h[4];
-    CICY_CUDA(cudaMemcpyAsync(h, g.coef.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
+    double h = 0;
+    CICY_CUDA(cudaMemcpyAsync(&h, loss, sizeof(h), cudaMemcpyDeviceToHost, s));
     CICY_CUDA(cudaStreamSynchronize(s));
     CICY_LAUNCH_CHECK();
-    return h[2] / K;
+    return h / K;
 }
 
 // u <- u - 0.9 T^-1 A u, `sweeps` times, for each of K probe vectors
 void gnn_smooth_probes(GnnState& g, int K, double* u, int sweeps, cudaStream_t s, int64_t& launches) {
     const int n = g.n;
-    g.vr.ensure(n + 1);
-    g.vy.ensure(n + 1);
-    for (int p = 0; p < K; p++) {
+    g.vr.ensure((size_t)n * std::min(std::max(K, 1), kProbeGroup) + 1);
+    for (int p = 0; p < K; p += kProbeGroup) {
         double* up = u + (size_t)p * n;
+        const dim3 grid(grid_for(n), std::min(kProbeGroup, K - p));
         for (int it = 0; it < sweeps; it++) {
-            k_spmv<<<grid_for(n), 256, 0, s>>>(n, g.rp, g.ci, g.val, up, g.vr.get());
-            k_tapply<<<grid_for(n), 256, 0, s>>>(n, g.sw.tinv.get(), g.sw.row_off.get(), g.sw.row_base.get(), g.sw.row_m.get(), g.vr.get(),
-                                                 g.vy.get());
-            k_axpy<<<grid_for(n), 256, 0, s>>>(n, -0.9, g.vy.get(), up, up);
-            launches += 3;
+            k_spmv<<<grid, 256, 0, s>>>(n, g.rp, g.ci, g.val, up, g.vr.get());
+            k_tapply<<<grid, 256, 0, s>>>(n, g.sw.tinv.get(), g.sw.row_off.get(), g.sw.row_base.get(), g.sw.row_m.get(), g.vr.get(), -0.9, up,
+                                          up);
+            launches += 2;
         }
     }
     CICY_LAUNCH_CHECK();
