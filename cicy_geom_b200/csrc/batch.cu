@@ -173,26 +173,94 @@ __device__ void factor_chains(const BatchSys& S, PT* lf, PT* ip) {
     }
 }
 
-// z = T^-1 r chain by chain: forward (y_k = r_k - l_k y_{k-1}), backward
-// (z_k = y_k / p_k - l_{k+1} z_{k+1}); l = 0 at block starts ends a block.
+// z = T^-1 r on chains [c_lo, c_hi), a thread each: forward (y_k = r_k - l_k y_{k-1}), backward
+// (z_k = y_k / p_k - l_{k+1} z_{k+1}); l = 0 at block starts ends a block.  A serial recurrence
+// over data in L2: four rows' operands are loaded together.
 template <typename PT>
-__device__ void apply_chains(const BatchSys& S, const PT* lf, const PT* ip, const double* r, double* z) {
-    for (int c = threadIdx.x; c < S.nchains; c += blockDim.x) {
-        const int s0 = S.cs[c], m = S.cl[c];
-        if (m <= 0) continue;
-        PT y = (PT)r[s0];
-        z[s0] = (double)y;
-        for (int k = 1; k < m; k++) {
-            y = (PT)r[s0 + k] - lf[s0 + k] * y;
-            z[s0 + k] = (double)y;
+__device__ __forceinline__ void apply_chains(const BatchSys& S, int c_lo, int c_hi, const PT* lf, const PT* ip, const double* r, double* z) {
+    for (int c = c_lo + threadIdx.x; c < c_hi; c += blockDim.x) {
+        const int s0 = S.cs[c], s1 = s0 + S.cl[c];
+        PT y = (PT)0;
+        for (int k0 = s0; k0 < s1; k0 += 4) {
+            PT rv[4], lv[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int k = min(k0 + u, s1 - 1);
+                rv[u] = (PT)r[k];
+                lv[u] = k > s0 ? lf[k] : (PT)0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (k0 + u < s1) {
+                    y = rv[u] - lv[u] * y;
+                    z[k0 + u] = (double)y;
+                }
         }
-        PT zn = (PT)z[s0 + m - 1] * ip[s0 + m - 1];
-        z[s0 + m - 1] = (double)zn;
-        for (int k = m - 2; k >= 0; k--) {
-            zn = (PT)z[s0 + k] * ip[s0 + k] - lf[s0 + k + 1] * zn;
-            z[s0 + k] = (double)zn;
+        PT zn = (PT)0;
+        for (int k0 = s1 - 1; k0 >= s0; k0 -= 4) {
+            PT zv[4], pv[4], lv[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int k = max(k0 - u, s0);
+                zv[u] = (PT)z[k];
+                pv[u] = ip[k];
+                lv[u] = k + 1 < s1 ? lf[k + 1] : (PT)0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (k0 - u >= s0) {
+                    zn = zv[u] * pv[u] - lv[u] * zn;
+                    z[k0 - u] = (double)zn;
+                }
         }
     }
+}
+
+// Row products of the iteration, four entries at a time: indices and weights first, vector entries
+// second (rows have two to five entries, and an entry at a time was two dependent L2 loads each).
+// sum_k val[k] x(ci[k])
+template <class X>
+__device__ __forceinline__ double row_dot(const BatchSys& S, int i, X x) {
+    const int e = S.rp[i + 1];
+    double s = 0;
+    for (int k0 = S.rp[i]; k0 < e; k0 += 4) {
+        int c[4];
+        double w[4], v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            c[u] = k0 + u < e ? S.ci[k0 + u] : -1;
+            w[u] = k0 + u < e ? S.val[k0 + u] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = c[u] >= 0 ? x(c[u]) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; u++) s += w[u] * v[u];
+    }
+    return s;
+}
+
+// The learned coupling term: sum_k ew[k] (-val[k]) y(ci[k]) over the weighted entries
+template <class X>
+__device__ __forceinline__ double row_coupling(const BatchSys& S, int i, X y) {
+    const int e = S.rp[i + 1];
+    double s = 0;
+    for (int k0 = S.rp[i]; k0 < e; k0 += 4) {
+        int c[4];
+        float w[4];
+        double g[4], v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            c[u] = k0 + u < e ? S.ci[k0 + u] : 0;
+            w[u] = k0 + u < e ? S.ew[k0 + u] : 0.0f;
+            g[u] = k0 + u < e ? S.val[k0 + u] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) v[u] = w[u] != 0.0f ? y(c[u]) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (w[u] != 0.0f) s += (double)w[u] * (-g[u]) * v[u];
+    }
+    return s;
 }
 
 // FP64 residual r = b - A x, returns this thread's share of |r|^2.
@@ -275,9 +343,9 @@ __global__ void __launch_bounds__(T) k_batch_pcg(BatchArgs a) {
             if (PK == 0) {
                 for (int i = threadIdx.x; i < n; i += T) z[i] = (double)((PT)r[i] * ip[i]);
             } else if (PK == 2) {
-                apply_chains<PT>(S, lf, ip, r, z);
+                apply_chains<PT>(S, 0, S.nchains, lf, ip, r, z);
             } else {
-                apply_chains<PT>(S, lf, ip, r, y);
+                apply_chains<PT>(S, 0, S.nchains, lf, ip, r, y);
                 __syncthreads();
                 for (int i = threadIdx.x; i < n; i += T) {
                     if (MX) {
@@ -288,16 +356,11 @@ __global__ void __launch_bounds__(T) k_batch_pcg(BatchArgs a) {
                         }
                         u[i] = (double)s;
                     } else {
-                        double s = 0;
-                        for (int kk = S.rp[i]; kk < S.rp[i + 1]; kk++) {
-                            const float w = S.ew[kk];
-                            if (w != 0.0f) s += (double)w * (-S.val[kk]) * y[S.ci[kk]];
-                        }
-                        u[i] = s;
+                        u[i] = row_coupling(S, i, [&](int c) { return y[c]; });
                     }
                 }
                 __syncthreads();
-                apply_chains<PT>(S, lf, ip, u, z);
+                apply_chains<PT>(S, 0, S.nchains, lf, ip, u, z);
                 __syncthreads();
                 for (int i = threadIdx.x; i < n; i += T) z[i] += y[i];
             }
@@ -319,8 +382,7 @@ __global__ void __launch_bounds__(T) k_batch_pcg(BatchArgs a) {
                     for (int kk = S.rp[i]; kk < S.rp[i + 1]; kk++) f += g32[kk] * (float)(pi - p[S.ci[kk]]);
                     s = (double)f;
                 } else {
-                    s = 0;
-                    for (int kk = S.rp[i]; kk < S.rp[i + 1]; kk++) s += S.val[kk] * p[S.ci[kk]];
+                    s = row_dot(S, i, [&](int c) { return p[c]; });
                 }
                 qv[i] = s;
                 pq_l += p[i] * s;
@@ -419,26 +481,6 @@ __device__ __forceinline__ void cl_sum2(double a, double b, double* sm, double* 
     for (int r = 0; r < kClCtas; r++) {
         ra += __ldcg(&slot[2 * r]);
         rb += __ldcg(&slot[2 * r + 1]);
-    }
-}
-
-// z = T^-1 r over this CTA's chains (see apply_chains).
-template <typename PT>
-__device__ void apply_chains_range(const BatchSys& S, int c_lo, int c_hi, const PT* lf, const PT* ip, const double* r, double* z) {
-    for (int c = c_lo + threadIdx.x; c < c_hi; c += blockDim.x) {
-        const int s0 = S.cs[c], m = S.cl[c];
-        PT y = (PT)r[s0];
-        z[s0] = (double)y;
-        for (int k = 1; k < m; k++) {
-            y = (PT)r[s0 + k] - lf[s0 + k] * y;
-            z[s0 + k] = (double)y;
-        }
-        PT zn = (PT)z[s0 + m - 1] * ip[s0 + m - 1];
-        z[s0 + m - 1] = (double)zn;
-        for (int k = m - 2; k >= 0; k--) {
-            zn = (PT)z[s0 + k] * ip[s0 + k] - lf[s0 + k + 1] * zn;
-            z[s0 + k] = (double)zn;
-        }
     }
 }
 
@@ -543,9 +585,9 @@ __global__ void __launch_bounds__(kClThreads) k_batch_pcg_cl(BatchArgs a) {
             if (PK == 0) {
                 for (int i = r_lo + threadIdx.x; i < r_hi; i += T) z[i] = (double)((PT)r[i] * ip[i]);
             } else if (PK == 2) {
-                apply_chains_range<PT>(S, c_lo, c_hi, lf, ip, r, z);
+                apply_chains<PT>(S, c_lo, c_hi, lf, ip, r, z);
             } else {
-                apply_chains_range<PT>(S, c_lo, c_hi, lf, ip, r, y);
+                apply_chains<PT>(S, c_lo, c_hi, lf, ip, r, y);
                 cluster_sync();  // the coupling term reads y of other CTAs' rows
                 for (int i = r_lo + threadIdx.x; i < r_hi; i += T) {
                     if (MX) {
@@ -556,16 +598,11 @@ __global__ void __launch_bounds__(kClThreads) k_batch_pcg_cl(BatchArgs a) {
                         }
                         u[i] = (double)f;
                     } else {
-                        double sacc = 0;
-                        for (int kk = S.rp[i]; kk < S.rp[i + 1]; kk++) {
-                            const float w = S.ew[kk];
-                            if (w != 0.0f) sacc += (double)w * (-S.val[kk]) * __ldcg(&y[S.ci[kk]]);
-                        }
-                        u[i] = sacc;
+                        u[i] = row_coupling(S, i, [&](int c) { return __ldcg(&y[c]); });
                     }
                 }
                 __syncthreads();
-                apply_chains_range<PT>(S, c_lo, c_hi, lf, ip, u, z);
+                apply_chains<PT>(S, c_lo, c_hi, lf, ip, u, z);
                 __syncthreads();
                 for (int i = r_lo + threadIdx.x; i < r_hi; i += T) z[i] += y[i];
             }
@@ -588,8 +625,7 @@ __global__ void __launch_bounds__(kClThreads) k_batch_pcg_cl(BatchArgs a) {
                     for (int kk = S.rp[i]; kk < S.rp[i + 1]; kk++) f += g32[kk] * (float)(pi - __ldcg(&p[S.ci[kk]]));
                     sq = (double)f;
                 } else {
-                    sq = 0;
-                    for (int kk = S.rp[i]; kk < S.rp[i + 1]; kk++) sq += S.val[kk] * __ldcg(&p[S.ci[kk]]);
+                    sq = row_dot(S, i, [&](int c) { return __ldcg(&p[c]); });
                 }
                 qv[i] = sq;
                 pq_l += p[i] * sq;
