@@ -943,10 +943,10 @@ __global__ void __launch_bounds__(CL ? kMgClusterThreads : kMgThreads) k_mg_pcg(
     mg_pcg_body<CL>(a, blockIdx.x, gridDim.x);
 }
 
-// Batched solves: every 16-CTA cluster takes the next system of the queue and
+// Batched solves: every cluster (of `ctas` CTAs) takes the next system of the queue and
 // runs the MG-PCG on it; `slots` passes the index from cluster rank 0 to the others.
-__global__ void __launch_bounds__(kMgClusterThreads) k_mg_batch(const MgArgs* __restrict__ all, int count, int* queue, int* slots) {
-    const int cl = blockIdx.x / kMgClusterCtas, rank = blockIdx.x % kMgClusterCtas;
+__global__ void __launch_bounds__(kMgClusterThreads) k_mg_batch(const MgArgs* __restrict__ all, int count, int ctas, int* queue, int* slots) {
+    const int cl = blockIdx.x / ctas, rank = blockIdx.x % ctas;
     while (true) {
         if (rank == 0 && threadIdx.x == 0) slots[cl] = atomicAdd(queue, 1);
         asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
@@ -956,7 +956,7 @@ __global__ void __launch_bounds__(kMgClusterThreads) k_mg_batch(const MgArgs* __
         asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
         if (s >= count) return;
         const MgArgs a = all[s];
-        mg_pcg_body<true>(a, rank, kMgClusterCtas);
+        mg_pcg_body<true>(a, rank, ctas);
     }
 }
 
@@ -2596,7 +2596,7 @@ struct MgBatch {
     DBuf<MgArgs> args;
     DBuf<int> queue, slots;
     DBuf<double> stats;
-    int count = 0, nclusters = 0;
+    int count = 0, nclusters = 0, ctas = kMgClusterCtas;  // ctas: CTAs per cluster
     double tol = 0;
     ~MgBatch() {
         for (auto* w : works) delete w;
@@ -2623,6 +2623,31 @@ MgBatch* mg_batch_build(const std::vector<MgBatchInput>& in, double tol, long lo
         B->count = (int)in.size();
         B->tol = tol;
         B->stats.ensure(4 * in.size() + 4);
+        auto resident = [](int ctas) {  // clusters of `ctas` CTAs that fit at once
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute attr[1];
+            cfg.gridDim = dim3(ctas);
+            cfg.blockDim = dim3(kMgClusterThreads);
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = ctas;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int n = 0;
+            CICY_CUDA(cudaOccupancyMaxActiveClusters(&n, (void*)k_mg_batch, &cfg));
+            return n;
+        };
+        // Smaller clusters once the batch does not fit in one round (up to two rounds of eight CTAs):
+        // 7, 15 and 33 clusters of 16, 8 and 4 CTAs are resident.  Batch times in ms for 16 / 8 / 4 CTAs
+        // (sides 2 - 3.5 um, 1.5 %): 6 systems 2.5 / 3.2 / 4.5, 9 (from 2.5 um) 3.5 / 3.1 / 4.5, 16
+        // 4.1 / 3.4 / 4.9; sides 2 - 3 um: 24 systems 5.0 / 3.3 / 4.2, 48 9.6 / 5.5 / 4.3.
+        int nclusters = resident(B->ctas);
+        if (B->count > nclusters) {
+            nclusters = resident(B->ctas = 8);
+            if (B->count > 2 * nclusters) nclusters = resident(B->ctas = 4);
+        }
+        if (nclusters < 1) throw Fail{CICY_E_DEVICE, "batched multigrid: no cluster fits"};
         std::vector<MgArgs> host(in.size());
         for (size_t k = 0; k < in.size(); k++) {
             const MgBatchInput& x = in[k];
@@ -2648,9 +2673,9 @@ MgBatch* mg_batch_build(const std::vector<MgBatchInput>& in, double tol, long lo
             w->r.ensure(x.n); w->z.ensure(x.n); w->p.ensure(x.n); w->q.ensure(x.n);
             g.z0.ensure(x.n);
             g.wtmp.ensure(x.n);
-            w->cta_row.ensure(kMgClusterCtas + 1);
-            launch_cta_rows(kMgClusterCtas, x.n, w->is_start.get(), w->cta_row.get(), s);
-            w->part.ensure(4 * kMgClusterCtas + 8);
+            w->cta_row.ensure(B->ctas + 1);
+            launch_cta_rows(B->ctas, x.n, w->is_start.get(), w->cta_row.get(), s);
+            w->part.ensure(4 * B->ctas + 8);
             MgArgs a{};
             a.n = x.n;
             a.rp = x.rp; a.ci = x.ci; a.val = x.val; a.b = x.b; a.x = x.x; a.x0 = x.x0;
@@ -2662,7 +2687,7 @@ MgBatch* mg_batch_build(const std::vector<MgBatchInput>& in, double tol, long lo
             a.cinv = g.dense ? g.cinv.get() : nullptr;
             a.omega0 = kOmega0;
             a.partA = w->part.get();
-            a.partB = w->part.get() + 2 * kMgClusterCtas;
+            a.partB = w->part.get() + 2 * B->ctas;
             a.stats = B->stats.get() + 4 * k;
             a.bar = nullptr;
             a.spin_limit = kSpinLimit;
@@ -2673,23 +2698,11 @@ MgBatch* mg_batch_build(const std::vector<MgBatchInput>& in, double tol, long lo
             a.cap_b = 1;
             host[k] = a;
         }
+        // largest first: a cluster that takes a large system last would finish long after the others
+        std::stable_sort(host.begin(), host.end(), [](const MgArgs& a, const MgArgs& b) { return a.n > b.n; });
         B->args.ensure(in.size());
         CICY_CUDA(cudaMemcpyAsync(B->args.get(), host.data(), sizeof(MgArgs) * in.size(), cudaMemcpyHostToDevice, s));
         B->queue.ensure(1);
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        cfg.gridDim = dim3(kMgClusterCtas);
-        cfg.blockDim = dim3(kMgClusterThreads);
-        cfg.stream = s;
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = kMgClusterCtas;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int nclusters = 0;
-        CICY_CUDA(cudaOccupancyMaxActiveClusters(&nclusters, (void*)k_mg_batch, &cfg));
-        if (nclusters < 1) throw Fail{CICY_E_DEVICE, "batched multigrid: no 16-CTA cluster fits"};
         B->nclusters = std::min(nclusters, B->count);
         B->slots.ensure(B->nclusters + 1);
         CICY_CUDA(cudaStreamSynchronize(s));
@@ -2705,16 +2718,16 @@ void mg_batch_enqueue(MgBatch* B, cudaStream_t s) {
     CICY_CUDA(cudaMemsetAsync(B->queue.get(), 0, sizeof(int), s));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
-    cfg.gridDim = dim3(kMgClusterCtas * B->nclusters);
+    cfg.gridDim = dim3(B->ctas * B->nclusters);
     cfg.blockDim = dim3(kMgClusterThreads);
     cfg.stream = s;
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kMgClusterCtas;
+    attr[0].val.clusterDim.x = B->ctas;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    CICY_CUDA(cudaLaunchKernelEx(&cfg, k_mg_batch, (const MgArgs*)B->args.get(), B->count, B->queue.get(), B->slots.get()));
+    CICY_CUDA(cudaLaunchKernelEx(&cfg, k_mg_batch, (const MgArgs*)B->args.get(), B->count, B->ctas, B->queue.get(), B->slots.get()));
 }
 
 void mg_batch_stats(MgBatch* B, std::vector<double>& stats, cudaStream_t s) {
