@@ -902,6 +902,7 @@ void run_hybrid_electrical(Ctx& c, const cicy_hybrid_state& h, const cicy_params
                 H.cmj_len[j] = compact_list(c, mxl, nmj, H.alive, H.alive_scan, H.tmp_list);
             }
             if (ngj > 0) {
+                H.alive.ensure(ngj);  // (sized for the mixed junctions so far)
                 CICY_CUDA(cudaMemcpyAsync(H.alive.get(), H.gj_alive.get(), sizeof(int32_t) * ngj, cudaMemcpyDeviceToDevice, s));
                 H.cgj_len[j] = compact_list(c, gjl, ngj, H.alive, H.alive_scan, H.tmp_list);
             }
