@@ -123,7 +123,7 @@ typedef struct {
     int32_t max_iter_factor;  /* max iterations = factor * nodes (upstream 300, Direct_Electrifying.cpp:1559) */
     int32_t flags;            /* bit 0: never use the cluster-resident solver (grid-wide persistent kernel only);
                                  bit 1: multigrid above 20,000 rows keeps its first pairwise prolongator piecewise
-                                 constant (no smoothing) */
+                                 constant (else it is smoothed on sparse chain graphs) */
 } cicy_solver_opts;
 
 #define CICY_SOLVER_NO_CLUSTER 1
@@ -139,7 +139,7 @@ typedef struct {
     int64_t iterations;       /* CG iterations */
     double rel_residual;      /* FP64 |b - A x| / |b| after the solve */
     double seconds;           /* device time of the solve (CUDA events) */
-    int32_t kernel;           /* 0: grid-wide persistent PCG, 1: cluster-resident PCG, 2: multigrid PCG */
+    int32_t kernel;           /* 0: grid-wide persistent PCG, 1: PCG resident in one CTA or cluster, 2: multigrid PCG */
     int32_t restarts;         /* FP64 true-residual restarts taken */
     int32_t levels;           /* multigrid levels (0 for one-level preconditioners) */
     int32_t fallback;         /* 1: the learned preconditioner did not reach the tolerance; Jacobi-PCG solved it */
@@ -401,7 +401,7 @@ cicy_status cicy_spmv_csr(int32_t n, const int32_t* row_ptr, const int32_t* col_
  *      the next system of a largest-first queue and runs preconditioned CG on
  *      it alone, with the preconditioner and precision of cicy_batch_set_solver
  *      (the largest systems optionally on 16-CTA clusters, cicy_batch_set_split);
- *   1  one 16-CTA cluster per system running the chain-aggregation multigrid
+ *   1  one cluster per system (16, 8 or 4 CTAs by the number of systems) running the chain-aggregation multigrid
  *      PCG (after cicy_batch_enable_multigrid; FP64);
  *   2  one system after another through the per-network grid-wide persistent
  *      PCG (the path cicy_electrical_analysis uses), same preconditioner and
