@@ -53,7 +53,12 @@ namespace {
 constexpr int kMgThreads = 256;
 constexpr int kMgClusterThreads = 1024;
 constexpr int kMgClusterCtas = 16;            // non-portable cluster size
-constexpr int kMgClusterMaxRows = 20000;  // above this the grid-wide variant (more threads per row) is faster on B200
+// Largest system for the one-cluster kernel.  The shared-memory-resident grid kernel, with its fused
+// rows, smoothed prolongator and larger dense coarsest, is faster as soon as the cluster's hierarchy
+// has a third level: solve in ms, cluster / grid, 333 rows 0.33 / 0.35, 409 0.29 / 0.29, 448 0.34 / 0.36,
+// 488 0.49 / 0.33, 1,552 0.90 / 0.40, 3,992 1.05 / 0.54, 10.2k 1.47 / 0.72, 18.5k 2.44 / 1.03; whole calls
+// of 1,600 - 6,400 CNTs 3.7 - 7.3 against 2.7 - 4.9.
+constexpr int kMgClusterMaxRows = 450;
 constexpr int kMgMaxRestarts = 24;
 constexpr double kOmega0 = 0.95;
 
@@ -2577,7 +2582,7 @@ namespace cicy {
 
 // ---------------------------------------------------------------------------
 // Batched MG solves (used by batch.cu): per-system hierarchies built once, all
-// systems solved by k_mg_batch, one 16-CTA cluster per system at a time.
+// systems solved by k_mg_batch, one cluster per system at a time.
 namespace {
 __global__ void k_diag_of(int n, const int32_t* __restrict__ rp, const int32_t* __restrict__ ci, const double* __restrict__ v,
                           double* __restrict__ d) {

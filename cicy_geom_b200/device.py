@@ -71,7 +71,7 @@ class Context:
                    smoothed: bool = True):
         """precision: 0 FP64, 1 mixed; preconditioner: 0 Jacobi (upstream), 1 learned, 2 chain blocks, 3 multigrid;
         cluster: allow the cluster-resident solver for systems that fit in shared memory; smoothed: the multigrid
-        hierarchy above 20,000 rows smooths its first pairwise prolongator (CICY_SOLVER_NO_SMOOTHED when false)."""
+        hierarchy above 450 rows smooths, on sparse chain graphs, its first pairwise prolongator (CICY_SOLVER_NO_SMOOTHED when false)."""
         flags = (0 if cluster else _abi.SOLVER_NO_CLUSTER) | (0 if smoothed else _abi.SOLVER_NO_SMOOTHED)
         o = _abi.SolverOpts(precision, preconditioner, max_iter_factor, flags)
         self._check(lib().cicy_ctx_set_solver(self._h, C.byref(o)), "cicy_ctx_set_solver")

@@ -122,7 +122,7 @@ typedef struct {
     int32_t preconditioner;   /* cicy_preconditioner */
     int32_t max_iter_factor;  /* max iterations = factor * nodes (upstream 300, Direct_Electrifying.cpp:1559) */
     int32_t flags;            /* bit 0: never use the cluster-resident solver (grid-wide persistent kernel only);
-                                 bit 1: multigrid above 20,000 rows keeps its first pairwise prolongator piecewise
+                                 bit 1: multigrid above 450 rows keeps its first pairwise prolongator piecewise
                                  constant (else it is smoothed on sparse chain graphs) */
 } cicy_solver_opts;
 

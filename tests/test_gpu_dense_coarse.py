@@ -24,3 +24,20 @@ def test_ladder_multigrid(cuda_ok, rungs):
     assert [s[0] for s in solves[0]] == [s[0] for s in solves[3]]
     assert all(s[2] <= 1e-10 for s in solves[0] + solves[3]) and solves[3][0][1] <= 150
     assert 0 < r[0] < 1e18 and abs(r[3] - r[0]) <= 1e-9 * r[0]
+
+
+@pytest.mark.parametrize("rungs", [70, 74, 75, 80])
+def test_around_the_one_cluster_limit(cuda_ok, rungs):
+    """Unit passes of 422 to 482 rows: the one-cluster kernel up to 450, the grid kernel above."""
+    cfg, net = ladder(rungs)
+    r = {}
+    for pre, cluster in ((0, False), (3, True), (3, False)):
+        with Context(0) as ctx:
+            ctx.set_solver(preconditioner=pre, cluster=cluster)
+            ctx.upload(net)
+            res = ctx.network_to_conductance(cfg.params())
+            assert all(s.rel_residual <= 1e-10 for s in res.solves[:res.n_solves])
+            assert pre == 0 or res.solves[0].kernel == 2
+            r[pre, cluster] = res.resistances[0]
+    for k in ((3, True), (3, False)):
+        assert 0 < r[0, False] < 1e18 and abs(r[k] - r[0, False]) <= 1e-9 * r[0, False]
