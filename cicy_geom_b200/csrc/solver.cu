@@ -440,6 +440,8 @@ __global__ void __launch_bounds__(kCgThreads) k_pcg(PcgArgs a) {
             rz_l = 0;
             if (!precond_all<PRE, MIXED>(a, r_lo, r_hi, rr_l, rz_l)) return;
             block_reduce2(rr_l, rz_l, sm, s0, s1);
+            // every CTA has read the partials that are rewritten here (the SPAI form's own barrier sees to it)
+            if (PRE != PRECOND_KIND_SPAI && !grid_sync(a.bar, nb, a.err)) return;
             if (threadIdx.x == 0) { a.partA[2 * blockIdx.x] = s0; a.partA[2 * blockIdx.x + 1] = s1; }
             if (!grid_sync(a.bar, nb, a.err)) return;
             sum_partials(a.partA, 2, nb, sm, rr_new, rz);

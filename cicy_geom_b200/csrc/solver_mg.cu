@@ -436,7 +436,7 @@ struct MgArgs {
     const MgLevel* lv;     // device descriptors
     const double* cinv;    // dense inverse of the coarsest level, or nullptr
     double omega0;
-    double* partA;
+    double* partA;  // 4 x CTAs: r.r, p.q, then partB (r.z), r.r's second bank
     double* partB;
     double* stats;
     unsigned long long* bar;  // monotonic arrival counter (zeroed before the launch)
@@ -753,6 +753,13 @@ __device__ __forceinline__ double block_apply(const MgArgs& a, const double* __r
     return s;
 }
 
+// Partials of r.r.  A residual replacement sums r.r twice with no barrier between the reads of the
+// first sum's partials and the writes of the second's, so the two take different banks; a bank is
+// written again only after the barriers of an iteration.
+__device__ __forceinline__ double* residual_bank(const MgArgs& a, int restarts, int nctas) {
+    return a.partA + (restarts & 1 ? 3 * nctas : 0);
+}
+
 // One MG-PCG solve by `nctas` CTAs (this is CTA `cta` of them).
 template <bool CL>
 __device__ void mg_pcg_body(const MgArgs& a, int cta, int nctas) {
@@ -802,9 +809,10 @@ __device__ void mg_pcg_body(const MgArgs& a, int cta, int nctas) {
         }
         double s0;
         mg_reduce1(rr_l, sm, s0);
-        if (threadIdx.x == 0) a.partA[cta] = s0;
+        double* const part = residual_bank(a, restarts, nb);
+        if (threadIdx.x == 0) part[cta] = s0;
         if (!sync_all<CL>(a.bar, target, a.err, &s_ok, a.spin_limit)) return;
-        rr = mg_sum_partials(a.partA, nb, sm);
+        rr = mg_sum_partials(part, nb, sm);
         if (k == 0 && !recursive && restarts == 0) R0 = a.tol * (a.cap_b ? fmin(sqrt(rr), bnorm) : sqrt(rr));
         if (k > 0 && sqrt(rr) <= R0) {
             if (!recursive || restarts >= a.max_restarts) break;
@@ -1356,7 +1364,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mg_pcg_sm(MgArgs a, MgSmArgs 
             const double ri = L.r[li];
             rr_l += ri * ri;
         }
-        if (!sm_sum(a, a.partA, target, rr_l, sm, &s_ok, rr)) return;
+        if (!sm_sum(a, residual_bank(a, restarts, nb), target, rr_l, sm, &s_ok, rr)) return;
         if (k == 0 && !recursive && restarts == 0) R0 = a.tol * sqrt(rr);
         if (k > 0 && sqrt(rr) <= R0) {
             if (!recursive || restarts >= a.max_restarts) break;
