@@ -1188,7 +1188,9 @@ __device__ __forceinline__ void chain_solve(const double* r, const double* lf, c
     }
 }
 
-constexpr int kSmMaxStages = 16 + 7 * kMgMaxLevels;
+// Copies of one CTA: seven of level 0's rows, nine of each level between it and the coarsest (four of
+// its restriction rows, five of its prolongation rows), five of level 0's matrix, x and the dense inverse.
+constexpr int kSmMaxStages = 7 + 9 * (kMgMaxLevels - 2) + 5;
 
 __global__ void __launch_bounds__(kSmThreads, 1) k_mg_pcg_sm(MgArgs a, MgSmArgs sa) {
     extern __shared__ __align__(16) unsigned char sm_dyn[];
@@ -1227,17 +1229,25 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mg_pcg_sm(MgArgs a, MgSmArgs 
             used = u + (unsigned int)bytes;
             return sm_dyn + u;
         };
+        // room for a copy of `count` entries of `elem` bytes and its record, or null
+        auto copy = [&](const void* src, int count, int elem, int rebase) -> unsigned char* {
+            unsigned char* m = count > 0 && ns < kSmMaxStages ? take((size_t)elem * count) : nullptr;
+            if (m) st[ns++] = SmStage{m, src, count, elem, rebase};
+            return m;
+        };
         // dst: the staged copy, or `src` itself when it does not fit
         auto stage_i = [&](const int32_t*& dst, const int32_t* src, int count, int rebase) {
-            unsigned char* m = count > 0 ? take(4 * (size_t)count) : nullptr;
+            unsigned char* m = copy(src, count, 4, rebase);
             dst = m ? reinterpret_cast<const int32_t*>(m) : src;
-            if (m) st[ns++] = SmStage{m, src, count, 4, rebase};
             return m != nullptr;
         };
         auto stage_d = [&](const double*& dst, const double* src, int count) {
-            unsigned char* m = count > 0 ? take(8 * (size_t)count) : nullptr;
+            unsigned char* m = copy(src, count, 8, 0);
             dst = m ? reinterpret_cast<const double*>(m) : src;
-            if (m) st[ns++] = SmStage{m, src, count, 8, 0};
+        };
+        auto stage_v = [&](double* src, int count) {
+            unsigned char* m = copy(src, count, 8, 0);
+            return m ? reinterpret_cast<double*>(m) : src;
         };
         auto vec = [&](double* src, int count) {
             unsigned char* m = count > 0 ? take(8 * (size_t)count) : nullptr;
@@ -1251,8 +1261,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mg_pcg_sm(MgArgs a, MgSmArgs 
         P.prod = reinterpret_cast<double*>(take(8 * kSmProd));
         P.aux = reinterpret_cast<double*>(take(16 * kSmAux));
         // what every phase of level 0 reads: residual, smoothed vectors, chain factors and ranges
-        L.r = vec(a.r + L.lo, nr);
-        if (L.r != a.r + L.lo) st[ns++] = SmStage{L.r, a.r + L.lo, nr, 8, 0};
+        L.r = stage_v(a.r + L.lo, nr);
         L.z0 = vec(a.z0 + L.lo, nr);
         L.w = vec(a.w + L.lo, nr);
         L.z = vec(a.z + L.lo, nr);
@@ -1289,8 +1298,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) k_mg_pcg_sm(MgArgs a, MgSmArgs 
         stage_i(L.cagg, G0.cagg + ent0, ent, 0);
         L.q = vec(a.q + L.lo, nr);
         L.p = vec(a.p + L.lo, nr);
-        L.x = vec(a.x + L.lo, nr);
-        if (L.x != a.x + L.lo) st[ns++] = SmStage{L.x, a.x + L.lo, nr, 8, 0};
+        L.x = stage_v(a.x + L.lo, nr);
         L.b = a.b + L.lo;
         const int nC = lv[C].n;
         P.clo = (int)((long long)nC * cta / nb);
