@@ -591,14 +591,20 @@ __global__ void __launch_bounds__(kCtaThreads, 1) k_pcg_cta(CtaArgs a) {
     }
 }
 
-// Launches `solve` between two events, waits and reads its statistics.
+// Launches `solve` between two events, waits and reads its statistics.  False, with x untouched, when
+// the launch is refused (a device or partition without room for the CTA or cluster).
 template <class F>
-void timed_solve(SolverWork& w, cudaStream_t s, int64_t& launches, PcgStats& st, F solve) {
+bool timed_solve(SolverWork& w, cudaStream_t s, int64_t& launches, PcgStats& st, F solve) {
     cudaEvent_t e0, e1;
     CICY_CUDA(cudaEventCreate(&e0));
     CICY_CUDA(cudaEventCreate(&e1));
     CICY_CUDA(cudaEventRecord(e0, s));
-    solve();
+    if (solve() != cudaSuccess) {
+        cudaGetLastError();
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        return false;
+    }
     CICY_CUDA(cudaEventRecord(e1, s));
     launches++;
     double hs[4];
@@ -612,11 +618,14 @@ void timed_solve(SolverWork& w, cudaStream_t s, int64_t& launches, PcgStats& st,
     st.restarts = (int)hs[3];
     st.seconds = ms * 1e-3;
     st.cluster = true;
+    return true;
 }
 
 template <int R, int C>
-void launch_pcg_cta(const CtaArgs& a, cudaStream_t s, PcgStats& st) {
-    CICY_CUDA(cudaFuncSetAttribute(k_pcg_cta<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(double) * kCtaThreads * R * C));
+cudaError_t launch_pcg_cta(const CtaArgs& a, cudaStream_t s, PcgStats& st) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_pcg_cta<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(double) * kCtaThreads * R * C);
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(C);
     cfg.blockDim = dim3(kCtaThreads);
@@ -629,14 +638,14 @@ void launch_pcg_cta(const CtaArgs& a, cudaStream_t s, PcgStats& st) {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = C > 1 ? 1 : 0;
-    CICY_CUDA(cudaLaunchKernelEx(&cfg, k_pcg_cta<R, C>, a));
     st.ctas = C;
+    return cudaLaunchKernelEx(&cfg, k_pcg_cta<R, C>, a);
 }
 
-void pcg_solve_cta(SolverWork& w, const SolverSystem& sys, double tol, long long max_iter, cudaStream_t s, int64_t& launches, PcgStats& st) {
+bool pcg_solve_cta(SolverWork& w, const SolverSystem& sys, double tol, long long max_iter, cudaStream_t s, int64_t& launches, PcgStats& st) {
     w.stats.ensure(4);
     const CtaArgs a{sys.n, sys.rp, sys.ci, sys.val, sys.b, sys.diag, sys.x, tol, max_iter, 24, w.stats.get()};
-    timed_solve(w, s, launches, st, [&] {
+    return timed_solve(w, s, launches, st, [&] {
         switch (ceil_div(sys.n, kCtaThreads)) {
             case 1: return launch_pcg_cta<1, 1>(a, s, st);
             case 2: return launch_pcg_cta<2, 1>(a, s, st);
@@ -664,10 +673,7 @@ bool pcg_solve_cluster(SolverWork& w, const SolverSystem& sys, bool block_precon
     st = PcgStats{};
     if (n <= 0) return true;
     if (n < 4 * C || n >= (1 << 16) * C / 2) return false;
-    if (!block_precond && n <= kCtaMax) {
-        pcg_solve_cta(w, sys, tol, max_iter, s, launches, st);
-        return true;
-    }
+    if (!block_precond && n <= kCtaMax && pcg_solve_cta(w, sys, tol, max_iter, s, launches, st)) return true;
     static int attr_state = 0;  // 0 unknown, 1 ok, -1 unsupported
     if (attr_state == 0) {
         cudaError_t e1 = cudaFuncSetAttribute(k_pcg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -777,9 +783,8 @@ bool pcg_solve_cluster(SolverWork& w, const SolverSystem& sys, bool block_precon
         return false;
     }
     tr.mark("cluster.occupancy");
-    timed_solve(w, s, launches, st, [&] { CICY_CUDA(cudaLaunchKernelEx(&cfg, k_pcg_cluster, a)); });
     st.ctas = C;
-    return true;
+    return timed_solve(w, s, launches, st, [&] { return cudaLaunchKernelEx(&cfg, k_pcg_cluster, a); });
 }
 
 }  // namespace cicy
