@@ -735,10 +735,10 @@ void* cl_kernel_for(int pk, bool mx) {
     return mx ? cl_kernel<2, true>() : cl_kernel<2, false>();
 }
 
-// 16-CTA clusters are a non-portable size: opt every instantiation in once.
+// 16-CTA clusters are a non-portable size: opt every instantiation in once per batch (`clusters`
+// negative before; the opt-in belongs to the device).
 // Returns the number of clusters of one instantiation that fit at once (0: none).
-int cl_setup(int sms) {
-    static int clusters = -1;
+int cl_setup(int sms, int& clusters) {
     if (clusters >= 0) return clusters;
     clusters = 0;
     bool ok = true;
@@ -812,6 +812,7 @@ struct cicy_batch {
     int split = 0;   // method 0: systems of at least this many rows run on 16-CTA clusters (0: none)
     int n_split = 0; // how many systems that is (the first ones of the largest-first order)
     int nclusters = 0;
+    int cl_resident = -1;  // 16-CTA clusters that fit at once (-1: not asked yet)
     bool have_weights = false;
     cicy::MgBatch* mg = nullptr;
     int64_t launches = 0;
@@ -1129,7 +1130,7 @@ void apply_split(cicy_batch* b, int rows) {
     if (rows <= 0) return;
     for (const auto& in : b->inputs) b->n_split += in.n >= rows ? 1 : 0;
     if (b->n_split == 0) return;
-    b->nclusters = cicy::cl_setup(b->sms);
+    b->nclusters = cicy::cl_setup(b->sms, b->cl_resident);
     if (b->nclusters < 1) throw cicy::Fail{CICY_E_DEVICE, "cicy_batch_set_split: 16-CTA clusters are not available"};
     b->queue2.ensure(1);
     b->slots.ensure(b->nclusters);
@@ -1198,7 +1199,7 @@ cicy_status cicy_batch_autotune(cicy_batch* b, int32_t* method, int32_t* threads
         b->ctas_per_sm = bc;
         // method 0: the largest systems on 16-CTA clusters, at a few size thresholds
         int bs = 0;
-        if (bm == 0 && cicy::cl_setup(b->sms) > 0) {
+        if (bm == 0 && cicy::cl_setup(b->sms, b->cl_resident) > 0) {
             for (int rows : {131072, 32768, 8192}) {
                 apply_split(b, rows);
                 if (b->n_split == 0) continue;

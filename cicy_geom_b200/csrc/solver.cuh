@@ -124,6 +124,9 @@ struct MgWork {
     bool fused = false;  // fused rows built (build_mg_hierarchy with fused = true)
     bool smooth = true;  // with fused: level 1's prolongator smoothed (coarsen_smoothed)
     DBuf<unsigned char> sec_lv;  // device descriptors of the clustered kernel
+    // kernel attributes belong to a device, as these buffers do: set once for each work object
+    bool gather_attr[2] = {false, false};  // k_gather_rows* with one and two value sets
+    int cl_state = 0, sm_state = 0;        // one-cluster and grid kernel: 0 unknown, 1 ok, -1 unsupported
 };
 
 struct SolverWork {
@@ -138,6 +141,7 @@ struct SolverWork {
     long long spin_limit = kSpinLimit;  // polls of a grid-barrier wait before it gives up (DEV_TIMEOUT)
     MgWork mg;
     DBuf<double> y, u;
+    int cluster_state = 0;  // 16-CTA cluster kernel (solver_cluster.cu): 0 unknown, 1 ok, -1 unsupported
 };
 
 // ---- learned preconditioner (learned.cu) ----

@@ -674,14 +674,13 @@ bool pcg_solve_cluster(SolverWork& w, const SolverSystem& sys, bool block_precon
     if (n <= 0) return true;
     if (n < 4 * C || n >= (1 << 16) * C / 2) return false;
     if (!block_precond && n <= kCtaMax && pcg_solve_cta(w, sys, tol, max_iter, s, launches, st)) return true;
-    static int attr_state = 0;  // 0 unknown, 1 ok, -1 unsupported
-    if (attr_state == 0) {
+    if (w.cluster_state == 0) {
         cudaError_t e1 = cudaFuncSetAttribute(k_pcg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         cudaError_t e2 = cudaFuncSetAttribute(k_pcg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmemMax);
-        attr_state = (e1 == cudaSuccess && e2 == cudaSuccess) ? 1 : -1;
+        w.cluster_state = (e1 == cudaSuccess && e2 == cudaSuccess) ? 1 : -1;
         cudaGetLastError();
     }
-    if (attr_state < 0) return false;
+    if (w.cluster_state < 0) return false;
     TraceSeq tr(s);
     // ---- preconditioner blocks: chain blocks (<= kBlockMax) or single rows (Jacobi)
     w.total.ensure(2);

@@ -2029,16 +2029,15 @@ __global__ void k_pq_fill_sa(int n, int lanes, const int32_t* __restrict__ rp, c
 }
 
 template <bool TWO>
-void launch_gather(int nrows, const RowSrc& S, const RowMat& B, const GatherOut& O, bool global_tier, cudaStream_t s, int64_t& launches) {
+void launch_gather(MgWork& g, int nrows, const RowSrc& S, const RowMat& B, const GatherOut& O, bool global_tier, cudaStream_t s, int64_t& launches) {
     constexpr int kSets = TWO ? 3 : 2;
     constexpr int warp_sm = (int)sizeof(double) * kGrWarps * kGrWarpCap * kSets;
     constexpr int mid_sm = (int)sizeof(double) * kGrMidCap * kSets, big_sm = (int)sizeof(double) * kGrBigCap * kSets;
-    static bool attr = false;
-    if (!attr) {
+    if (!g.gather_attr[TWO]) {
         CICY_CUDA(cudaFuncSetAttribute(k_gather_rows<TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, warp_sm));
         CICY_CUDA(cudaFuncSetAttribute(k_gather_rows_cta<kGrMidThreads, kGrMidCap, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, mid_sm));
         CICY_CUDA(cudaFuncSetAttribute(k_gather_rows_cta<kGrBigThreads, kGrBigCap, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, big_sm));
-        attr = true;
+        g.gather_attr[TWO] = true;
     }
     // grids: the CTAs that are resident at once (4 to 6 of the small, 1 of the large CTAs per SM); lists are shared out by stride
     k_gather_rows<TWO><<<grid_for((long long)nrows * 32, kGrWarps * 32), kGrWarps * 32, warp_sm, s>>>(nrows, S, B, O);
@@ -2086,8 +2085,8 @@ long long gather_product(MgWork& g, int nrows, const RowSrc& S, const RowMat& B,
     w.ulen.ensure(nrows + 1);
     const GatherOut O{w.seg.get(), w.gkey.get(), w.gv.get(), w.gv2.get(), w.ocol.get(), w.ov.get(), two ? w.ov2.get() : nullptr, w.ulen.get(),
                       w.longr.get(), nlist, skip_diag ? 1 : 0, rsv, rs_out, diag_out, l1_out};
-    if (two) launch_gather<true>(nrows, S, B, O, global_tier, s, launches);
-    else launch_gather<false>(nrows, S, B, O, global_tier, s, launches);
+    if (two) launch_gather<true>(g, nrows, S, B, O, global_tier, s, launches);
+    else launch_gather<false>(g, nrows, S, B, O, global_tier, s, launches);
     optr.ensure(nrows + 1);
     exclusive_scan_i32(w.ulen.get(), optr.get(), nrows + 1, nullptr, g.scan_tmp, s, launches);
     ocol.ensure(cap);
@@ -2458,15 +2457,14 @@ void pcg_solve_mg(SolverWork& w, const SolverSystem& sys, double tol, long long 
     launches++;
     // one 16-CTA cluster with hardware barriers when it can be launched, else the
     // grid-wide cooperative launch
-    static int cl_state = 0;  // 0 unknown, 1 ok, -1 unsupported
-    if (cl_state == 0) {
-        cl_state = cudaFuncSetAttribute(k_mg_pcg<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess ? 1 : -1;
+    if (g.cl_state == 0) {
+        g.cl_state = cudaFuncSetAttribute(k_mg_pcg<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess ? 1 : -1;
         cudaGetLastError();
     }
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     bool cluster = false;
-    if (allow_cluster && !g.fused && cl_state > 0 && n <= kMgClusterMaxRows) {
+    if (allow_cluster && !g.fused && g.cl_state > 0 && n <= kMgClusterMaxRows) {
         cfg.gridDim = dim3(kMgClusterCtas);
         cfg.blockDim = dim3(kMgClusterThreads);
         cfg.dynamicSmemBytes = 0;
@@ -2485,13 +2483,12 @@ void pcg_solve_mg(SolverWork& w, const SolverSystem& sys, double tol, long long 
     bool sec = false;
     int nb = kMgClusterCtas;
     if (!cluster && g.fused && g.levels >= 2) {
-        static int sm_state = 0;  // 0 unknown, 1 ok, -1 unsupported
-        if (sm_state == 0) {
-            sm_state = cudaFuncSetAttribute(k_mg_pcg_sm, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmBytes) == cudaSuccess ? 1 : -1;
+        if (g.sm_state == 0) {
+            g.sm_state = cudaFuncSetAttribute(k_mg_pcg_sm, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmBytes) == cudaSuccess ? 1 : -1;
             cudaGetLastError();
         }
         int occ = 0;
-        if (sm_state > 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mg_pcg_sm, kSmThreads, kSmBytes) == cudaSuccess && occ >= 1) {
+        if (g.sm_state > 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mg_pcg_sm, kSmThreads, kSmBytes) == cudaSuccess && occ >= 1) {
             nb = std::max(1, std::min({num_sms, kSmThreads, ceil_div(n, 128)}));
             sec = true;
         }
@@ -2633,12 +2630,10 @@ struct MgBatch {
 };
 
 MgBatch* mg_batch_build(const std::vector<MgBatchInput>& in, double tol, long long iter_factor, cudaStream_t s, int64_t& launches) {
-    static int cl_attr = 0;
-    if (cl_attr == 0) {
-        cl_attr = cudaFuncSetAttribute(k_mg_batch, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess ? 1 : -1;
+    if (cudaFuncSetAttribute(k_mg_batch, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
+        throw Fail{CICY_E_DEVICE, "batched multigrid: 16-CTA clusters are not available"};
     }
-    if (cl_attr < 0) throw Fail{CICY_E_DEVICE, "batched multigrid: 16-CTA clusters are not available"};
     MgBatch* B = new MgBatch;
     try {
         B->count = (int)in.size();
