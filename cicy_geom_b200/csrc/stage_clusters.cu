@@ -757,6 +757,7 @@ void upload_network(Ctx& c, const cicy_network& n) {
         throw Fail{CICY_E_INPUT, "cicy_upload_network: missing arrays"};
     if (n.n_points >= (1LL << 31) - 1) throw Fail{CICY_E_CAPACITY, "cicy_upload_network: 2^31 or more points"};
     cudaStream_t s = c.stream;
+    c.stage = 0;  // no network until the upload is complete
     c.n_points = (int)n.n_points;
     c.n_cnts = n.n_cnts;
     c.n_inside = n.n_inside;
@@ -836,7 +837,7 @@ void run_contact_grid(Ctx& c, const cicy_params& p, bool wait) {
     CICY_TRACE("contact_grid", s);
     const cicy_cuboid& w = c.window;
     // Generate_contact_grid + Adjust_regions_if_needed (Contact_grid.cpp:18-102)
-    GridGeom& g = c.grid;
+    GridGeom g{};
     g.n[0] = std::max(1, (int)(w.len_x / p.gs_min[0]));
     g.n[1] = std::max(1, (int)(w.len_y / p.gs_min[1]));
     g.n[2] = std::max(1, (int)(w.len_z / p.gs_min[2]));
@@ -854,6 +855,8 @@ void run_contact_grid(Ctx& c, const cicy_params& p, bool wait) {
     if (g.total <= 0) throw Fail{CICY_E_INPUT, "Generate_contact_grid: invalid number of subregions"};
     if (g.total >= (1LL << 31) - 2 || g.total >= (1LL << 38)) throw Fail{CICY_E_CAPACITY, "Generate_contact_grid: too many regions"};
     const int R = (int)g.total;
+    c.stage = 1;  // no grid until this one is complete
+    c.grid = g;
     c.region_cnt.ensure(R + 1);
     c.region_ptr.ensure(R + 1);
     c.trav_pt.ensure(std::max(c.n_trav, 1));

@@ -289,6 +289,7 @@ void extract_window_device(Ctx& c, const cicy_window_params& w) {
     if (!window_geom(w, g, win))
         throw Fail{CICY_E_INPUT, std::string(where) + ": only single-window runs (win_max == win_min, cut_num = 0) are supported"};
 
+    c.stage = 0;  // trimmed in place: no network until the trim is complete
     const int nc = c.n_cnts;
     Pts p{c.x.get(), c.y.get(), c.z.get(), c.flag.get()};
     // word 0 of win_cnt: error; the per-CNT arrays follow
@@ -417,6 +418,7 @@ void generate_network_device(Ctx& c, const cicy_gen_params& g) {
         throw Fail{CICY_E_CAPACITY, std::string(where) + ": 2^30 or more points per CNT"};
     cudaStream_t s = c.stream;
     CICY_TRACE("generate_network", s);
+    c.stage = 0;  // no network until this one is complete
     const int nc = g.n_cnts;
     const PhiloxDev rng{(uint32_t)(g.seed & 0xffffffffu), (uint32_t)(g.seed >> 32)};
     c.clen.ensure(std::max(nc, 1));
