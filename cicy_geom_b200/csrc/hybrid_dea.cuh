@@ -228,10 +228,10 @@ __global__ void k_current_max_gnp(int ng, const int32_t* __restrict__ gnps, cons
             for (int k = 0; k < tri_cnt[g]; k++) m = fmax(m, fabs(volt[lmm_g[e[2 * k]]] - volt[lmm_g[e[2 * k + 1]]]));
         } else if (i < ng + ngj) {
             const int idx = gj[i - ng];
-            m = fabs(volt[lmm_g[jg_p1[idx]]] - volt[lmm_g[jg_p2[idx]]]);
+            m = junction_current(volt, lmm_g[jg_p1[idx]], lmm_g[jg_p2[idx]]);
         } else {
             const int idx = mix[i - ng - ngj];
-            m = fabs(volt[lmm[jm_p1[idx]]] - volt[lmm_g[jm_p2[idx]]]);
+            m = junction_current(volt, lmm[jm_p1[idx]], lmm_g[jm_p2[idx]]);
         }
         atomic_max_pos(imax, m);
     }
@@ -258,7 +258,7 @@ __global__ void k_mix_below_zero(int nseg, const int32_t* __restrict__ seg_start
             const int i = (int)order[k];
             const int idx = mix[i];
             const int P1 = jm_p1[idx], c = jm_n1[idx], P2 = jm_p2[idx];
-            const double Ij = fabs(volt[lmm[P1]] - volt[lmm_g[P2]]);
+            const double Ij = junction_current(volt, lmm[P1], lmm_g[P2]);
             const int lo = cur_lo[c], hi = cur_hi[c];
             const bool empty = lo < 0;
             const int q = elem_pos[P1];
@@ -288,7 +288,7 @@ __global__ void k_gj_below_zero(int nj, const int32_t* __restrict__ gj, const in
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nj; i += gridDim.x * blockDim.x) {
         const int idx = gj[i];
         const int P1 = jg_p1[idx], P2 = jg_p2[idx];
-        if (fabs(volt[lmm_g[P1]] - volt[lmm_g[P2]]) - zero_current < kZero) {
+        if (junction_current(volt, lmm_g[P1], lmm_g[P2]) - zero_current < kZero) {
             gj_alive[i] = 0;
             pt_removed[P1] = 1;
             pt_removed[P2] = 1;

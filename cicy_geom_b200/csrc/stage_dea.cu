@@ -471,6 +471,12 @@ __device__ __forceinline__ void atomic_max_pos(unsigned long long* addr, double 
     atomicMax(addr, (unsigned long long)__double_as_longlong(v));  // v >= 0: IEEE order == integer order
 }
 
+// Current of a junction (unit resistors) between nodes a and b.  A junction with a point that has no
+// node (-1) is not in the system and carries none.
+__device__ __forceinline__ double junction_current(const double* __restrict__ volt, int a, int b) {
+    return a < 0 || b < 0 ? 0.0 : fabs(volt[a] - volt[b]);
+}
+
 __global__ void k_current_max(int n, const int32_t* __restrict__ eb, const int32_t* __restrict__ ee, const int32_t* __restrict__ elem,
                               const int32_t* __restrict__ lmm, const double* __restrict__ volt, int nj,
                               const int32_t* __restrict__ jlist, const int32_t* __restrict__ jp1, const int32_t* __restrict__ jp2,
@@ -481,7 +487,7 @@ __global__ void k_current_max(int n, const int32_t* __restrict__ eb, const int32
             for (int k = eb[i]; k < ee[i] - 1; k++) m = fmax(m, fabs(volt[lmm[elem[k]]] - volt[lmm[elem[k + 1]]]));
         } else {
             int j = jlist[i - n];
-            m = fabs(volt[lmm[jp1[j]]] - volt[lmm[jp2[j]]]);
+            m = junction_current(volt, lmm[jp1[j]], lmm[jp2[j]]);
         }
         atomic_max_pos(imax, m);
     }
