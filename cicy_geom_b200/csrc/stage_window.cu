@@ -1,6 +1,6 @@
 // Network construction on the device, before the contact grid:
 //  * the seeded CNT generator (the Philox-4x32-10 streams of the host generator,
-//    one thread per CNT), and
+//    one to 32 threads per CNT), and
 //  * the window-0 extraction of a single-window run: Shells::Generate_shells /
 //    Find_shell (Shells.cpp:21-149) and Cutoff_Wins::Trim_boundary_cnts
 //    (Cutoff_Wins.cpp:82-276), Add_cnt_segment_to_structure (:298-467),
@@ -9,7 +9,7 @@
 //    (:745-769) and Fill_cnts_inside (:803-831), CNT_wires branch.
 //
 // Upstream trims the CNTs of shell 0 one after another.  A CNT's trim reads and
-// writes only its own points, so here one thread replays it per CNT; what is
+// writes only its own points, so here one warp replays it per CNT; what is
 // global in upstream's loop is rebuilt from counts:
 //  * a CNT that leaves and re-enters the window is cut into pieces that take
 //    new indices n_cnts, n_cnts + 1, ... in shell-0 order: the trim marks the
@@ -40,6 +40,15 @@ namespace {
 
 using namespace win;
 
+struct Warp {
+    static constexpr int kThreads = 32;
+    int lane;
+    __device__ bool any(bool b) const { return __any_sync(0xffffffffu, b); }
+    template <class F>
+    __device__ uint32_t bits(F f) const { return __ballot_sync(0xffffffffu, f(lane)); }
+    __device__ void sync() const { __syncwarp(); }
+};
+
 // One warp per CNT: its run and flags checked against the generator's layout, its shell, the
 // in/out bits of its points 32 at a time (coalesced, in parallel); lane 0 walks the bits and cuts
 // the segments.  With one thread per CNT reading its ~100 points one after another the layout
@@ -49,37 +58,9 @@ using namespace win;
 __global__ void k_win_trim(int nc, WinGeom g, Pts p, const int32_t* __restrict__ cstart, const int32_t* __restrict__ clen,
                            const int32_t* __restrict__ expect, int32_t* __restrict__ npieces, int32_t* __restrict__ first,
                            int32_t* __restrict__ slots, int64_t* __restrict__ ev, int32_t* __restrict__ nev, int* __restrict__ err) {
-    const int lane = threadIdx.x & 31;
+    const Warp w{(int)(threadIdx.x & 31)};
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nc; i += (gridDim.x * blockDim.x) >> 5) {
-        const int base = cstart[i], n = clen[i];
-        bool bad = n > 0 && base != expect[i], sh0 = false;
-        for (int k = lane; k < n; k += 32) {
-            bad |= p.flag[base + k] != i;
-            sh0 = sh0 || in_shell0(g, p, base + k);
-        }
-        bad = __any_sync(0xffffffffu, bad);
-        sh0 = __any_sync(0xffffffffu, sh0);
-        TrimOut o;
-        int e = WIN_OK;
-        if (sh0) {
-            TrimWalk w;
-            const int last_loc = where_is(g, p, base + n - 1);
-            __syncwarp();
-            for (int b = 0; b < n; b += 32) {
-                const uint32_t out = __ballot_sync(0xffffffffu, b + lane < n && where_is(g, p, base + b + lane) == L_OUTSIDE);
-                if (lane == 0) w.block(g, p, base, b, out, true, o, slots + (size_t)i * kSlot, ev + (size_t)i * kMaxEv);
-                __syncwarp();
-            }
-            if (lane == 0) e = w.finish(g, p, base, n, last_loc, true, o, slots + (size_t)i * kSlot, ev + (size_t)i * kMaxEv);
-        }
-        if (lane != 0) continue;
-        const bool cut = sh0 && e == WIN_OK, kept = cut && o.segments > 0;
-        npieces[i] = kept ? o.segments - 1 : 0;
-        nev[i] = cut ? o.nev : 0;
-        // a CNT outside shell 0 (or whose trim failed) keeps its run
-        first[2 * i] = cut ? (kept ? base + o.first : 0) : (n ? base : 0);
-        first[2 * i + 1] = cut ? (kept ? o.last - o.first + 1 : 0) : n;
-        if (bad) e = WIN_LAYOUT;
+        const int e = trim_cnt(w, i, g, p, cstart, clen, expect, npieces, first, slots, ev, nev);
         if (e) atomicMax(err, e);
     }
 }

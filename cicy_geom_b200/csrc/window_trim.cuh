@@ -1,5 +1,6 @@
-// Window-0 trimming of a single-window run as host/device code (one call per
-// CNT or per list entry; stage_window.cu launches them as kernels).  Restates
+// Window-0 trimming of a single-window run as host/device code: one call per
+// CNT or per list entry, the first pass by one thread or by a warp per CNT
+// (stage_window.cu launches them as kernels, host builds loop over them).  Restates
 // Shells::Find_shell / Find_minimum_shell (Shells.cpp:120-149) and
 // Cutoff_Wins::Trim_boundary_cnts (Cutoff_Wins.cpp:82-276),
 // Add_cnt_segment_to_structure (:298-467), Substitute_boundary_point (:468-548),
@@ -230,16 +231,34 @@ struct TrimWalk {
     }
 };
 
-__host__ __device__ inline int trim_run(const WinGeom& g, const Pts& p, int base, int n, bool allow_pieces, TrimOut& o, int32_t* slots,
+// The threads that trim one CNT: one thread (the pieces' pass, host builds) or a warp (stage_window.cu).
+// bits(f): bit k is f(k), for 32 k.
+struct OneThread {
+    static constexpr int kThreads = 1;
+    int lane = 0;
+    __host__ __device__ bool any(bool b) const { return b; }
+    template <class F>
+    __host__ __device__ uint32_t bits(F f) const {
+        uint32_t v = 0;
+        for (int k = 0; k < 32; k++) v |= (f(k) ? 1u : 0u) << k;
+        return v;
+    }
+    __host__ __device__ void sync() const {}
+};
+
+// All threads call it; the segments are cut, and the result is returned, by lane 0.
+template <class T>
+__host__ __device__ inline int trim_run(const T& t, const WinGeom& g, const Pts& p, int base, int n, bool allow_pieces, TrimOut& o, int32_t* slots,
                                         int64_t* ev) {
     TrimWalk w;
     const int last_loc = where_is(g, p, base + n - 1);
+    t.sync();
     for (int first = 0; first < n; first += 32) {
-        uint32_t out = 0;
-        for (int k = 0; k < 32 && first + k < n; k++) out |= (uint32_t)(where_is(g, p, base + first + k) == L_OUTSIDE) << k;
-        w.block(g, p, base, first, out, allow_pieces, o, slots, ev);
+        const uint32_t out = t.bits([&](int k) { return first + k < n && where_is(g, p, base + first + k) == L_OUTSIDE; });
+        if (t.lane == 0) w.block(g, p, base, first, out, allow_pieces, o, slots, ev);
+        t.sync();
     }
-    return w.finish(g, p, base, n, last_loc, allow_pieces, o, slots, ev);
+    return t.lane == 0 ? w.finish(g, p, base, n, last_loc, allow_pieces, o, slots, ev) : WIN_OK;
 }
 
 // Window 0 and the shell geometry: Geom_sample::update_observation_window_geometry(0, ...)
@@ -273,34 +292,46 @@ inline bool window_geom(const cicy_window_params& w, WinGeom& g, cicy_cuboid& wi
 
 // ---- per-item bodies of the passes (i: CNT, u: unit = CNT then piece, t: list entry) ----
 
-// CNT i is the i-th run (expect = exclusive scan of the run lengths) and its points carry flag i.
+// CNT i is the i-th run (expect = exclusive scan of the run lengths) ...
+__host__ __device__ inline bool run_in_place(int i, const int32_t* cstart, const int32_t* clen, const int32_t* expect) {
+    return clen[i] == 0 || cstart[i] == expect[i];
+}
+// ... and its points carry flag i.
 __host__ __device__ inline bool layout_ok(int i, const int32_t* cstart, const int32_t* clen, const int32_t* expect, const int32_t* flag) {
-    const int n = clen[i];
-    if (n == 0) return true;
-    bool ok = cstart[i] == expect[i];
-    for (int k = 0; k < n && ok; k++) ok = flag[cstart[i] + k] == i;
+    bool ok = run_in_place(i, cstart, clen, expect);
+    for (int k = 0; k < clen[i] && ok; k++) ok = flag[cstart[i] + k] == i;
     return ok;
 }
 
-// First pass: the trim of an original CNT of shell 0 (Trim_boundary_cnts over shells_cnt[0]).
+// First pass: the layout of CNT i (with `expect`) and the trim of an original CNT of shell 0
+// (Trim_boundary_cnts over shells_cnt[0]).  The result is lane 0's.
+template <class T>
+__host__ __device__ inline int trim_cnt(const T& t, int i, const WinGeom& g, const Pts& p, const int32_t* cstart, const int32_t* clen,
+                                        const int32_t* expect, int32_t* npieces, int32_t* first, int32_t* slots, int64_t* ev, int32_t* nev) {
+    const int base = cstart[i], n = clen[i];
+    bool bad = expect && !run_in_place(i, cstart, clen, expect), sh0 = false;
+    for (int k = t.lane; k < n; k += T::kThreads) {
+        if (expect) bad = bad || p.flag[base + k] != i;
+        sh0 = sh0 || in_shell0(g, p, base + k);
+    }
+    bad = t.any(bad);
+    sh0 = t.any(sh0);
+    TrimOut o;
+    const int e = sh0 ? trim_run(t, g, p, base, n, true, o, slots + (size_t)i * kSlot, ev + (size_t)i * kMaxEv) : (int)WIN_OK;
+    if (t.lane != 0) return WIN_OK;
+    const bool cut = sh0 && e == WIN_OK, kept = cut && o.segments > 0;
+    npieces[i] = kept ? o.segments - 1 : 0;
+    nev[i] = cut ? o.nev : 0;
+    // a CNT outside shell 0 (or whose trim failed) keeps its run
+    first[2 * i] = cut ? (kept ? base + o.first : 0) : (n ? base : 0);
+    first[2 * i + 1] = cut ? (kept ? o.last - o.first + 1 : 0) : n;
+    return bad ? (int)WIN_LAYOUT : e;
+}
+
+// The same by one thread, without the layout check.
 __host__ __device__ inline int trim_cnt(int i, const WinGeom& g, const Pts& p, const int32_t* cstart, const int32_t* clen, int32_t* npieces,
                                         int32_t* first, int32_t* slots, int64_t* ev, int32_t* nev) {
-    const int base = cstart[i], n = clen[i];
-    npieces[i] = 0;
-    nev[i] = 0;
-    first[2 * i] = n ? base : 0;
-    first[2 * i + 1] = n;
-    bool sh0 = false;
-    for (int k = 0; k < n && !sh0; k++) sh0 = in_shell0(g, p, base + k);
-    if (!sh0) return WIN_OK;
-    TrimOut o;
-    const int e = trim_run(g, p, base, n, true, o, slots + (size_t)i * kSlot, ev + (size_t)i * kMaxEv);
-    if (e) return e;
-    nev[i] = o.nev;
-    npieces[i] = o.segments > 0 ? o.segments - 1 : 0;
-    first[2 * i] = o.segments > 0 ? base + o.first : 0;
-    first[2 * i + 1] = o.segments > 0 ? o.last - o.first + 1 : 0;
-    return WIN_OK;
+    return trim_cnt(OneThread{}, i, g, p, cstart, clen, nullptr, npieces, first, slots, ev, nev);
 }
 
 // Second pass: the pieces of CNT i in creation order (upstream's loop reaches them after
@@ -325,7 +356,7 @@ __host__ __device__ inline int trim_pieces(int i, int nc, const WinGeom& g, cons
         if (!sl3[2] || err) continue;
         TrimOut o;
         int64_t evq[kMaxEv];
-        int r = trim_run(g, p, s, e - s + 1, false, o, nullptr, evq);
+        int r = trim_run(OneThread{}, g, p, s, e - s + 1, false, o, nullptr, evq);
         if (!r && o.nev > 2) r = WIN_INTERNAL;
         if (r) {
             err = r;
