@@ -2347,9 +2347,10 @@ void build_mg_hierarchy(SolverWork& w, const SolverSystem& sys, cudaStream_t s, 
         g.cinv.ensure((size_t)Lc.n * Lc.n);
         CICY_CUDA(cudaMemsetAsync(g.cinv.get(), 0, sizeof(double) * Lc.n * Lc.n, s));
         k_dense_coarse<<<grid_for(32LL * Lc.n, 128), 128, 0, s>>>(Lc.n, 32, Lc.rp.get(), Lc.ci.get(), Lc.val.get(), Lc.diag.get(), g.cinv.get());
-        const size_t smem = sizeof(double) * ((size_t)Lc.n * Lc.n + 2 * (size_t)Lc.n * kGjBlock + kGjBlock * (kGjBlock + 1) + kGjBlock);
-        if (smem > 48 * 1024)
-            CICY_CUDA(cudaFuncSetAttribute(k_gauss_jordan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        auto bytes = [](size_t m) { return sizeof(double) * (m * m + 2 * m * kGjBlock + kGjBlock * (kGjBlock + 1) + kGjBlock); };
+        const size_t smem = bytes(Lc.n);
+        // always the limit of the largest level: a context in another thread may set it between this and the launch
+        CICY_CUDA(cudaFuncSetAttribute(k_gauss_jordan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(kMgDenseMax)));
         k_gauss_jordan<<<1, kGjThreads, smem, s>>>(Lc.n, g.cinv.get());
         launches += 2;
         g.dense = true;
