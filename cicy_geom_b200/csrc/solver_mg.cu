@@ -43,6 +43,7 @@
 #include <cmath>
 #include <vector>
 
+#include "batch_shape.h"
 #include "solver.cuh"
 #include "trace.cuh"
 
@@ -2655,16 +2656,14 @@ MgBatch* mg_batch_build(const std::vector<MgBatchInput>& in, double tol, long lo
             CICY_CUDA(cudaOccupancyMaxActiveClusters(&n, (void*)k_mg_batch, &cfg));
             return n;
         };
-        // Smaller clusters once the batch does not fit in one round (up to two rounds of eight CTAs):
-        // 7, 15 and 33 clusters of 16, 8 and 4 CTAs are resident.  Batch times in ms for 16 / 8 / 4 CTAs
-        // (sides 2 - 3.5 um, 1.5 %): 6 systems 2.5 / 3.2 / 4.5, 9 (from 2.5 um) 3.5 / 3.1 / 4.5, 16
-        // 4.1 / 3.4 / 4.9; sides 2 - 3 um: 24 systems 5.0 / 3.3 / 4.2, 48 9.6 / 5.5 / 4.3.
-        int nclusters = resident(B->ctas);
-        if (B->count > nclusters) {
-            nclusters = resident(B->ctas = 8);
-            if (B->count > 2 * nclusters) nclusters = resident(B->ctas = 4);
-        }
-        if (nclusters < 1) throw Fail{CICY_E_DEVICE, "batched multigrid: no cluster fits"};
+        std::vector<int> rows;
+        for (const MgBatchInput& x : in) rows.push_back(x.n);
+        int fits[kMgBatchShapes];
+        for (int k = 0; k < kMgBatchShapes; k++) fits[k] = resident(kMgBatchCtas[k]);
+        const int shape = mg_batch_shape(std::move(rows), fits);
+        if (shape < 0) throw Fail{CICY_E_DEVICE, "batched multigrid: no cluster fits"};
+        B->ctas = kMgBatchCtas[shape];
+        const int nclusters = fits[shape];
         std::vector<MgArgs> host(in.size());
         for (size_t k = 0; k < in.size(); k++) {
             const MgBatchInput& x = in[k];

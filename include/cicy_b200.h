@@ -401,7 +401,7 @@ cicy_status cicy_spmv_csr(int32_t n, const int32_t* row_ptr, const int32_t* col_
  *      the next system of a largest-first queue and runs preconditioned CG on
  *      it alone, with the preconditioner and precision of cicy_batch_set_solver
  *      (the largest systems optionally on 16-CTA clusters, cicy_batch_set_split);
- *   1  one cluster per system (16, 8 or 4 CTAs by the number of systems) running the chain-aggregation multigrid
+ *   1  one cluster per system (16, 8 or 4 CTAs by the number and sizes of the systems) running the chain-aggregation multigrid
  *      PCG (after cicy_batch_enable_multigrid; FP64);
  *   2  one system after another through the per-network grid-wide persistent
  *      PCG (the path cicy_electrical_analysis uses), same preconditioner and
