@@ -671,7 +671,7 @@ def batched_monte_carlo(count, device, reps=3):
             "sample": "cube side U[2,5] um, CNT volume fraction U[0.5%,3%], seeds 3,000,000+k; solve stage only "
                       "(generation, contacts, clusters, assembly and the unit-resistor pass run per network before it); "
                       "learned/Jacobi: one CTA per system, the largest systems on 16-CTA clusters when the autotuner picks it, in one "
-                      "graph launch; multigrid: one 16-CTA cluster per system"}
+                      "graph launch; multigrid: one cluster of 16, 8 or 4 CTAs per system"}
 
 
 def sharded_monte_carlo(count, device, rank, world):

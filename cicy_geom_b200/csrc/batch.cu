@@ -808,7 +808,7 @@ struct cicy_batch {
     double tol = 1e-8;
     long long iter_factor = 300;
     int threads = 512, ctas_per_sm = 2, sms = 148;
-    int method = 0;  // 0: one CTA per system, 1: one 16-CTA cluster per system (multigrid), 2: one system at a time, grid-wide
+    int method = 0;  // 0: one CTA per system, 1: one cluster per system (multigrid), 2: one system at a time, grid-wide
     int split = 0;   // method 0: systems of at least this many rows run on 16-CTA clusters (0: none)
     int n_split = 0; // how many systems that is (the first ones of the largest-first order)
     int nclusters = 0;

@@ -9,7 +9,7 @@
 // Included at the end of stage_dea.cu (same translation unit, built without FMA
 // contraction): the CNT part of every system is stage_dea.cu's solve_dea, which
 // calls the three hooks below for the GNP part, so both kinds of resistors go
-// through one sort-and-reduce assembly in upstream's insertion order.
+// through one assembly by rows in upstream's insertion order.
 //
 // Layout: GNP point lists are a CSR of fixed capacity per GNP with the current
 // length in scount (the backbone keeps points at the front); node numbers of GNP

@@ -99,7 +99,7 @@ struct MgWork {
         const double* val_ptr = nullptr;
         DBuf<int32_t> rp, ci, agg, mptr, midx, cagg, ra_ptr, ra_col;
         DBuf<double> val, diag, l1inv, rs, r, z, zf, ra_val;
-        // fused rows for the clustered solve kernel: restriction into level l+1 (members on
+        // fused rows for the grid solve kernel: restriction into level l+1 (members on
         // r_l, P^T A_l on z_l) and prolongation-smoother rows of level l (A_l on z_l and on P zc)
         DBuf<int32_t> rr_ptr, rr_col, pq_ptr, pq_col;
         DBuf<double> rr_val, pq_val;
@@ -123,7 +123,7 @@ struct MgWork {
     bool dense = false;
     bool fused = false;  // fused rows built (build_mg_hierarchy with fused = true)
     bool smooth = true;  // with fused: level 1's prolongator smoothed (coarsen_smoothed)
-    DBuf<unsigned char> sec_lv;  // device descriptors of the clustered kernel
+    DBuf<unsigned char> sec_lv;  // device descriptors of the grid kernel
     // kernel attributes belong to a device, as these buffers do: set once for each work object
     bool gather_attr[2] = {false, false};  // k_gather_rows* with one and two value sets
     int cl_state = 0, sm_state = 0;        // one-cluster and grid kernel: 0 unknown, 1 ok, -1 unsupported
@@ -200,11 +200,11 @@ bool pcg_solve_cluster(SolverWork& w, const SolverSystem& sys, bool block_precon
 
 // Multigrid hierarchy over the chain blocks of build_block_preconditioner (which
 // must have run on the same system), then the MG-preconditioned CG solve.
-// fused: also build the fused restriction / prolongation rows the clustered grid kernel
+// fused: also build the fused restriction / prolongation rows the grid kernel
 // reads (systems above the single-cluster size).
 void build_mg_hierarchy(SolverWork& w, const SolverSystem& sys, cudaStream_t s, int64_t& launches, bool fused = false, bool smooth = true,
                         int* status = nullptr);
-// Whether pcg_solve_mg takes the clustered grid kernel for a system of n rows (build the
+// Whether pcg_solve_mg takes the grid kernel for a system of n rows (build the
 // hierarchy with fused = this).
 bool mg_fused_path(int n, bool allow_cluster);
 // allow_cluster: one 16-CTA cluster with hardware barriers when it fits, else the grid-wide kernel.

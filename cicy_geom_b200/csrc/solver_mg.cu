@@ -10,7 +10,8 @@
 // it.  The hierarchy:
 //
 //   level 0   the free-node system; smoother: the chain blocks (explicit
-//             tridiagonal inverses), damped by kOmega0 so 2 M^-1 - A stays
+//             tridiagonal inverses in the cluster kernels, LDL^T factors in the
+//             grid kernel), damped by kOmega0 so 2 M^-1 - A stays
 //             positive definite on floating islands (bipartite trees of CNTs
 //             that no prescribed node reaches, where the undamped block smoother
 //             would make the V-cycle singular)
@@ -18,23 +19,29 @@
 //   level l+1 pairwise aggregates of level l: three rounds of handshake
 //             matching on the strongest coupling |a_ij| (ties: smaller j), then
 //             every unmatched row joins the pair of its strongest neighbour
-//   coarsest  <= kMgDenseMax rows: dense inverse (Gauss-Jordan in shared
-//             memory, 1e-8 diagonal regularisation, variables with a vanishing
-//             pivot dropped); otherwise an l1-Jacobi step
+//   coarsest  dense inverse (Gauss-Jordan, 1e-8 diagonal regularisation,
+//             variables with a vanishing pivot dropped) of up to kMgDenseMax rows,
+//             by one CTA in shared memory, for the grid kernel of up to
+//             kMgDenseGridMax, by the grid; otherwise an l1-Jacobi step
 //
-// Coarse operators are Galerkin products P^T A P with piecewise-constant P: one
-// thread per aggregate gathers its members' cross-aggregate couplings, sorts
-// them stably by coarse column and sums each run in order (deterministic, no
-// host synchronisation inside a level).  Their diagonals come from summed row
+// Coarse operators are Galerkin products P^T A P with piecewise-constant P (the
+// grid kernel's first one smoothed, see coarsen_smoothed): a warp or a CTA per
+// aggregate gathers its members' cross-aggregate couplings, sorts them by coarse
+// column and gather position and sums each column's run in that order
+// (deterministic).  The host reads each level's size and entries, and the size of
+// each product of the smoothed level.  Their diagonals come from summed row
 // sums, diag_J = sum_{I in J} rowsum_I - sum_{J' != J} A_JJ', so the large
 // intra-aggregate conductances never cancel in floating point and an aggregate
 // with no outside coupling gets an exact zero row.  Levels >= 1 are smoothed by
 // l1-Jacobi (1 / (|d| + sum |a|)), which makes the symmetric V(1,1)-cycle an SPD
 // preconditioner.
 //
-// The solve is one persistent cooperative launch.  Level-0 rows are split over
-// CTAs at block boundaries (the block smoother only reads rows of its own CTA);
-// coarse levels are spread over all threads.  Per CG iteration the grid barriers
+// The solve is one persistent launch: a 16-CTA cluster (k_mg_pcg<true>) up to
+// kMgClusterMaxRows rows, a cooperative grid with the operators in shared memory
+// (k_mg_pcg_sm) above, clusters of 16, 8 or 4 CTAs in a batch (k_mg_batch).
+// Level-0 rows are split over CTAs at block boundaries (the block smoother only
+// reads rows of its own CTA); coarse levels are spread over all threads or dealt by
+// entries.  Per CG iteration the barriers
 // are: 1 after the pre-smoother and r.r, one per restriction, one after the
 // coarse solve, one per prolongation above level 1, one after the post-smoother
 // and r.z, one after p.q.  The stopping rule, FP64 true-residual replacement and
@@ -58,7 +65,9 @@ constexpr int kMgClusterCtas = 16;            // non-portable cluster size
 // rows, smoothed prolongator and larger dense coarsest, is faster as soon as the cluster's hierarchy
 // has a third level: solve in ms, cluster / grid, 333 rows 0.33 / 0.35, 409 0.29 / 0.29, 448 0.34 / 0.36,
 // 488 0.49 / 0.33, 1,552 0.90 / 0.40, 3,992 1.05 / 0.54, 10.2k 1.47 / 0.72, 18.5k 2.44 / 1.03; whole calls
-// of 1,600 - 6,400 CNTs 3.7 - 7.3 against 2.7 - 4.9.
+// of 1,600 - 6,400 CNTs 3.7 - 7.3 against 2.7 - 4.9.  Several contexts at once gain too, although seven
+// clusters fit at once and the grid takes up to every SM: eight threads with a context each make 491 calls/s
+// with clusters up to 20,000 rows and 790 so on 1,000 CNTs, 240 and 318 on 6,400.
 constexpr int kMgClusterMaxRows = 450;
 constexpr int kMgMaxRestarts = 24;
 constexpr double kOmega0 = 0.95;
@@ -349,7 +358,7 @@ __global__ void k_ra_fill(int nc, int lanes, const int32_t* __restrict__ mptr, c
     }
 }
 
-// Fused restriction rows of level l >= 1 into level l + 1 (clustered kernel): row J holds
+// Fused restriction rows of level l >= 1 into level l + 1 (grid kernel): row J holds
 // the members of aggregate J (column m < n: r_l[m], weight 1), then for each member I its
 // diagonal and couplings (column n + c: z_l[c], weight -a), the rows of P^T A_l, so
 // r_{l+1} = P^T (r_l - A_l z_l) is one gathered dot product.  rr_ptr = mptr + ra_ptr, both
@@ -1544,7 +1553,7 @@ __global__ void k_cagg(const int32_t* __restrict__ nnz, const int32_t* __restric
 }
 
 // ---------------------------------------------------------------------------
-// Smoothed level-1 prolongator (hierarchies of the clustered kernel).
+// Smoothed level-1 prolongator (hierarchies of the grid kernel).
 //
 // Why: with piecewise-constant aggregates below the chain level the V-cycle is weak on
 // a sparse chain graph (smoothing_pays), whose junction conductances span five orders of magnitude.  Smoothing
@@ -2170,7 +2179,7 @@ void coarsen_smoothed(MgWork& g, int nc, cudaStream_t s, int64_t& launches) {
 
 // Galerkin coarse level l+1 from level l and its aggregates (g.L[l].agg, nc of
 // them), plus level l's member lists, restriction rows (l >= 1) and column
-// aggregates.  No host synchronisation: buffers are sized by the fine level's
+// aggregates.  No host synchronisation here: buffers are sized by the fine level's
 // non-zeros, an upper bound of the coarse level's.
 void coarsen(MgWork& g, int l, int nc, cudaStream_t s, int64_t& launches) {
     if ((int)g.L.size() < l + 2) g.L.resize(l + 2);
@@ -2214,7 +2223,7 @@ void coarsen(MgWork& g, int l, int nc, cudaStream_t s, int64_t& launches) {
     G.rp_ptr = G.rp.get();
     G.ci_ptr = G.ci.get();
     G.val_ptr = G.val.get();
-    // restriction rows of level l (l >= 1) and its column aggregates; the clustered kernel
+    // restriction rows of level l (l >= 1) and its column aggregates; the grid kernel
     // (g.fused) reads the fused rows instead of P^T A_l and the coarse column aggregates
     if (l >= 1) {
         exclusive_scan_i32(F.ra_ptr.get(), F.ra_ptr.get(), nc + 1, nullptr, g.scan_tmp, s, launches);
@@ -2323,7 +2332,7 @@ void build_mg_hierarchy(SolverWork& w, const SolverSystem& sys, cudaStream_t s, 
     launches += 2;
     int nc = w.n_blocks;
     int C = 0;
-    // the clustered kernel solves a dense coarsest of up to kMgDenseGridMax rows on all CTAs
+    // the grid kernel solves a dense coarsest of up to kMgDenseGridMax rows on all CTAs
     int dense_cap = kMgDenseMax;
     if (fused) {
         int dev = 0, sms = 0;
@@ -2356,7 +2365,7 @@ void build_mg_hierarchy(SolverWork& w, const SolverSystem& sys, cudaStream_t s, 
         launches += 2;
         g.dense = true;
     } else if (Lc.n <= dense_cap) {
-        // larger dense coarsest: the grid Gauss-Jordan (one cooperative launch, column strips)
+        // larger dense coarsest: the grid Gauss-Jordan (one cooperative launch, square tiles)
         int nC = Lc.n, dev = 0, sms = 0;
         CICY_CUDA(cudaGetDevice(&dev));
         CICY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -2457,7 +2466,7 @@ void pcg_solve_mg(SolverWork& w, const SolverSystem& sys, double tol, long long 
     g.wtmp.ensure(n);
     k_residual<<<grid_for(n), 256, 0, s>>>(n, sys.rp, sys.ci, sys.val, sys.x, sys.b, w.r.get());
     launches++;
-    // one 16-CTA cluster with hardware barriers when it can be launched, else the
+    // up to kMgClusterMaxRows one 16-CTA cluster with hardware barriers when it can be launched, else the
     // grid-wide cooperative launch
     if (g.cl_state == 0) {
         g.cl_state = cudaFuncSetAttribute(k_mg_pcg<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess ? 1 : -1;
@@ -2496,7 +2505,7 @@ void pcg_solve_mg(SolverWork& w, const SolverSystem& sys, double tol, long long 
         }
         cudaGetLastError();
     }
-    if (g.fused && !sec) throw Fail{CICY_E_INTERNAL, "multigrid: the clustered kernel cannot be launched for a hierarchy built for it"};
+    if (g.fused && !sec) throw Fail{CICY_E_INTERNAL, "multigrid: the grid kernel cannot be launched for a hierarchy built for it"};
     if (!sec && !cluster) {
         int occ = 0;
         CICY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_mg_pcg<false>, kMgThreads, 0));

@@ -1,5 +1,5 @@
 // Direct Electrifying Algorithm on the device: node numbering, resistor
-// assembly by sort-and-reduce, boundary-condition elimination, the Jacobi-PCG
+// assembly by rows, boundary-condition elimination, the Jacobi-PCG
 // voltage solve, backbone extraction and boundary currents
 // (Direct_Electrifying.cpp, Backbone_Network.cpp, Electrical_analysis.cpp).
 #include <algorithm>
