@@ -180,7 +180,9 @@ const char* cicy_last_error(const cicy_ctx* ctx);
 int64_t cicy_ctx_kernel_launches(const cicy_ctx* ctx);
 
 /* ---------------- inputs ---------------- */
-/* Copy a window-trimmed network from host memory into the context's device buffers. */
+/* Copy a window-trimmed network from host memory into the context's device buffers.  An upload,
+ * device construction or contact grid that fails after it has begun to write leaves the context
+ * without the network or grid it wrote over: the stages that need it return CICY_E_STATE. */
 cicy_status cicy_upload_network(cicy_ctx* ctx, const cicy_network* net);
 
 /* ---------------- hot path stages ---------------- */
